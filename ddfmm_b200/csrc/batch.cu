@@ -179,16 +179,6 @@ Batch::Batch(const std::vector<Session*>& sessions) : sessions_(sessions) {
                         add(VINV, subs, n, gg.first);
                     }
                 }
-            } else if (kind == 4) {
-                std::vector<ZeroSub> subs;
-                std::vector<long long> n;
-                for (auto& e : kk.second) {
-                    const Session::Memset& m = e.second->ms;
-                    if (m.bytes % 8) throw std::logic_error("temporary size is not a multiple of 8 bytes");
-                    subs.push_back(ZeroSub{m.p, (long long)(m.bytes / 8), e.first, 0});
-                    n.push_back((long long)(m.bytes / 8));
-                }
-                add(ZERO, subs, n);
             } else {
                 throw std::logic_error("step kind not supported in a batch");
             }

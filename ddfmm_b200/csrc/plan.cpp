@@ -195,7 +195,7 @@ void ColLists::add(std::vector<int>& tab, int k, long long xv, long long yv) {
 }
 
 HfColumns hf_columns(const Tree& T, const HfNodes& up, const HfNodes& dn, const std::vector<int>& kids,
-                     const std::vector<long long>& lf_off, size_t ndirs, size_t ncanon) {
+                     const std::vector<long long>& lf_off, size_t ndirs, size_t ncanon, bool skeleton) {
     HfColumns out;
     // jobs (level, pass, child position): an M2M / L2L pass splits by child
     // position, whose keys (wedge id * 8 + position) are disjoint, and the
@@ -210,7 +210,7 @@ HfColumns hf_columns(const Tree& T, const HfNodes& up, const HfNodes& dn, const 
             (pass == 0 ? out.m2m : pass == 1 ? out.e2 : pass == 2 ? out.e2t : out.l2l)[kv.first];
             if (pass == 0 || pass == 3)
                 for (int ind = 0; ind < 8; ++ind) jobs.push_back(Job{kv.first, pass, ind});
-            else
+            else if (skeleton)
                 jobs.push_back(Job{kv.first, pass, -1});
         }
     std::vector<ColLists> part(jobs.size());

@@ -96,10 +96,13 @@ struct ColLists {
 // 938-991 downward).  kids: the children with points of every box (8 per box,
 // -1 where none); lf_off: the low-frequency vector offset of a box (children
 // of width-1 boxes); ndirs, ncanon: the ranges of HfNode::did and ::canon.
+// skeleton = false leaves the E2 / E2^T lists out (a session folds E2 into its
+// translation operators).
 struct HfColumns {
     std::map<int, ColLists> m2m, e2, e2t, l2l;  // by level
 };
 HfColumns hf_columns(const Tree& T, const HfNodes& up, const HfNodes& dn, const std::vector<int>& kids,
-                     const std::vector<long long>& lf_off, size_t ndirs, size_t ncanon);
+                     const std::vector<long long>& lf_off, size_t ndirs, size_t ncanon,
+                     bool skeleton = true);
 
 }  // namespace ddfmm

@@ -353,10 +353,9 @@ void Session::begin_block(int phase, double W) {
 
 void Session::push_step(Step st) {
     // step types in the order the blocks emit them
-    static const char* const order[] = {"lf_s2m",   "lf_m2m",       "lf_uc2ue",     "memset",   "hf_m2m",
-                                        "hf_uc2ue", "hf_m2l",       "hf_dc2de",     "hf_l2l",   "lf_vlist_fft",
-                                        "lf_vlist_m2l", "lf_vlist_inv", "lf_xlist", "lf_ulist", "lf_wlist",
-                                        "lf_dc2de", "lf_l2t",       "lf_l2l"};
+    static const char* const order[] = {"lf_s2m",       "lf_m2m",       "lf_uc2ue", "hf_m2m",   "hf_m2l",
+                                        "hf_l2l",       "lf_vlist_fft", "lf_vlist_m2l", "lf_vlist_inv",
+                                        "lf_xlist",     "lf_ulist",     "lf_wlist", "lf_dc2de", "lf_l2t", "lf_l2l"};
     std::string base(st.label);
     const size_t u = base.rfind("_w");
     if (u != std::string::npos && u + 2 < base.size() && std::isdigit((unsigned char)base[u + 2]))
@@ -579,25 +578,19 @@ void Session::build() {
     d_pos_ids_ = upload(pos_);
     d_pos_sorted_ = upload(pos_sorted);
     d_den_sorted_ = salloc(npts_);
-    d_val_sorted_ = salloc(npts_);
     d_den_io_ = dalloc<double2>(npts_);
     d_val_io_ = dalloc<double2>(npts_);
-    zero_at_start_.push_back(Memset{d_val_sorted_, es * npts_});
 
     phase("points");
     std::map<int, std::vector<int> > lflevels;  // level -> lf ids (key order)
     for (int l = 0; l < nLF; ++l) lflevels[T.boxes[lfbox[l]].level].push_back(l);
 
     double2* lf_upeq = salloc((size_t)nLF * nE);
-    double2* lf_upchk = salloc((size_t)nLF * nE);
     double2* lf_mid = salloc((size_t)nLF * nE);
-    double2* lf_dnchk = salloc((size_t)nLF * nE);
     double2* lf_dneq = salloc((size_t)nLF * nE);
     double2* lf_spec = salloc((size_t)nLF * G3);
     spectra_elems_ = (size_t)nLF * G3;
     stats_.fft_spectra_bytes = (long long)nLF * G3 * 16;
-    zero_at_start_.push_back(Memset{lf_upchk, es * (size_t)nLF * nE});
-    zero_at_start_.push_back(Memset{lf_dnchk, es * (size_t)nLF * nE});
 
     // per-LF-level device operators
     struct LfLevelOps {
@@ -841,8 +834,7 @@ void Session::build() {
         up.v.reserve(nu);
         dn.v.reserve(nd);
     }
-    std::map<int, long long> tmp_up_level;  // level -> temporary elements of its M2M sums
-    long long upeq_total = 0, dnchk_total = 0, tmp_max = 0;
+    long long upeq_total = 0, dnchk_total = 0;
     for (auto& kv : hflevels) {
         const double W = T.width(kv.first);
         const std::vector<int>& bx = kv.second;
@@ -865,25 +857,15 @@ void Session::build() {
             }
             return dirpts.at(std::make_pair(W, d));
         };
-        std::vector<long long> uo(nbx + 1, 0), ut(nbx + 1, 0), dof(nbx + 1, 0), dt(nbx + 1, 0);
+        std::vector<long long> uo(nbx + 1, 0), dof(nbx + 1, 0);
         std::vector<int> un(nbx + 1, 0), dnn(nbx + 1, 0);
         host_parallel_for(nbx, [&](size_t i) {
             const Box& B = T.boxes[bx[i]];
-            long long a = 0, at = 0, c = 0, ct = 0;
-            for (const Idx3& d : B.outdirs) {
-                const DirPts& dp = lookup(d);
-                a += dp.r1;
-                at += std::max(dp.r1, dp.r2);
-            }
-            for (const Idx3& d : B.incdirs) {
-                const DirPts& dp = lookup(d);
-                c += dp.r1;
-                ct += std::max(dp.r1, dp.r2);
-            }
+            long long a = 0, c = 0;
+            for (const Idx3& d : B.outdirs) a += lookup(d).r1;
+            for (const Idx3& d : B.incdirs) c += lookup(d).r1;
             uo[i + 1] = a;
-            ut[i + 1] = at;
             dof[i + 1] = c;
-            dt[i + 1] = ct;
             un[i + 1] = (int)B.outdirs.size();
             dnn[i + 1] = (int)B.incdirs.size();
         });
@@ -894,9 +876,7 @@ void Session::build() {
         dnn[0] = d0;
         for (size_t i = 0; i < nbx; ++i) {
             uo[i + 1] += uo[i];
-            ut[i + 1] += ut[i];
             dof[i + 1] += dof[i];
-            dt[i + 1] += dt[i];
             un[i + 1] += un[i];
             dnn[i + 1] += dnn[i];
         }
@@ -907,55 +887,61 @@ void Session::build() {
             const Box& B = T.boxes[b];
             up.first[b] = un[i];
             up.cnt[b] = un[i + 1] - un[i];
-            long long o = uo[i], t = ut[i];
+            long long o = uo[i];
             int k = un[i];
             for (const Idx3& d : B.outdirs) {
                 const DirPts& dp = lookup(d);
-                up.v[k++] = HfNode{b, d, dp.canon, o, t, dp.did};
+                up.v[k++] = HfNode{b, d, dp.canon, o, o, dp.did};  // M2M adds straight into the vector
                 o += dp.r1;
-                t += std::max(dp.r1, dp.r2);
             }
             dn.first[b] = dnn[i];
             dn.cnt[b] = dnn[i + 1] - dnn[i];
             o = dof[i];
-            t = dt[i];
             k = dnn[i];
             for (const Idx3& d : B.incdirs) {
                 const DirPts& dp = lookup(d);
-                dn.v[k++] = HfNode{b, d, dp.canon, o, t, dp.did};
+                dn.v[k++] = HfNode{b, d, dp.canon, o, o, dp.did};  // L2L reads the vector itself
                 o += dp.r1;
-                t += std::max(dp.r1, dp.r2);
             }
         });
         upeq_total = uo[nbx];
         dnchk_total = dof[nbx];
-        const long long tmp_up = ut[nbx], tmp_dn = dt[nbx];
         up.range[kv.first] = std::make_pair(u0, (int)up.v.size());
-        tmp_up_level[kv.first] = tmp_up;
         dn.range[kv.first] = std::make_pair(d0, (int)dn.v.size());
-        tmp_max = std::max(tmp_max, std::max(tmp_up, tmp_dn));
     }
     phase("hf_nodes");
     stats_.hf_up_nodes = (long long)up.v.size();
     stats_.hf_down_nodes = (long long)dn.v.size();
-    double2* hf_upeq = salloc((size_t)upeq_total);
-    double2* hf_dnchk = salloc((size_t)dnchk_total);
-    double2* T0 = salloc((size_t)tmp_max);
-    double2* T1 = salloc((size_t)tmp_max);
-    zero_at_start_.push_back(Memset{hf_dnchk, es * (size_t)dnchk_total});
+    // every accumulator of an eval in one allocation, zeroed by one memset at its start
+    const size_t acc_elems[5] = {(size_t)npts_, (size_t)nLF * nE, (size_t)nLF * nE, (size_t)upeq_total,
+                                 (size_t)dnchk_total};
+    size_t acc_off[6] = {0};
+    for (int i = 0; i < 5; ++i) acc_off[i + 1] = acc_off[i] + ((acc_elems[i] + 31) & ~(size_t)31);
+    double2* acc = salloc(acc_off[5]);
+    zero_at_start_.push_back(Memset{acc, es * acc_off[5]});
+    d_val_sorted_ = acc;
+    double2* lf_upchk = E(acc, acc_off[1]);
+    double2* lf_dnchk = E(acc, acc_off[2]);
+    double2* hf_upeq = E(acc, acc_off[3]);
+    double2* hf_dnchk = E(acc, acc_off[4]);
 
     // ---------------------------------------------------------------- HF operators
     // Raw kernel matrices -- M2M ue2uc and L2L de2dc per (W, wedge, child), M2L per
     // (W, canonical wedge, canonical offset) -- are generated once, then folded
     // with the skeleton factors of uc2ue = {E1, E2, E3} (src/mlib3d.cpp:204-207,
     // :246-250) so that the eval applies one dense operator per translation plus
-    // E2 / E2^T per (box, wedge):
-    //   upward   w    = E2 * sum_c [E3 * ue2uc_c * E1(child)] w_c        (upeqnden = E1 w)
+    // nothing else:
+    //   upward   w   += [E2 * (E3 * ue2uc_c * E1(child))] w_c           (upeqnden = E1 w)
     //   M2L      u_t += [E1^T * M(o) * E1] w_s                          (u = E1^T dnchkval)
-    //   downward u_c += [E1(child)^T * de2dc_c * E3^T] (E2^T u)          (dneqnden = E3^T E2^T u)
+    //   downward u_c += [(E1(child)^T * de2dc_c * E3^T) * E2^T] u       (dneqnden = E3^T E2^T u)
     // At W = 1 the children are low-frequency boxes and carry no E1 factor.
     // E1 = inv(R1) and E3 = inv(R2^H) are ill-conditioned (~1e7), so they are
-    // only ever multiplied into the smooth kernel matrices, never into each other.
+    // only ever multiplied into the smooth kernel matrices, never into each other;
+    // E2 joins last.  Applied per node instead, E2 and E2^T were 14% of the HF
+    // products and four of the ten HF launches of a width, and their inputs and
+    // outputs another pass over the node vectors; folded, the rounding of a
+    // translation is the same in FP64 (2e-15 against a long-double product, within
+    // 15% of the two-step form) and 2-4 times smaller in FP32.
     auto take = [](size_t& pool, size_t n) {
         size_t o = pool;
         pool += (n + 15) & ~(size_t)15;
@@ -970,7 +956,7 @@ void Session::build() {
     };
     struct DirMats {
         size_t raw[8], tmp[8], fin[8];
-        int mrows, mcols, canon, ccanon;
+        int mrows, mcols, rmid, canon, ccanon;  // rmid: the wedge's r2, between the factors
         bool cached;            // all eight come from the shared cache
         const float* pk[8];     // their packed copies
     };
@@ -1003,16 +989,16 @@ void Session::build() {
             const DirPts& dp = get_dir(W, up.v[i].dir);
             DirMats M{};
             child_pts(W, up.v[i].dir, true, M.mcols, M.ccanon);
-            M.mrows = dp.r2;
+            M.mrows = dp.r1;
+            M.rmid = dp.r2;
             M.canon = dp.canon;
             M.cached = !opctx_.empty();
             for (int ind = 0; ind < 8 && M.cached; ++ind)
                 M.cached = (M.pk[ind] = cached_op(opk("m2m", W, up.v[i].dir, ind))) != nullptr;
             for (int ind = 0; ind < 8 && !M.cached; ++ind) {
-                size_t n = (size_t)M.mrows * M.mcols;
-                M.raw[ind] = take(scr, n);
-                if (M.ccanon >= 0) M.tmp[ind] = take(scr, n);
-                M.fin[ind] = take(keep, n);
+                M.raw[ind] = take(scr, (size_t)M.rmid * M.mcols);
+                M.tmp[ind] = take(scr, (size_t)M.rmid * M.mcols);
+                M.fin[ind] = take(keep, (size_t)M.mrows * M.mcols);
             }
             m2m_mats[key] = M;
         }
@@ -1023,16 +1009,16 @@ void Session::build() {
             const DirPts& dp = get_dir(W, dn.v[i].dir);
             DirMats M{};
             child_pts(W, dn.v[i].dir, false, M.mrows, M.ccanon);
-            M.mcols = dp.r2;
+            M.mcols = dp.r1;
+            M.rmid = dp.r2;
             M.canon = dp.canon;
             M.cached = !opctx_.empty();
             for (int ind = 0; ind < 8 && M.cached; ++ind)
                 M.cached = (M.pk[ind] = cached_op(opk("l2l", W, dn.v[i].dir, ind))) != nullptr;
             for (int ind = 0; ind < 8 && !M.cached; ++ind) {
-                size_t n = (size_t)M.mrows * M.mcols;
-                M.raw[ind] = take(scr, n);
-                M.fin[ind] = take(keep, n);
-                M.tmp[ind] = M.ccanon >= 0 ? take(scr, n) : M.fin[ind];
+                M.raw[ind] = take(scr, (size_t)M.mrows * M.rmid);
+                M.tmp[ind] = take(scr, (size_t)M.mrows * M.rmid);
+                M.fin[ind] = take(keep, (size_t)M.mrows * M.mcols);
             }
             l2l_mats[key] = M;
         }
@@ -1105,10 +1091,11 @@ void Session::build() {
     }
     phase("m2l_plan");
     stats_.m2l_matrices = (long long)m2l_mats.size();
-    // right factors E1 and E3^T as gatherable columns in the scratch pool
-    std::vector<size_t> scr_E1(hfcanon.size()), scr_E3t(hfcanon.size());
+    // right factors E1, E2^T and E3^T as gatherable columns in the scratch pool
+    std::vector<size_t> scr_E1(hfcanon.size()), scr_E2t(hfcanon.size()), scr_E3t(hfcanon.size());
     for (size_t c = 0; c < hfcanon.size(); ++c) {
         scr_E1[c] = take(scr, (size_t)hfcanon[c].r1 * hfcanon[c].r1);
+        scr_E2t[c] = take(scr, (size_t)hfcanon[c].r1 * hfcanon[c].r2);
         scr_E3t[c] = take(scr, (size_t)hfcanon[c].r2 * hfcanon[c].r2);
     }
     double2* dkeep = dalloc<double2>(keep);
@@ -1117,6 +1104,8 @@ void Session::build() {
     flush_uploads();
     for (size_t c = 0; c < hfcanon.size(); ++c) {
         CK(cudaMemcpyAsync(dscr + scr_E1[c], hfcanon[c].E1, sizeof(double2) * hfcanon[c].r1 * hfcanon[c].r1,
+                           cudaMemcpyDeviceToDevice, stream_));
+        CK(cudaMemcpyAsync(dscr + scr_E2t[c], hfcanon[c].E2t, sizeof(double2) * hfcanon[c].r1 * hfcanon[c].r2,
                            cudaMemcpyDeviceToDevice, stream_));
         CK(cudaMemcpyAsync(dscr + scr_E3t[c], hfcanon[c].E3t, sizeof(double2) * hfcanon[c].r2 * hfcanon[c].r2,
                            cudaMemcpyDeviceToDevice, stream_));
@@ -1153,39 +1142,40 @@ void Session::build() {
     }
 
     phase("kmat");
-    // fold: right products (raw * E1 or raw * E3^T), then left products (E3 * . or E1^T * .)
+    // fold, in three rounds of products (raw doubles as scratch once read):
+    //   M2M  tmp = ue2uc E1(child);  mid = E3 tmp (or E3 raw);  fin = E2 mid
+    //   L2L  tmp = de2dc E3^T;       mid = E1(child)^T tmp;     fin = mid E2^T
+    //   M2L  tmp = M E1;                                        fin = E1^T tmp
     if (scr) {
-        GemmBatch right_s, right_k, left;
+        GemmBatch right, left, last;
         for (auto& kv : m2m_mats) {
             const DirMats& M = kv.second;
             for (int ind = 0; ind < 8 && !M.cached; ++ind) {
-                if (M.ccanon >= 0) {  // tmp = ue2uc * E1(child)
-                    right_s.product(dscr + M.raw[ind], M.mrows, M.mcols, scr_E1[M.ccanon], M.mcols, M.tmp[ind]);
-                    left.product(hfcanon[M.canon].E3, M.mrows, M.mrows, M.tmp[ind], M.mcols, M.fin[ind]);
-                } else {
-                    left.product(hfcanon[M.canon].E3, M.mrows, M.mrows, M.raw[ind], M.mcols, M.fin[ind]);
-                }
+                const bool hf = M.ccanon >= 0;  // else the children are low-frequency boxes
+                const size_t in = hf ? M.tmp[ind] : M.raw[ind], mid = hf ? M.raw[ind] : M.tmp[ind];
+                if (hf) right.product(dscr + M.raw[ind], M.rmid, M.mcols, scr_E1[M.ccanon], M.mcols, M.tmp[ind]);
+                left.product(hfcanon[M.canon].E3, M.rmid, M.rmid, in, M.mcols, mid);
+                last.product(hfcanon[M.canon].E2, M.mrows, M.rmid, mid, M.mcols, M.fin[ind]);
             }
         }
         for (auto& kv : l2l_mats) {
             const DirMats& M = kv.second;
             for (int ind = 0; ind < 8 && !M.cached; ++ind) {
-                if (M.ccanon >= 0) {  // tmp = de2dc * E3^T ; fin = E1(child)^T * tmp
-                    right_s.product(dscr + M.raw[ind], M.mrows, M.mcols, scr_E3t[M.canon], M.mcols, M.tmp[ind]);
-                    left.product(hfcanon[M.ccanon].E1t, M.mrows, M.mrows, M.tmp[ind], M.mcols, M.fin[ind]);
-                } else {  // children are low-frequency boxes: fin = de2dc * E3^T
-                    right_k.product(dscr + M.raw[ind], M.mrows, M.mcols, scr_E3t[M.canon], M.mcols, M.fin[ind]);
-                }
+                const bool hf = M.ccanon >= 0;
+                const size_t mid = hf ? M.raw[ind] : M.tmp[ind];
+                right.product(dscr + M.raw[ind], M.mrows, M.rmid, scr_E3t[M.canon], M.rmid, M.tmp[ind]);
+                if (hf) left.product(hfcanon[M.ccanon].E1t, M.mrows, M.mrows, M.tmp[ind], M.rmid, mid);
+                last.product(dscr + mid, M.mrows, M.rmid, scr_E2t[M.canon], M.mcols, M.fin[ind]);
             }
         }
         for (const M2LMat& M : m2l_mats) {
             if (M.pk) continue;
-            right_s.product(dscr + M.raw, M.r1, M.r1, scr_E1[M.canon], M.r1, M.tmp);
-            left.product(hfcanon[M.canon].E1t, M.r1, M.r1, M.tmp, M.r1, M.fin);
+            right.product(dscr + M.raw, M.r1, M.r1, scr_E1[M.canon], M.r1, M.tmp);
+            last.product(hfcanon[M.canon].E1t, M.r1, M.r1, M.tmp, M.r1, M.fin);
         }
-        right_s.run(dscr, dscr, stream_);
-        right_k.run(dscr, dkeep, stream_);
-        left.run(dscr, dkeep, stream_);
+        right.run(dscr, dscr, stream_);
+        left.run(dscr, dscr, stream_);
+        last.run(dscr, dkeep, stream_);
         CK(cudaStreamSynchronize(stream_));
         CK(cudaFree(dscr));
     }
@@ -1264,13 +1254,12 @@ void Session::build() {
                 const int c = T.child(b, ind);
                 if (c >= 0 && T.boxes[c].has_pts()) kids[(size_t)b * 8 + ind] = c;
             }
-    // the column lists of every level's M2M, E2, E2^T and L2L launches, built on
-    // all host cores (plan.cpp)
+    // the column lists of every level's M2M and L2L launches, built on all host cores (plan.cpp)
     std::vector<std::pair<double, Idx3> > did_wedge(dirpts.size());
     for (auto& kv : dirpts) did_wedge[kv.second.did] = kv.first;
     std::vector<long long> lf_off(nb, -1);
     for (int l = 0; l < nLF; ++l) lf_off[lfbox[l]] = (long long)l * nE;
-    HfColumns cols = hf_columns(T, up, dn, kids, lf_off, dirpts.size(), hfcanon.size());
+    HfColumns cols = hf_columns(T, up, dn, kids, lf_off, dirpts.size(), hfcanon.size(), false);
     phase("hf_columns");
     // ---------------------------------------------------------------- steps: HF upward
     // widths ascending = levels descending; hf_upeq holds w (upeqnden = E1 w)
@@ -1280,14 +1269,9 @@ void Session::build() {
         auto ur = up.range[level];
         if (ur.first == ur.second) continue;
         begin_block(1, W);
-        Step ms{};
-        ms.kind = 4;
-        ms.label = "memset";
-        ms.ms = Memset{T0, es * (size_t)tmp_up_level[level]};  // this level's sums only
-        push_step(ms);
-        // M2M: E3 upchkval = sum_children [E3 ue2uc E1(child)] w_child (src/wave3d_eval.cpp:796-834),
+        // M2M: w = sum_children [E2 E3 ue2uc E1(child)] w_child (src/wave3d_eval.cpp:796-849),
         // one launch for the 8 child positions: a problem per (wedge, child), all adding into
-        // the parents' sums
+        // the parents' vectors
         {
             ColLists& L = cols.m2m.at(level);
             std::vector<GemmProblem> probs;
@@ -1302,24 +1286,7 @@ void Session::build() {
                     if (!opctx_.empty()) opkey_[KP(M.fin[ind])] = opk("m2m", W, dir, ind);
                 }
             }
-            add_gemm(probs, L.x, L.y, W == 1.0 ? lf_upeq : hf_upeq, T0, GEMM_ATOMIC, width_label("hf_m2m", W));
-        }
-        // w = E2 * (E3 upchkval)   (src/wave3d_eval.cpp:837-849)
-        {
-            ColLists& L = cols.e2.at(level);
-            std::vector<GemmProblem> p2;
-            for (int k : L.key) {
-                const Canon& c = hfcanon[k];
-                const std::string key = opk("e2", c.W, c.srt, 0);
-                if (const float* pk = cached_op(key)) {
-                    p2.push_back(GemmProblem{nullptr, c.r1, c.r2, c.r1, 0, 0, pk});
-                } else {
-                    const double2* a = opm(c.E2, (size_t)c.r1 * c.r2);
-                    p2.push_back(GemmProblem{a, c.r1, c.r2, c.r1, 0, 0});
-                    if (!opctx_.empty()) opkey_[a] = key;
-                }
-            }
-            add_gemm(p2, L.x, L.y, T0, hf_upeq, GEMM_SET, width_label("hf_uc2ue", W));
+            add_gemm(probs, L.x, L.y, W == 1.0 ? lf_upeq : hf_upeq, hf_upeq, GEMM_ATOMIC, width_label("hf_m2m", W));
         }
     }
 
@@ -1346,24 +1313,7 @@ void Session::build() {
             }
             add_gemm(probs, m2l_x[level], m2l_y[level], hf_upeq, hf_dnchk, GEMM_ATOMIC, width_label("hf_m2l", W));
         }
-        // t = E2^T u   (dneqnden = E3^T t, src/wave3d_eval.cpp:938-948, src/mlib3d.cpp:246-250)
-        {
-            ColLists& L = cols.e2t.at(level);
-            std::vector<GemmProblem> p2;
-            for (int k : L.key) {
-                const Canon& c = hfcanon[k];
-                const std::string key = opk("e2t", c.W, c.srt, 0);
-                if (const float* pk = cached_op(key)) {
-                    p2.push_back(GemmProblem{nullptr, c.r2, c.r1, c.r2, 0, 0, pk});
-                } else {
-                    const double2* a = opm(c.E2t, (size_t)c.r1 * c.r2);
-                    p2.push_back(GemmProblem{a, c.r2, c.r1, c.r2, 0, 0});
-                    if (!opctx_.empty()) opkey_[a] = key;
-                }
-            }
-            add_gemm(p2, L.x, L.y, hf_dnchk, T1, GEMM_SET, width_label("hf_dc2de", W));
-        }
-        // L2L into the children's (pdir) u, or LF dnchkval at W=1 (src/wave3d_eval.cpp:950-991),
+        // L2L into the children's (pdir) u, or LF dnchkval at W=1 (src/wave3d_eval.cpp:938-991),
         // one launch for the 8 child positions: a problem per (wedge, child)
         {
             ColLists& L = cols.l2l.at(level);
@@ -1379,7 +1329,7 @@ void Session::build() {
                     if (!opctx_.empty()) opkey_[KP(M.fin[ind])] = opk("l2l", W, dir, ind);
                 }
             }
-            add_gemm(probs, L.x, L.y, T1, W == 1.0 ? lf_dnchk : hf_dnchk, GEMM_ATOMIC, width_label("hf_l2l", W));
+            add_gemm(probs, L.x, L.y, hf_dnchk, W == 1.0 ? lf_dnchk : hf_dnchk, GEMM_ATOMIC, width_label("hf_l2l", W));
         }
     }
 
@@ -1422,12 +1372,11 @@ void Session::build() {
                 push_step(f);
                 // summed target spectra: a high-frequency buffer when one is large enough
                 // (every high-frequency pass has run before this low-frequency downward
-                // step, so the outgoing densities, the incoming check values and both
-                // temporaries are all free by then), else a buffer of their own
+                // step, so the outgoing densities and the incoming check values are free
+                // by then), else a buffer of their own
                 const size_t tsp_elems = trg.size() * (size_t)G3;
                 double2* tsp = tsp_elems <= (size_t)upeq_total    ? hf_upeq
                                : tsp_elems <= (size_t)dnchk_total ? hf_dnchk
-                               : tsp_elems <= (size_t)tmp_max     ? T0
                                                                   : salloc(tsp_elems);
                 const int ngroups = (int)vg.gptr.size() - 1;
                 const long long npairs = vg.pairs;
@@ -1620,8 +1569,7 @@ static const char* kernel_name(int kind, int tpi) {
         case 2: return "vlist_forward_kernel";
         case 3: return "vlist_group_kernel";
         case 6: return "vlist_inverse_kernel";
-        case 5: return "umma_cgemm_kernel";
-        default: return "memset";
+        default: return "umma_cgemm_kernel";
     }
 }
 
@@ -1660,9 +1608,6 @@ void Session::launch_step(const Step& st, cudaStream_t s, double2* spec) {
                                        &st.hvi);
             else
                 launch_vlist_inverse(st.v.L, st.v.trg, st.v.ntrg, st.v.tsp, st.v.dnchk, s);
-            break;
-        case 4:
-            CK(cudaMemsetAsync(st.ms.p, 0, st.ms.bytes, s));
             break;
         case 5: {
             const unsigned long long wait_ns = stall_wait_ns_;

@@ -124,14 +124,13 @@ private:
     };
     // one step of the eval: exactly one of these is used
     struct Step {
-        int kind;  // 0 gemm, 1 pt, 2 vfwd, 3 V-list sums, 4 memset, 5 tcgen05 gemm, 6 V-list inverse
+        int kind;  // 0 gemm, 1 pt, 2 vfwd, 3 V-list sums, 5 tcgen05 gemm, 6 V-list inverse
         const char* label;  // pass name for profiling
         double flops;       // algorithmic flops of the launch
         double bytes;       // algorithmic DRAM bytes of the launch
         GemmLaunch g;
         PtLaunch pt;
         VLaunch v;
-        Memset ms;
         // Position of the step in the pass structure, equal across sessions for steps
         // that play the same part (phase, width, step type, occurrence): a Batch
         // merges the steps of its sessions that share a key into one launch.
