@@ -717,6 +717,18 @@ def run_ours(args):
                 "algorithmic_bytes": dk["bytes"] / max(1, dk["launches"]),
                 "peak_source": "measured cuBLAS DGEMM 4096^3 on this GPU (FP64 has no entry in MEASURED_PEAKS.json)",
                 "launches": dk["launches"]}
+    elif dom == "i8_gemm_kernel":
+        # 34 int8 products per real product: 8 algorithmic flops are 4 real products, 272 int8 operations
+        if "bf16_tflops_sustained" in peaks:
+            peak, src = 2 * peaks["bf16_tflops_sustained"], "2 x MEASURED_PEAKS.json bf16_tflops_sustained"
+        else:
+            peak, src = 2 * 1400.0, "2 x fallback 1.4 PFLOP/s bf16 sustained"
+        algo = dk["flops"] / (dk["ms"] * 1e-3) / 1e12
+        roof = {"bound": "tensor", "pipe": "int8 (tcgen05.mma kind::i8)", "kernel": dom, "achieved": 34 * algo,
+                "peak": peak, "unit": "TOP/s", "frac": 34 * algo / peak, "algorithmic_fp64_tflops": algo,
+                "algorithmic_bytes": dk["bytes"] / max(1, dk["launches"]),
+                "peak_source": src + " (dense int8 runs at twice the BF16 rate)",
+                "launches": dk["launches"]}
     else:
         peak = peaks.get("hbm_gbs", 6650.0)
         achieved = dk["bytes"] / (dk["ms"] * 1e-3) / 1e9

@@ -303,6 +303,15 @@ int ddfmm_session_test_gemm_stall(ddfmm_session* s, double wait_s) {
     return guarded([&] { s->impl->arm_gemm_stall(wait_s); });
 }
 
+int ddfmm_test_gemm(const double* A, int m, int k, const double* X, int ncol, int path, double* Y) {
+    if (!A || !X || !Y || m < 1 || m > 400 || k < 1 || k > 400 || ncol < 1 || ncol > (1 << 20) || path < 0 || path > 1)
+        return fail(DDFMM_EINVAL, "bad GEMM test arguments");
+    return guarded([&] {
+        ddfmm::test_gemm(reinterpret_cast<const double2*>(A), m, k, reinterpret_cast<const double2*>(X), ncol, path,
+                         reinterpret_cast<double2*>(Y));
+    });
+}
+
 int ddfmm_tree_stats(const double* pos3n, int n, double K, const double* ctr3, int ptsmax, int maxlevel, int ncell,
                      int npq, int* total_boxes, int* empty_boxes, int* nlevels, ddfmm_tree_level* levels) {
     if (!pos3n || n <= 0 || !total_boxes || !empty_boxes || !nlevels || !levels)

@@ -1,0 +1,86 @@
+// One complex product through a session's GEMM kernels (test entry point
+// ddfmm_test_gemm): what a translation of an eval runs, on the caller's matrices.
+#include <cuda_runtime.h>
+
+#include <stdexcept>
+#include <string>
+#include <vector>
+
+#include "kernels.cuh"
+
+namespace ddfmm {
+
+namespace {
+void ck(cudaError_t e) {
+    if (e != cudaSuccess) throw std::runtime_error(std::string("CUDA error: ") + cudaGetErrorString(e));
+}
+struct Pool {  // device copies, freed together
+    std::vector<void*> p;
+    ~Pool() {
+        for (void* q : p) cudaFree(q);
+    }
+    template <class T>
+    T* put(const std::vector<T>& v) {
+        T* d = nullptr;
+        ck(cudaMalloc(&d, sizeof(T) * (v.empty() ? 1 : v.size())));
+        p.push_back(d);
+        if (!v.empty()) ck(cudaMemcpy(d, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice));
+        return d;
+    }
+};
+}  // namespace
+
+// Y (m x ncol) += A (m x k) X (k x ncol), all column-major complex; the columns
+// are gathered from and scattered to padded vectors in reverse order.
+void test_gemm(const double2* A, int m, int k, const double2* X, int ncol, int path, double2* Y) {
+    Pool P;
+    const int sx = (k + 15) / 16 * 16, sy = (m + 15) / 16 * 16;
+    std::vector<double2> hx((size_t)sx * ncol, make_double2(0, 0)), hy((size_t)sy * ncol, make_double2(0, 0));
+    std::vector<long long> xo(ncol), yo(ncol);
+    std::vector<int> xg(ncol);
+    std::vector<I8Vec> vecs(ncol);
+    for (int c = 0; c < ncol; ++c) {
+        const int at = ncol - 1 - c;
+        xo[c] = (long long)at * sx;
+        yo[c] = (long long)at * sy;
+        xg[c] = at * (sx / 16);
+        vecs[c] = I8Vec{xo[c], xg[c], k};
+        for (int i = 0; i < k; ++i) hx[xo[c] + i] = X[(size_t)c * k + i];
+        for (int i = 0; i < m; ++i) hy[yo[c] + i] = Y[(size_t)c * m + i];
+    }
+    const double2* dA = P.put(std::vector<double2>(A, A + (size_t)m * k));
+    const double2* dX = P.put(hx);
+    double2* dY = P.put(hy);
+    const long long* dyo = P.put(yo);
+    if (path == 0) {
+        std::vector<GemmTile> tiles;
+        for (int r = 0; r < m; r += GEMM_TILE_M)
+            for (int c = 0; c < ncol; c += GEMM_TILE_N) tiles.push_back(GemmTile{0, r, c, 0});
+        gemm_init();
+        launch_gemm(P.put(std::vector<GemmProblem>(1, GemmProblem{dA, m, k, m, 0, ncol, nullptr})), P.put(tiles),
+                    (int)tiles.size(), P.put(xo), dyo, dX, dY, GEMM_ATOMIC, nullptr);
+    } else {
+        const int nkb = (k + 15) / 16;
+        char* B = P.put(std::vector<char>(i8_packed_bytes(m, k)));
+        double* ra = P.put(std::vector<double>(m));
+        char* X8 = P.put(std::vector<char>((size_t)ncol * (sx / 16) * I8_GRANULE));
+        double* cx = P.put(std::vector<double>((size_t)ncol * (sx / 16)));
+        std::vector<I8Tile> tiles;
+        i8_tiles(B, ra, m, k, 0, ncol, tiles);
+        int* err = P.put(std::vector<int>(1, 0));
+        i8_init();
+        launch_i8_pack(P.put(std::vector<I8PackJob>(1, I8PackJob{dA, B, ra, m, k, m, nkb, i8_tile_rows(m)})), 1,
+                       i8_row_tiles(m), nullptr);
+        launch_i8_slice(P.put(vecs), ncol, dX, X8, cx, nullptr);
+        launch_i8_gemm(I8Sub{P.put(tiles), P.put(xg), dyo, X8, cx, dY, (int)tiles.size()}, err, nullptr);
+        int h = 0;
+        ck(cudaMemcpy(&h, err, sizeof(int), cudaMemcpyDeviceToHost));
+        if (h) throw std::runtime_error("CUDA error: the int8 GEMM timed out waiting on its pipeline");
+    }
+    ck(cudaGetLastError());
+    ck(cudaMemcpy(hy.data(), dY, sizeof(double2) * hy.size(), cudaMemcpyDeviceToHost));
+    for (int c = 0; c < ncol; ++c)
+        for (int i = 0; i < m; ++i) Y[(size_t)c * m + i] = hy[yo[c] + i];
+}
+
+}  // namespace ddfmm

@@ -55,6 +55,26 @@ void launch_kmat(const KmatJob* jobs, int njobs, long long total, int kernel, cu
     kmat_kernel<<<(unsigned)blocks, 256, 0, s>>>(jobs, njobs, total, kernel);
 }
 
+__global__ void list_columns_kernel(const ColumnSpan* __restrict__ spans, int nspans, long long ncols,
+                                    long long* __restrict__ xoff, long long* __restrict__ yoff) {
+    const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= ncols) return;
+    int lo = 0, hi = nspans - 1;
+    while (lo < hi) {  // last span with first <= c
+        const int mid = (lo + hi + 1) >> 1;
+        if (spans[mid].first <= c) lo = mid; else hi = mid - 1;
+    }
+    const ColumnSpan S = spans[lo];
+    xoff[c] = S.bx + (c - S.first) * S.sx;
+    yoff[c] = S.cy + (c - S.first) * S.sy;
+}
+
+void launch_list_columns(const ColumnSpan* spans, int nspans, long long ncols, long long* xoff, long long* yoff,
+                         cudaStream_t s) {
+    if (nspans > 0 && ncols > 0)
+        list_columns_kernel<<<(unsigned)((ncols + 255) / 256), 256, 0, s>>>(spans, nspans, ncols, xoff, yoff);
+}
+
 // ---------------------------------------------------------------- gemm
 // Grouped complex FP64 GEMM with gathered input columns and scattered output
 // columns, on the FP64 tensor path (mma.sync m16n8k8 f64; the m8n8k4 and

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
+#include <vector>
 
 namespace ddfmm {
 
@@ -59,6 +60,13 @@ struct PtSrc {
 };
 
 void launch_kmat(const KmatJob* jobs_dev, int njobs, long long total, int kernel, cudaStream_t s);
+// Columns of a setup product: column c of the span's is X + bx + c sx and Y + cy + c sy.
+struct ColumnSpan {
+    long long first, bx, cy;  // first: the span's first column in the launch
+    int sx, sy;
+};
+void launch_list_columns(const ColumnSpan* spans_dev, int nspans, long long ncols, long long* xoff, long long* yoff,
+                         cudaStream_t s);
 void launch_gemm(const GemmProblem* probs_dev, const GemmTile* tiles_dev, int ntiles,
                  const long long* xoff, const long long* yoff, const double2* X, double2* Y, int mode,
                  cudaStream_t s);
@@ -241,6 +249,51 @@ void launch_umma_pack(const UmmaPackJob* jobs_dev, int njobs, cudaStream_t s);
 void launch_umma_cgemm(const UmmaSub* subs, const int* prefix, int nsub, int ntiles, const int* active, int* err,
                        cudaStream_t s, const UmmaSub* one, unsigned long long wait_ns = 0, int withhold = 0,
                        const int* order = nullptr);
+
+// FP64 GEMM on the int8 tensor path (kernels_i8.cu): 128 gathered columns x up to
+// I8_TILE_ROWS complex operator rows per tile; both operands as seven int8 digit
+// planes under a power-of-two scale per vector / operator row.
+constexpr int I8_DIGITS = 7;
+constexpr int I8_TILE_ROWS = 56;
+constexpr int I8_GRANULE = 16 * 2 * I8_DIGITS;  // bytes of the digits of 16 complex numbers
+struct I8Vec {      // a vector to write as digits
+    long long src;  // its first element in X
+    int gran;       // its first granule (and its entry of cx)
+    int len;        // complex numbers
+};
+void launch_i8_slice(const I8Vec* vecs, int n, const double2* X, char* X8, double* cx, cudaStream_t s);
+struct alignas(16) I8Tile {  // everything about a tile, so that its next one can be read ahead
+    const char* B;         // the row tile's packed operator (i8_pack_kernel)
+    const double* ra;      // output scales of its rows
+    int col, row0;         // first column (of xgran, yoff), first operator row
+    unsigned short ncol, rows, n, nkb;  // columns, valid complex rows, int8 rows, 16-wide complex K blocks
+};
+struct I8Sub {
+    const I8Tile* tiles;
+    const int* xgran;        // first granule of each column's vector
+    const long long* yoff;   // element of Y each column adds into
+    const char* X8;
+    const double* cx;
+    double2* Y;
+    int ntiles;
+};
+struct I8PackJob {
+    const double2* A;  // complex operator, column-major
+    char* dst;
+    double* ra;
+    int m, k, lda, nkb, rows_t;
+};
+void i8_init();
+int i8_row_tiles(int m);
+int i8_tile_rows(int m);
+size_t i8_packed_bytes(int m, int k);
+// the tiles of one problem: m x k operator packed at B with row scales ra, columns col0 .. col0 + ncol
+void i8_tiles(const char* B, const double* ra, int m, int k, int col0, int ncol, std::vector<I8Tile>& out);
+void launch_i8_pack(const I8PackJob* jobs_dev, int njobs, int max_tiles, cudaStream_t s);
+// *err is set when a block gave up waiting on its pipeline
+void launch_i8_gemm(const I8Sub& sub, int* err, cudaStream_t s);
+// gemm_test.cu: Y += A X through a GEMM kernel of the plain form (0: FP64, 1: int8 tensor path)
+void test_gemm(const double2* A, int m, int k, const double2* X, int ncol, int path, double2* Y);
 
 // gather/scatter helpers
 void launch_gather_den(const double2* den, const int* perm, double2* out, int n, cudaStream_t s);

@@ -1,0 +1,674 @@
+// FP64 complex GEMM on the integer tensor cores (tcgen05 kind::i8).
+//
+// Problem (as in zgemm_kernel): Y[:, c] += A X[:, c] for gathered columns c, A
+// an m x k complex operator.  The FP64 tensor path peaks at 37 TF/s; the int8
+// path does 34 exact integer products per FP64 product at over 100 times that
+// rate.  Every column (and every operator row) is written as
+//     x_j = 2^(ex - 54) q_j,   q_j = sum_{i=0}^{6} d_i 256^(6-i),  d_i in [-128, 127],
+// 2^ex above the vector's largest component: 54 bits below it, a rounding of at
+// most half the last place of the largest FP64 entry.  With X's digits d and A's
+// digits e, a product of two numbers is sum_{i,j} d_i e_j 256^(12-i-j); the terms
+// i + j <= 7 are kept (34 of 49; the dropped ones are below 2^-58 of the largest
+// product).  Those of one diagonal i + j are summed over k by the tensor core in
+// int32 without any rounding, the eight diagonals joined in int64 and rounded to
+// FP64 twice per output, so the sums over k carry no rounding error at all: on
+// folded translation operators at P = 4, 6, 8 the result is 0.9-2.2e-16 from a
+// long-double product in relative 2-norm, the three-MMA FP64 form 3-8e-16.
+//
+// One tile is 128 gathered columns (the MMA's M, one TMEM lane each) x up to 56
+// complex operator rows; operator row i becomes the int8 rows [Ar, -Ai] and
+// [Ai, Ar] (N = 2 rows), K = 2k interleaved real and imaginary digits.  int32
+// accumulators of eight diagonals would need 8 N of the 512 TMEM columns, so a
+// tile runs its K loop twice: diagonals 4 .. 7 (24 MMAs per 32-wide K block,
+// 4 N <= 448 columns; drained to one FP64 per output), then 0 .. 3 (10 MMAs, of
+// which only the first four planes are loaded).
+//
+// Operands sit in shared memory K-major in the 32-byte swizzled layout, one
+// plane per digit.  Digits come from memory: the operator's are packed at setup
+// in the order a K block is consumed (one bulk copy per block), a vector's are
+// written once by i8_slice_kernel as 224-byte granules (16 complex numbers x 7
+// digit planes) and gathered by every column that uses it with 16-byte
+// cp.async (eight lanes fill four 32-byte rows: all banks once).
+//
+// Persistent, one 512-thread block per SM.  Warp groups (registers moved from
+// the first two to the last two):
+//   0     operands: warps 0 .. 2 fill ring slot 0 .. 2, the operator block by one
+//         bulk copy, the columns by cp.async
+//   1     warp 4: MMA issue, one thread
+//   2, 3  epilogue: warp w on TMEM lanes 32 (w % 4) .., group 2 on the tile's
+//         first half of the rows, group 3 on the second.  After the second K
+//         loop a thread holds its column's outputs as FP64 in registers, hands
+//         the accumulators back, then scales and parks 14 rows at a time in
+//         shared memory and adds each column's piece with one bulk reduction
+//         (warp-wide FP64 atomics from the parked rows took twice as long: their
+//         shared loads queue behind the tensor core's operand reads).
+// Measured (m 100, k 152, 491,520 gathered columns): 1.02 ms, 59 TF/s of complex
+// products against 28 for zgemm_kernel; 105 clocks an MMA, of which 60 are the
+// operand reads (4 KB + 32 N bytes at 128 a clock; the MMA itself needs 56), 19
+// the slots' fill, 11 the drain of the accumulators.
+// Every mbarrier wait is bounded as in umma_cgemm_kernel (1 s, or until another
+// role failed); a block that gives up drains its copies, frees its TMEM and
+// sets *err.
+#include <cuda_runtime.h>
+
+#include <cstdint>
+#include <stdexcept>
+
+#include "kernels.cuh"
+
+namespace ddfmm {
+
+namespace {
+constexpr int IS = I8_DIGITS;                 // digit planes
+constexpr int IM = 128;                       // gathered columns per tile
+constexpr int INMAX = 2 * I8_TILE_ROWS;       // int8 operator rows per tile
+constexpr int ISTAGES = 3;                    // ring depth
+constexpr int I_X_PLANE = IM * 32;            // bytes of one digit plane of a column block
+constexpr int I_X_BYTES = IS * I_X_PLANE;
+constexpr int I_B_BYTES = IS * INMAX * 32;
+constexpr int I_STAGE_BYTES = I_X_BYTES + I_B_BYTES;
+constexpr int IPR = 14;                       // complex rows parked per column
+constexpr int IPS = IPR * 16 + 16;            // bytes per parked column: 16-byte stores of 8 lanes hit all banks
+constexpr int I_PARK_WARP = 32 * IPS;
+constexpr int I_SMEM = ISTAGES * I_STAGE_BYTES + 8 * I_PARK_WARP + 1024;
+static_assert(I_SMEM + 1024 <= 232448, "shared memory per block");
+constexpr int ITHREADS = 512;
+constexpr int ICH = 8;                        // accumulator columns per TMEM load
+constexpr int ICHUNKS = INMAX / 2 / ICH;      // chunks of a warp's half tile
+constexpr unsigned long long I_WAIT_NS = 1000000000ull;
+constexpr uint32_t I_WAIT_ITERS = 1u << 26;
+static_assert(I_STAGE_BYTES % 256 == 0 && INMAX % 16 == 0 && INMAX <= 128, "swizzle atoms");
+
+__device__ __forceinline__ uint32_t su32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// byte offset of byte b (0 .. 31) of row r in a 32-byte swizzled K-major plane:
+// 8-row groups of 256 bytes, the row's two 16-byte halves exchanged in rows 4 .. 7
+__host__ __device__ __forceinline__ int i8_off(int r, int b) { return r * 32 + ((((b >> 4) ^ ((r >> 2) & 1)) << 4) | (b & 15)); }
+
+// K-major operand descriptor, 32-byte swizzle (layout type 6), 8-row groups 256
+// bytes apart: the low word holds the address, the high word is constant
+__device__ __forceinline__ uint32_t i8_desc(uint32_t saddr) { return ((saddr >> 4) & 0x3FFF) | (1u << 16); }
+constexpr uint32_t I_DESC_HI = (256 >> 4) | (1u << 14) | (6u << 29);
+// D s32 (bits 4-5 = 2), A and B s8 (bits 7-9, 10-12 = 1), N >> 3 at 17, M >> 4 at 24
+__device__ constexpr uint32_t i8_idesc(int n) {
+    return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(IM >> 4) << 24);
+}
+// whether the phase of this parity has completed; the caller may go on before it looks at the answer
+__device__ __forceinline__ uint32_t bar_peek(uint64_t* bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(done)
+        : "r"(su32(bar)), "r"(parity)
+        : "memory");
+    return done;
+}
+__device__ __forceinline__ void i8_mma(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "mov.b64 da, {%1, %6};\n\tmov.b64 db, {%2, %6};\n\t"
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], da, db, %3, {%5, %5, %5, %5}, p;\n\t}\n" ::"r"(d),
+        "r"(a), "r"(b), "r"(idesc), "r"(acc), "r"(0u), "r"(I_DESC_HI)
+        : "memory");
+}
+__device__ __forceinline__ void i8_commit(uint64_t* bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(su32(bar))
+                 : "memory");
+}
+__device__ __forceinline__ unsigned long long i8_timer() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;\n" : "=l"(t));
+    return t;
+}
+__device__ __forceinline__ void bar_init(uint64_t* bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(su32(bar)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(su32(bar)) : "memory");
+}
+// false after limit_ns, 2^26 polls, or once *failed is set by another role
+__device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity, volatile int* failed,
+                                         unsigned long long limit_ns) {
+    const uint32_t addr = su32(bar);
+    unsigned long long t0 = 0;
+    for (uint32_t it = 0; it < I_WAIT_ITERS; ++it) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}\n"
+            : "=r"(done)
+            : "r"(addr), "r"(parity)
+            : "memory");
+        if (done) return true;
+        if ((it & 255) == 255) {
+            if (failed && *failed) return false;
+            const unsigned long long t = i8_timer();
+            if (t0 == 0)
+                t0 = t;
+            else if (t - t0 > limit_ns)
+                return false;
+        }
+    }
+    return false;
+}
+
+// bar_wait by one lane for its warp: polls take shared-memory cycles from the
+// tensor core's operand reads
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* failed,
+                                          unsigned long long limit_ns) {
+    int ok = 1;
+    if ((threadIdx.x & 31) == 0) ok = !*failed && bar_wait(bar, parity, failed, limit_ns);
+    return __shfl_sync(0xffffffffu, ok, 0);
+}
+
+// The MMA issuer's place in the ring: slot, its parity, and whether the slot is
+// already known to be full.
+struct I8Ring {
+    uint32_t slot, parity, ready;
+};
+
+// One K loop of a tile: diagonals 4 .. 7 (PH 0) or 0 .. 3 (PH 1), per K block a
+// chain of plane pairs i + j = d on accumulator d % 4.  One thread issues
+// everything and the tensor core's queue is short, so what it does between two
+// MMAs shows: N is a template argument (every address is the slot's plus a
+// constant), slot and parity are counted rather than divided out, and the next
+// slot's barrier -- whose answer takes some 250 clocks beside the operand reads --
+// is asked before the block's last MMAs.
+template <int N, int PH>
+__device__ __forceinline__ bool i8_phase(uint32_t tmem, uint32_t dx0, int nkb, I8Ring& R, uint64_t* full, uint64_t* empty,
+                                         uint64_t* acc_full, volatile int* failed, unsigned long long wait_ns) {
+    for (int kb = 0; kb < nkb; ++kb) {
+        if (!R.ready && !bar_wait(full + R.slot, R.parity, failed, wait_ns)) return false;
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        const uint32_t dx = dx0 + R.slot * (I_STAGE_BYTES >> 4), db = dx + (I_X_BYTES >> 4);
+        uint64_t* const done = empty + R.slot;
+        const bool wrap = R.slot == ISTAGES - 1;
+        R.slot = wrap ? 0 : R.slot + 1;
+        R.parity ^= wrap;
+#pragma unroll
+        for (int d = PH ? 0 : 4; d < (PH ? 4 : 8); ++d) {
+            const int i0 = d < IS ? 0 : d - IS + 1;
+            if (d == (PH ? 2 : 7)) R.ready = bar_peek(full + R.slot, R.parity);
+#pragma unroll
+            for (int i = i0; i <= d - i0; ++i)
+                i8_mma(tmem + (uint32_t)((d & 3) * N), dx + i * (I_X_PLANE >> 4), db + (d - i) * (N * 2), i8_idesc(N),
+                       i > i0 ? 1u : (uint32_t)kb);
+        }
+        i8_commit(done);
+    }
+    i8_commit(acc_full);
+    return true;
+}
+
+// ---------------------------------------------------------------- digits
+// The seven balanced base-256 digits of q, |q| <= 2^54: adding 128 to every
+// digit place makes them the bytes of one sum; flipping each byte's top bit
+// takes the 128 off again.  Byte i of the result is digit 6 - i.
+constexpr unsigned long long I_BIAS = 0x0080808080808080ull;
+__device__ __forceinline__ unsigned long long i8_digits(long long q) { return ((unsigned long long)q + I_BIAS) ^ I_BIAS; }
+
+// Largest |x| of a vector by its high word (sign off): the vector's exponent ex
+// (largest |x| < 2^ex), the factor 2^(54 - ex) as two powers of two (a vector
+// below 2^-900 is brought up first, so subnormals keep their bits) and
+// 2^(ex - 1); NaN when the vector holds an infinity or a NaN, zero when it is zero.
+struct I8Scale {
+    double up, s, out;
+};
+__device__ __forceinline__ I8Scale i8_scale(uint32_t top) {
+    I8Scale r;
+    const int be = (int)(top >> 20);
+    if (be == 0x7ff) {
+        r.up = r.s = 0.0;
+        r.out = __longlong_as_double(0x7ff8000000000000ll);
+        return r;
+    }
+    const int b1 = be < 1 ? 1 : be;  // subnormals: below 2^-1022
+    const bool low = b1 < 123;
+    r.up = low ? __longlong_as_double((long long)(1023 + 200) << 52) : 1.0;
+    r.s = __longlong_as_double((long long)(2099 - b1 - (low ? 200 : 0)) << 52);  // 2^(1076 - b1 [- 200])
+    r.out = __longlong_as_double((long long)(b1 == 0 ? 1 : b1) << 52);           // 2^(b1 - 1023) = 2^(ex - 1)
+    return r;
+}
+__device__ __forceinline__ long long i8_quant(double x, const I8Scale& S) { return __double2ll_rn(x * S.up * S.s); }
+__device__ __forceinline__ uint32_t top_word(double x) { return (uint32_t)__double2hiint(x) & 0x7fffffffu; }
+// high word of |x| counting a nonzero low word of a value whose high word is zero
+__device__ __forceinline__ uint32_t top_of(double2 v) { return max(top_word(v.x), top_word(v.y)); }
+
+// eight digit bytes, place p of eight numbers: byte p of w[0..7]
+__device__ __forceinline__ uint2 gather_bytes(const unsigned long long (&w)[8], int p) {
+    uint32_t r[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        uint32_t v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = p < 4 ? (uint32_t)w[4 * h + j] : (uint32_t)(w[4 * h + j] >> 32);
+        const int b = p & 3;
+        const uint32_t lo = __byte_perm(v[0], v[1], b | ((b + 4) << 4));
+        const uint32_t hi = __byte_perm(v[2], v[3], b | ((b + 4) << 4));
+        r[h] = __byte_perm(lo, hi, 0x5410);
+    }
+    return make_uint2(r[0], r[1]);
+}
+}  // namespace
+
+// Digits of vectors: one warp per vector, four lanes per granule of 16 complex
+// numbers (each lane 4 of them: 8 bytes in each of the 7 planes).  Bound by
+// HBM: 16 bytes read and 14 written per complex number.
+__global__ void __launch_bounds__(256) i8_slice_kernel(const I8Vec* __restrict__ vecs, int n,
+                                                       const double2* __restrict__ X, char* __restrict__ X8,
+                                                       double* __restrict__ cx) {
+    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (w >= n) return;
+    const I8Vec V = vecs[w];
+    const double2* x = X + V.src;
+    uint32_t top = 0;
+    double2 v[4];
+    const int ng = (V.len + 15) >> 4;
+    for (int g0 = 0; g0 < ng; g0 += 8) {  // 8 granules a pass
+        const int j0 = g0 * 16 + lane * 4;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            v[j] = j0 + j < V.len ? x[j0 + j] : make_double2(0.0, 0.0);
+            top = max(top, top_of(v[j]));
+        }
+    }
+    top = __reduce_max_sync(0xffffffffu, top);
+    const I8Scale S = i8_scale(top);
+    if (lane == 0) cx[V.gran] = S.out;
+    for (int g0 = 0; g0 < ng; g0 += 8) {
+        const int j0 = g0 * 16 + lane * 4;
+        if (ng > 8) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = j0 + j < V.len ? x[j0 + j] : make_double2(0.0, 0.0);
+        }
+        if (g0 + (lane >> 2) < ng) {
+            unsigned long long q[8];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                q[2 * j] = i8_digits(i8_quant(v[j].x, S));
+                q[2 * j + 1] = i8_digits(i8_quant(v[j].y, S));
+            }
+            char* o = X8 + (size_t)(V.gran + g0 + (lane >> 2)) * I8_GRANULE + (lane & 3) * 8;
+#pragma unroll
+            for (int p = 0; p < IS; ++p) *reinterpret_cast<uint2*>(o + p * 32) = gather_bytes(q, IS - 1 - p);
+        }
+    }
+}
+
+void launch_i8_slice(const I8Vec* vecs, int n, const double2* X, char* X8, double* cx, cudaStream_t s) {
+    if (n > 0) i8_slice_kernel<<<(unsigned)(((size_t)n * 32 + 255) / 256), 256, 0, s>>>(vecs, n, X, X8, cx);
+}
+
+// Operator digits (setup only): block (row tile, job).  Row scales first, then
+// 4 complex numbers of a row at a time into K block order: block kb of a row
+// tile holds plane p of its 2 rows_t int8 rows at p * rows_t * 64.
+__global__ void __launch_bounds__(256) i8_pack_kernel(const I8PackJob* __restrict__ jobs, int njobs) {
+    __shared__ uint32_t tops[4][64];
+    __shared__ I8Scale sc[64];
+    const int tid = threadIdx.x;
+    for (int j = blockIdx.y; j < njobs; j += gridDim.y) {
+        const I8PackJob J = jobs[j];
+        const int row0 = blockIdx.x * J.rows_t;
+        if (row0 >= J.m) continue;  // uniform over the block
+        __syncthreads();
+        {
+            const int r = tid & 63;
+            uint32_t top = 0;
+            if (r < J.rows_t && row0 + r < J.m)
+                for (int k = tid >> 6; k < J.k; k += 4) top = max(top, top_of(J.A[(size_t)k * J.lda + row0 + r]));
+            tops[tid >> 6][r] = top;
+        }
+        __syncthreads();
+        if (tid < J.rows_t) {
+            sc[tid] = i8_scale(max(max(tops[0][tid], tops[1][tid]), max(tops[2][tid], tops[3][tid])));
+            // the output scale of a row: 2^(ea - 1) 2^-34 (the epilogue's sums count units
+            // of diagonal 3: 256^9 2^(ex - 54) 2^(ea - 54) = 2^(ex + ea - 36), and cx = 2^(ex - 1))
+            if (row0 + tid < J.m) J.ra[row0 + tid] = sc[tid].out * 0x1p-34;
+        }
+        __syncthreads();
+        const int nq = J.nkb * 4, N = 2 * J.rows_t;
+        char* dst = J.dst + (size_t)blockIdx.x * J.nkb * IS * N * 32;
+        for (int e = tid; e < nq * J.rows_t; e += 256) {
+            const int r = e % J.rows_t, q4 = e / J.rows_t, k0 = q4 * 4;
+            const I8Scale S = sc[r];
+            unsigned long long w0[8], w1[8];  // rows [Ar, -Ai] and [Ai, Ar]
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const bool ok = row0 + r < J.m && k0 + i < J.k;
+                const double2 a = ok ? J.A[(size_t)(k0 + i) * J.lda + row0 + r] : make_double2(0.0, 0.0);
+                const long long qr = i8_quant(a.x, S), qi = i8_quant(a.y, S);
+                w0[2 * i] = w1[2 * i + 1] = i8_digits(qr);
+                w0[2 * i + 1] = i8_digits(-qi);
+                w1[2 * i] = i8_digits(qi);
+            }
+            char* blk = dst + (size_t)(q4 >> 2) * IS * N * 32;
+            const int b = (q4 & 3) * 8;
+#pragma unroll
+            for (int p = 0; p < IS; ++p) {
+                *reinterpret_cast<uint2*>(blk + p * N * 32 + i8_off(2 * r, b)) = gather_bytes(w0, IS - 1 - p);
+                *reinterpret_cast<uint2*>(blk + p * N * 32 + i8_off(2 * r + 1, b)) = gather_bytes(w1, IS - 1 - p);
+            }
+        }
+    }
+}
+
+int i8_row_tiles(int m) { return (m + I8_TILE_ROWS - 1) / I8_TILE_ROWS; }
+int i8_tile_rows(int m) { return ((m + i8_row_tiles(m) - 1) / i8_row_tiles(m) + 7) / 8 * 8; }
+size_t i8_packed_bytes(int m, int k) {
+    return (size_t)i8_row_tiles(m) * ((k + 15) / 16) * IS * 2 * i8_tile_rows(m) * 32;
+}
+
+void i8_tiles(const char* B, const double* ra, int m, int k, int col0, int ncol, std::vector<I8Tile>& out) {
+    const int nrt = i8_row_tiles(m), rt = i8_tile_rows(m), nkb = (k + 15) / 16;
+    for (int c = 0; c < ncol; c += IM)
+        for (int r = 0; r < nrt; ++r)  // adjacent: the row tiles of a column block read its digits from L2 together
+            out.push_back(I8Tile{B + (size_t)r * nkb * IS * 2 * rt * 32, ra + r * rt, col0 + c, r * rt,
+                                 (unsigned short)(ncol - c < IM ? ncol - c : IM),
+                                 (unsigned short)(m - r * rt < rt ? m - r * rt : rt), (unsigned short)(2 * rt),
+                                 (unsigned short)nkb});
+}
+
+void launch_i8_pack(const I8PackJob* jobs, int njobs, int max_tiles, cudaStream_t s) {
+    if (njobs > 0) i8_pack_kernel<<<dim3(max_tiles, njobs < 32768 ? njobs : 32768), 256, 0, s>>>(jobs, njobs);
+}
+
+// ---------------------------------------------------------------- GEMM
+namespace {
+__device__ __forceinline__ I8Tile i8_tile(const I8Sub& S, int ti) {
+    union {
+        int4 w[2];
+        I8Tile t;
+    } u;
+    static_assert(sizeof(I8Tile) == 32, "two 16-byte loads");
+    const int4* p = reinterpret_cast<const int4*>(S.tiles + (ti < S.ntiles ? ti : 0));
+    u.w[0] = __ldg(p);
+    u.w[1] = __ldg(p + 1);
+    return u.t;
+}
+// four diagonals as one FP64 number, in units of the last, exactly (below 2^51)
+__device__ __forceinline__ double join4(int a, int b, int c, int d) {
+    return (double)(((long long)a * 256 + b) * 65536 + ((long long)c * 256 + d));
+}
+// a warp's copies of NP digit planes of K block kb: 128 columns, zero where absent
+template <int NP>
+__device__ __forceinline__ void i8_copy(uint32_t dst, const int (&gran)[8], const char* X8, int kb) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const char* a = X8 + (gran[j] < 0 ? 0 : (size_t)(gran[j] + kb) * I8_GRANULE);
+        const int n = gran[j] < 0 ? 0 : 16;
+#pragma unroll
+        for (int p = 0; p < NP; ++p)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst + p * I_X_PLANE + j * 512),
+                         "l"(a + p * 32), "r"(n));
+    }
+}
+template <int R>
+__device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(R)); }
+template <int R>
+__device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(R)); }
+__device__ __forceinline__ void tmem_ld8(uint32_t addr, int (&v)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(addr)
+                 : "memory");
+}
+// eight columns of four accumulators n columns apart
+__device__ __forceinline__ void tmem_ld4(uint32_t addr, int n, int (&d)[4][8]) {
+#pragma unroll
+    for (int a = 0; a < 4; ++a) tmem_ld8(addr + (uint32_t)(a * n), d[a]);
+}
+}  // namespace
+
+__global__ void __launch_bounds__(ITHREADS, 1) i8_gemm_kernel(const I8Sub S, int* err, unsigned long long wait_ns) {
+    extern __shared__ __align__(1024) unsigned char ism_raw[];
+    __shared__ __align__(8) uint64_t full[ISTAGES], empty[ISTAGES], acc_full, acc_empty, drained;
+    __shared__ uint32_t tmem_base;
+    __shared__ int failed_s;
+    volatile int* failed = &failed_s;
+    unsigned char* sm = (unsigned char*)(((uintptr_t)ism_raw + 1023) & ~(uintptr_t)1023);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        failed_s = 0;
+        for (int s = 0; s < ISTAGES; ++s) {
+            bar_init(&full[s], 2);        // the operator copy's bytes, the gathered columns
+            bar_init(&empty[s], 1);       // tcgen05.commit
+        }
+        bar_init(&acc_full, 1);     // tcgen05.commit
+        bar_init(&drained, 1);      // tcgen05.commit, after a failure
+        bar_init(&acc_empty, 8);    // epilogue warps
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(su32(&tmem_base)), "r"(512)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    const uint32_t tmem = tmem_base;
+
+    if (warp < 4) {
+        reg_dec<48>();
+        // ------------------------------------------------ operands
+        // warp w owns ring slot w, so all slots are filled at once and none waits for the
+        // next one to become free (one owner a slot: a warp that could run a second
+        // phase ahead would read the slot's empty barrier by the wrong parity).  Lane l
+        // copies half l % 2 of the 32-byte rows of columns l / 2 + 16 j
+        const int hf = lane & 1;
+        const uint32_t dst = su32(sm) + i8_off(lane >> 1, hf * 16);
+        int g = 0;
+        bool ok = true;
+        I8Tile Tn = i8_tile(S, blockIdx.x);
+        for (int ti = blockIdx.x; ti < S.ntiles && ok && warp < ISTAGES; ti += gridDim.x) {
+            const I8Tile T = Tn;
+            Tn = i8_tile(S, ti + gridDim.x);
+            int gran[8];  // the columns' first granules, -1 past the last one
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int c = (lane >> 1) + 16 * j;
+                gran[j] = c < T.ncol ? __ldg(S.xgran + T.col + c) : -1;
+            }
+            for (int ph = 0; ph < 2 && ok; ++ph)
+                for (int kb = 0; kb < T.nkb; ++kb, ++g) {
+                    const int s = g % ISTAGES;
+                    if (s != warp) continue;
+                    if (g >= ISTAGES && !warp_wait(&empty[s], ((g / ISTAGES) - 1) & 1, failed, wait_ns)) {
+                        *failed = 1;
+                        ok = false;
+                        break;
+                    }
+                    if (lane == 0) {
+                        const uint32_t bytes = (uint32_t)(ph == 0 ? IS : 4) * T.n * 32;
+                        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%1], %0;\n" ::"r"(bytes),
+                                     "r"(su32(&full[s]))
+                                     : "memory");
+                        asm volatile(
+                            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
+                                su32(sm + s * I_STAGE_BYTES + I_X_BYTES)),
+                            "l"(T.B + (size_t)kb * IS * T.n * 32), "r"(bytes), "r"(su32(&full[s]))
+                            : "memory");
+                    }
+                    const uint32_t so = dst + s * I_STAGE_BYTES;
+                    if (ph == 0)
+                        i8_copy<IS>(so, gran, S.X8 + hf * 16, kb);
+                    else
+                        i8_copy<4>(so, gran, S.X8 + hf * 16, kb);
+                    asm volatile("cp.async.wait_all;\n" ::: "memory");
+                    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) bar_arrive(&full[s]);
+                }
+        }
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+    } else if (warp < 8) {
+        reg_dec<48>();
+        if (warp == 4 && lane == 0) {
+            // -------------------------------------------- MMA issue
+            I8Ring R{0, 0, 0};
+            const uint32_t dx0 = i8_desc(su32(sm));
+            uint32_t parity = 1;  // of acc_empty; the first wait passes
+            bool ok = true;
+            I8Tile T = i8_tile(S, blockIdx.x);
+            for (int ti = blockIdx.x; ti < S.ntiles && ok; ti += gridDim.x) {
+                const int N = T.n, nkb = T.nkb;
+                T = i8_tile(S, ti + gridDim.x);  // read while this tile's MMAs run
+#define DDFMM_I8_PHASE(n, ph) i8_phase<n, ph>(tmem, dx0, nkb, R, full, empty, &acc_full, failed, wait_ns)
+#define DDFMM_I8_CASE(n) \
+    case n: ok = ph == 0 ? DDFMM_I8_PHASE(n, 0) : DDFMM_I8_PHASE(n, 1); break;
+                for (int ph = 0; ph < 2 && ok; ++ph) {
+                    ok = bar_wait(&acc_empty, parity, failed, wait_ns);
+                    parity ^= 1;
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                    switch (N) {
+                        DDFMM_I8_CASE(112)
+                        DDFMM_I8_CASE(96)
+                        DDFMM_I8_CASE(80)
+                        DDFMM_I8_CASE(64)
+                        DDFMM_I8_CASE(48)
+                        DDFMM_I8_CASE(32)
+                        DDFMM_I8_CASE(16)
+                    }
+                }
+#undef DDFMM_I8_CASE
+#undef DDFMM_I8_PHASE
+            }
+            if (!ok) {  // let the MMAs already issued finish before TMEM is freed
+                *failed = 1;
+                i8_commit(&drained);
+                bar_wait(&drained, 0, nullptr, wait_ns);
+            }
+        }
+    } else {
+        reg_inc<208>();
+        // ------------------------------------------------ epilogue
+        const int ew = warp - 8, qw = warp & 3, half = ew >> 2;
+        unsigned char* park = sm + ISTAGES * I_STAGE_BYTES + ew * I_PARK_WARP;
+        unsigned char* mine = park + lane * IPS;
+        int q = 0;
+        // a tile's column (granule, output element) and scale are read one tile ahead
+        I8Tile T = i8_tile(S, blockIdx.x);
+        const int col = qw * 32 + lane;
+        double c = 0.0;
+        long long yo = 0;
+        if (col < T.ncol) {
+            c = __ldg(S.cx + __ldg(S.xgran + T.col + col));
+            yo = __ldg(S.yoff + T.col + col);
+        }
+        for (int ti = blockIdx.x; ti < S.ntiles; ti += gridDim.x) {
+            const I8Tile Tn = i8_tile(S, ti + gridDim.x);
+            const int hN = T.n >> 1;  // this warp's accumulator columns: half hN .. (half + 1) hN
+            double2* y = col < T.ncol ? S.Y + yo + T.row0 + half * (hN >> 1) : nullptr;
+            const uint32_t base = tmem + ((uint32_t)(qw * 32) << 16) + (uint32_t)(half * hN);
+            double v[ICHUNKS * ICH];
+            if (!warp_wait(&acc_full, q & 1, failed, wait_ns)) {
+                *failed = 1;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            // diagonals 4 .. 7 (at most 50 bits), in units of diagonal 7; the loads of a
+            // chunk are in flight while the previous one is joined
+            int d[2][4][8];
+            tmem_ld4(base, T.n, d[0]);
+#pragma unroll
+            for (int ch = 0; ch < ICHUNKS; ++ch)
+                if (ch * ICH < hN) {
+                    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+                    if (ch + 1 < ICHUNKS && (ch + 1) * ICH < hN) tmem_ld4(base + (ch + 1) * ICH, T.n, d[(ch + 1) & 1]);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                        v[ch * ICH + e] = join4(d[ch & 1][0][e], d[ch & 1][1][e], d[ch & 1][2][e], d[ch & 1][3][e]);
+                }
+            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+            __syncwarp();
+            if (lane == 0) bar_arrive(&acc_empty);
+            ++q;
+            if (!warp_wait(&acc_full, q & 1, failed, wait_ns)) {
+                *failed = 1;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            // diagonals 0 .. 3 in units of diagonal 3, then both parts in one rounding
+            tmem_ld4(base, T.n, d[0]);
+#pragma unroll
+            for (int ch = 0; ch < ICHUNKS; ++ch)
+                if (ch * ICH < hN) {
+                    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+                    if (ch + 1 < ICHUNKS && (ch + 1) * ICH < hN) tmem_ld4(base + (ch + 1) * ICH, T.n, d[(ch + 1) & 1]);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                        v[ch * ICH + e] = fma(v[ch * ICH + e], 0x1p-32,
+                                              join4(d[ch & 1][0][e], d[ch & 1][1][e], d[ch & 1][2][e], d[ch & 1][3][e]));
+                }
+            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+            __syncwarp();
+            if (lane == 0) bar_arrive(&acc_empty);
+            ++q;
+            int gn = 0;
+            if (col < Tn.ncol) {
+                gn = __ldg(S.xgran + Tn.col + col);
+                yo = __ldg(S.yoff + Tn.col + col);
+            }
+            // scale, park, add: rows of this half tile, IPR at a time
+            const int r0 = half * (hN >> 1), nr = min(hN >> 1, (int)T.rows - r0);
+            const double* ra = T.ra + r0;
+#pragma unroll
+            for (int b = 0; b < ICHUNKS * ICH / 2; b += IPR) {
+                if (b < nr) {
+                    asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");  // this lane's last piece was read
+#pragma unroll
+                    for (int i = 0; i < IPR; ++i)
+                        if (b + i < ICHUNKS * ICH / 2 && b + i < nr) {
+                            const double f = __ldg(ra + b + i);
+                            *reinterpret_cast<double2*>(mine + i * 16) =
+                                make_double2(v[2 * (b + i)] * f * c, v[2 * (b + i) + 1] * f * c);
+                        }
+                    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                    if (y)
+                        asm volatile(
+                            "cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f64 [%0], [%1], %2;\n" ::"l"(y + b),
+                            "r"(su32(mine)), "r"(min(IPR, nr - b) * 16)
+                            : "memory");
+                    asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+                }
+            }
+            T = Tn;
+            if (col < T.ncol) c = __ldg(S.cx + gn);
+        }
+        asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");
+    }
+    __syncthreads();
+    if (*failed && tid == 0) {
+        // bounded drain of operator copies still in flight, then report
+        const unsigned long long t0 = i8_timer();
+        while (i8_timer() - t0 < 200000ull) __nanosleep(1000);
+        atomicExch(err, 1);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512) : "memory");
+}
+
+static int g_i8_sms = 0;
+
+void i8_init() {
+    cudaFuncSetAttribute(i8_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, I_SMEM);
+    // the register split (2 x 48 + 2 x 208 a thread) needs what the block was launched with
+    cudaFuncAttributes a;
+    if (cudaFuncGetAttributes(&a, i8_gemm_kernel) == cudaSuccess && a.numRegs * ITHREADS < 128 * (2 * 48 + 2 * 208))
+        throw std::runtime_error("int8 GEMM kernel built with too few registers for its register split");
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&g_i8_sms, cudaDevAttrMultiProcessorCount, dev);
+}
+
+void launch_i8_gemm(const I8Sub& S, int* err, cudaStream_t s) {
+    if (S.ntiles == 0) return;
+    const int sms = g_i8_sms > 0 ? g_i8_sms : 148;
+    i8_gemm_kernel<<<S.ntiles < sms ? S.ntiles : sms, ITHREADS, I_SMEM, s>>>(S, err, I_WAIT_NS);
+}
+
+}  // namespace ddfmm

@@ -201,7 +201,22 @@ Session::~Session() {
 
 void Session::add_gemm(std::vector<GemmProblem>& probs, std::vector<std::vector<long long> >& xo,
                        std::vector<std::vector<long long> >& yo, const double2* X, double2* Y, int mode,
-                       const char* label) {
+                       const char* label, const Digits* dg, const std::vector<char>* on_i8) {
+    if (on_i8 && !on_i8->empty()) {  // the problems chosen for the int8 path, then the others
+        std::vector<GemmProblem> big, small;
+        std::vector<std::vector<long long> > bx, by, sx, sy;
+        for (size_t i = 0; i < probs.size(); ++i) {
+            const bool b = (*on_i8)[i];
+            (b ? big : small).push_back(probs[i]);
+            (b ? bx : sx).push_back(std::move(xo[i]));
+            (b ? by : sy).push_back(std::move(yo[i]));
+        }
+        i8_target_ = dg;
+        add_gemm(big, bx, by, X, Y, mode, label);
+        i8_target_ = nullptr;
+        add_gemm(small, sx, sy, X, Y, mode, label);
+        return;
+    }
     struct Clock {
         double& acc;
         std::chrono::steady_clock::time_point t0 = std::chrono::steady_clock::now();
@@ -251,6 +266,14 @@ void Session::add_gemm(std::vector<GemmProblem>& probs, std::vector<std::vector<
     st.label = label;
     st.flops = flops;
     st.bytes = bytes;
+    if (i8_target_) {
+        st.label = width_label((std::string(label).substr(0, std::string(label).rfind("_w")) + "_i8").c_str(),
+                               std::atof(label + std::string(label).rfind("_w") + 2));
+        add_i8(P, xs.get(), ys.get(), ncols, Y, *i8_target_, st);
+        push_step(st);
+        stats_.gemm_launches++;
+        return;
+    }
     if (umma()) {
         add_umma(P, xs.get(), ys.get(), ncols, X, Y, mode, st);
         push_step(st);
@@ -333,6 +356,84 @@ void Session::add_umma(const std::vector<GemmProblem>& P, const long long* xs, c
     st.hu = UmmaSub{upload(U), upload(tiles), upload_n(xs, ncols), upload_n(ys, ncols), reinterpret_cast<const float2*>(X),
                     reinterpret_cast<float2*>(Y), (int)tiles.size(), mode, 0, 0};
     set_multi(st, st.hu, (int)tiles.size());
+}
+
+// Which problems (m, k, columns) of a plain-form launch run on the int8 path;
+// empty when none.  In clocks of one SM, fitted to launches of the K = 8 .. 64
+// workloads: an int8 tile (128 columns x up to 56 rows, full or not) costs 10500
+// and 2700 a K block (k = 76: 24 k, k = 152: 37 k); the FP64 tensor path does 11
+// complex products a clock with many columns, 8 with few.  So 128 columns of a
+// 100 x 152 operator cost 75 k against 177 k, 32 columns 75 k against 61 k.  The
+// launch must gain what its digits, its second launch and its last wave cost:
+// at K = 8, P = 4 a gain of 24 us an SM by this count is a loss of 30 us (0.435
+// ms on the FP64 path alone, 0.465 ms with the M2L problems split off).
+static std::vector<char> i8_choose(const std::vector<std::array<int, 3> >& shapes) {
+    std::vector<char> on(shapes.size(), 0);
+    double gain = 0;
+    for (size_t i = 0; i < shapes.size(); ++i) {
+        const double m = shapes[i][0], k = shapes[i][1], c = shapes[i][2];
+        const double t8 = std::ceil(c / 128) * i8_row_tiles(shapes[i][0]) * (10500 + 2700 * std::ceil(k / 16));
+        const double t64 = m * k * c / (c < 96 ? 8 : 11);
+        if (t8 < t64) {
+            on[i] = 1;
+            gain += t64 - t8;
+        }
+    }
+    if (gain < 148 * 60e3) on.clear();
+    return on;
+}
+
+// int8 form of one grouped GEMM launch: the operators packed as digits (now: they
+// are on the device).
+void Session::add_i8(const std::vector<GemmProblem>& P, const long long* xs, const long long* ys, size_t ncols,
+                     double2* Y, const Digits& dg, Step& st) {
+    std::vector<I8PackJob> jobs;
+    std::vector<I8Tile> tiles;
+    size_t bytes = 0, rows = 0;
+    int max_tiles = 1;
+    for (const GemmProblem& q : P) {
+        bytes += i8_packed_bytes(q.m, q.k);
+        rows += q.m;
+        max_tiles = std::max(max_tiles, i8_row_tiles(q.m));
+    }
+    char* B = dalloc<char>(bytes);
+    double* ra = dalloc<double>(rows);
+    for (size_t i = 0; i < P.size(); ++i) {
+        const GemmProblem& q = P[i];
+        jobs.push_back(I8PackJob{q.A, B, ra, q.m, q.k, q.lda, (q.k + 15) / 16, i8_tile_rows(q.m)});
+        i8_tiles(B, ra, q.m, q.k, q.col0, q.ncol, tiles);
+        B += i8_packed_bytes(q.m, q.k);
+        ra += q.m;
+    }
+    std::vector<int> xg(ncols);
+    host_parallel_for((ncols + 65535) / 65536, [&](size_t c) {
+        for (size_t j = c * 65536; j < std::min(ncols, (c + 1) * 65536); ++j)
+            xg[j] = (int)((xs[j] - dg.base) / dg.unit) * dg.gran;
+    });
+    if (!d_err_) {
+        d_err_ = dalloc<int>(1);
+        CK(cudaMemsetAsync(d_err_, 0, sizeof(int), stream_));
+    }
+    const I8PackJob* dj = upload(jobs);
+    flush_uploads();
+    launch_i8_pack(dj, (int)jobs.size(), max_tiles, stream_);
+    CK(cudaGetLastError());
+    st.kind = 8;
+    st.i8 = I8Sub{upload(tiles), upload(xg), upload_n(ys, ncols), dg.X8, dg.cx, Y, (int)tiles.size()};
+}
+
+// The digits of the given vectors of X, for the int8 GEMMs that gather them.
+void Session::add_digits(const std::vector<I8Vec>& vecs, const double2* X, const Digits& dg, const char* label) {
+    Step st{};
+    st.kind = 7;
+    st.label = label;
+    for (const I8Vec& v : vecs) st.bytes += 30.0 * v.len;
+    st.dg.vecs = upload(vecs);
+    st.dg.n = (int)vecs.size();
+    st.dg.X = X;
+    st.dg.X8 = dg.X8;
+    st.dg.cx = dg.cx;
+    push_step(st);
 }
 
 template <class Sub>
@@ -443,40 +544,40 @@ namespace {
 // columns of B (read from pool X) and of C (written to pool Y).
 struct GemmBatch {
     std::vector<GemmProblem> probs;
-    std::vector<long long> xs, ys;
+    std::vector<ColumnSpan> spans;  // the columns of each problem, listed on the device
+    long long ncols = 0;
     // A (m x k, lda m, device pointer), B = X[bx ..] (k x n), C = Y[cy ..] (m x n)
     void product(const double2* A, int m, int k, size_t bx, int n, size_t cy) {
-        GemmProblem p{A, m, k, m, (int)xs.size(), n};
-        for (int j = 0; j < n; ++j) {
-            xs.push_back((long long)(bx + (size_t)j * k));
-            ys.push_back((long long)(cy + (size_t)j * m));
-        }
-        probs.push_back(p);
+        probs.push_back(GemmProblem{A, m, k, m, (int)ncols, n, nullptr});
+        spans.push_back(ColumnSpan{ncols, (long long)bx, (long long)cy, k, m});
+        ncols += n;
     }
     void run(const double2* X, double2* Y, cudaStream_t s) {
         if (probs.empty()) return;
+        if (ncols > INT_MAX) throw std::runtime_error("too many operator columns in one setup launch");
         std::vector<GemmTile> tiles;
         for (size_t i = 0; i < probs.size(); ++i)
             for (int r0 = 0; r0 < probs[i].m; r0 += GEMM_TILE_M)
                 for (int c0 = 0; c0 < probs[i].ncol; c0 += GEMM_TILE_N) tiles.push_back(GemmTile{(int)i, r0, c0, 0});
         GemmProblem* dp;
         GemmTile* dt;
-        long long *dx, *dy;
+        ColumnSpan* ds;
+        long long* dx;
         CK(cudaMalloc(&dp, sizeof(GemmProblem) * probs.size()));
         CK(cudaMalloc(&dt, sizeof(GemmTile) * tiles.size()));
-        CK(cudaMalloc(&dx, sizeof(long long) * xs.size()));
-        CK(cudaMalloc(&dy, sizeof(long long) * ys.size()));
+        CK(cudaMalloc(&ds, sizeof(ColumnSpan) * spans.size()));
+        CK(cudaMalloc(&dx, 2 * sizeof(long long) * (size_t)ncols));
         CK(cudaMemcpyAsync(dp, probs.data(), sizeof(GemmProblem) * probs.size(), cudaMemcpyHostToDevice, s));
         CK(cudaMemcpyAsync(dt, tiles.data(), sizeof(GemmTile) * tiles.size(), cudaMemcpyHostToDevice, s));
-        CK(cudaMemcpyAsync(dx, xs.data(), sizeof(long long) * xs.size(), cudaMemcpyHostToDevice, s));
-        CK(cudaMemcpyAsync(dy, ys.data(), sizeof(long long) * ys.size(), cudaMemcpyHostToDevice, s));
-        launch_gemm(dp, dt, (int)tiles.size(), dx, dy, X, Y, GEMM_SET, s);
+        CK(cudaMemcpyAsync(ds, spans.data(), sizeof(ColumnSpan) * spans.size(), cudaMemcpyHostToDevice, s));
+        launch_list_columns(ds, (int)spans.size(), ncols, dx, dx + ncols, s);
+        launch_gemm(dp, dt, (int)tiles.size(), dx, dx + ncols, X, Y, GEMM_SET, s);
         CK(cudaGetLastError());
         CK(cudaStreamSynchronize(s));
         cudaFree(dp);
         cudaFree(dt);
+        cudaFree(ds);
         cudaFree(dx);
-        cudaFree(dy);
     }
 };
 
@@ -817,6 +918,9 @@ void Session::build() {
     for (int b : T.order)
         if (T.boxes[b].has_pts() && T.width(T.boxes[b].level) > 1 - eps) hflevels[T.boxes[b].level].push_back(b);
 
+    // node vectors start at multiples of 16 complex numbers: the granules of the
+    // int8 GEMM's digits, and aligned 128-byte (64-byte) pieces for the others
+    auto node_stride = [](int r) { return (long long)((r + 15) & ~15); };
     // nodes of a box are contiguous and in its (sorted) wedge order, so a
     // (box, wedge) node is found by binary search in the box's range (HfNodes::find)
     HfNodes up, dn;
@@ -862,8 +966,8 @@ void Session::build() {
         host_parallel_for(nbx, [&](size_t i) {
             const Box& B = T.boxes[bx[i]];
             long long a = 0, c = 0;
-            for (const Idx3& d : B.outdirs) a += lookup(d).r1;
-            for (const Idx3& d : B.incdirs) c += lookup(d).r1;
+            for (const Idx3& d : B.outdirs) a += node_stride(lookup(d).r1);
+            for (const Idx3& d : B.incdirs) c += node_stride(lookup(d).r1);
             uo[i + 1] = a;
             dof[i + 1] = c;
             un[i + 1] = (int)B.outdirs.size();
@@ -892,7 +996,7 @@ void Session::build() {
             for (const Idx3& d : B.outdirs) {
                 const DirPts& dp = lookup(d);
                 up.v[k++] = HfNode{b, d, dp.canon, o, o, dp.did};  // M2M adds straight into the vector
-                o += dp.r1;
+                o += node_stride(dp.r1);
             }
             dn.first[b] = dnn[i];
             dn.cnt[b] = dnn[i + 1] - dnn[i];
@@ -901,7 +1005,7 @@ void Session::build() {
             for (const Idx3& d : B.incdirs) {
                 const DirPts& dp = lookup(d);
                 dn.v[k++] = HfNode{b, d, dp.canon, o, o, dp.did};  // L2L reads the vector itself
-                o += dp.r1;
+                o += node_stride(dp.r1);
             }
         });
         upeq_total = uo[nbx];
@@ -1261,6 +1365,68 @@ void Session::build() {
     for (int l = 0; l < nLF; ++l) lf_off[lfbox[l]] = (long long)l * nE;
     HfColumns cols = hf_columns(T, up, dn, kids, lf_off, dirpts.size(), hfcanon.size(), false);
     phase("hf_columns");
+    // ---------------------------------------------------------------- digits of the HF inputs
+    // (plain form) of the launches with problems large enough for the int8 path
+    Digits lf_dg, up_dg, dn_dg;
+    std::map<int, std::vector<char> > m2m_i8, m2l_i8, l2l_i8;  // level -> problems on the int8 path
+    std::set<int> up_i8, dn_i8;  // levels whose outgoing / incoming vectors are written as digits
+    bool lf_i8 = false;
+    if (!mixed) {
+        long long dn_most = 0;
+        for (auto& kv : hflevels) {
+            const int level = kv.first;
+            const double W = T.width(level);
+            auto shapes = [&](const ColLists& L, const std::map<std::pair<double, Idx3>, DirMats>& mats) {
+                std::vector<std::array<int, 3> > v;
+                for (size_t i = 0; i < L.key.size(); ++i) {
+                    const DirMats& M = mats.at(std::make_pair(W, did_wedge[L.key[i] / 8].second));
+                    v.push_back({{M.mrows, M.mcols, (int)L.x[i].size()}});
+                }
+                return v;
+            };
+            std::vector<std::array<int, 3> > far;
+            for (size_t i = 0; i < m2l_probs[level].size(); ++i) {
+                const int r1 = m2l_mats[m2l_probs[level][i]].r1;
+                far.push_back({{r1, r1, (int)m2l_x[level][i].size()}});
+            }
+            m2m_i8[level] = i8_choose(shapes(cols.m2m.at(level), m2m_mats));
+            m2l_i8[level] = i8_choose(far);
+            l2l_i8[level] = i8_choose(shapes(cols.l2l.at(level), l2l_mats));
+            if (!m2m_i8[level].empty()) {
+                if (W == 1.0)
+                    lf_i8 = true;
+                else
+                    up_i8.insert(level + 1);
+            }
+            if (!m2l_i8[level].empty()) up_i8.insert(level);
+            if (!l2l_i8[level].empty()) {
+                dn_i8.insert(level);
+                const auto dr = dn.range[level];
+                dn_most = std::max(dn_most, (dr.second == (int)dn.v.size() ? dnchk_total : dn.v[dr.second].off) - dn.v[dr.first].off);
+            }
+        }
+        auto room = [&](Digits& d, size_t granules) {
+            d.X8 = dalloc<char>(granules * I8_GRANULE);
+            d.cx = dalloc<double>(granules);
+        };
+        lf_dg.unit = nE;
+        lf_dg.gran = (nE + 15) / 16;
+        if (lf_i8) room(lf_dg, (size_t)nLF * lf_dg.gran);
+        if (!up_i8.empty()) room(up_dg, (size_t)upeq_total / 16);
+        if (!dn_i8.empty()) room(dn_dg, (size_t)dn_most / 16);
+        if (lf_i8 || !up_i8.empty() || !dn_i8.empty()) i8_init();
+    }
+    auto node_vecs = [&](const HfNodes& N, int level, const Digits& d) {
+        const auto r = N.range.at(level);
+        std::vector<I8Vec> v((size_t)(r.second - r.first));
+        host_parallel_for((v.size() + 16383) / 16384, [&](size_t c) {
+            for (size_t i = c * 16384; i < std::min(v.size(), (c + 1) * 16384); ++i) {
+                const HfNode& u = N.v[r.first + i];
+                v[i] = I8Vec{u.off, (int)((u.off - d.base) / 16), hfcanon[u.canon].r1};
+            }
+        });
+        return v;
+    };
     // ---------------------------------------------------------------- steps: HF upward
     // widths ascending = levels descending; hf_upeq holds w (upeqnden = E1 w)
     for (auto hit = hflevels.rbegin(); hit != hflevels.rend(); ++hit) {
@@ -1269,6 +1435,11 @@ void Session::build() {
         auto ur = up.range[level];
         if (ur.first == ur.second) continue;
         begin_block(1, W);
+        if (W == 1.0 && lf_i8) {
+            std::vector<I8Vec> v;
+            for (int l : lflevels[level + 1]) v.push_back(I8Vec{(long long)l * nE, l * lf_dg.gran, nE});
+            add_digits(v, lf_upeq, lf_dg, "lf_digits");
+        }
         // M2M: w = sum_children [E2 E3 ue2uc E1(child)] w_child (src/wave3d_eval.cpp:796-849),
         // one launch for the 8 child positions: a problem per (wedge, child), all adding into
         // the parents' vectors
@@ -1286,8 +1457,10 @@ void Session::build() {
                     if (!opctx_.empty()) opkey_[KP(M.fin[ind])] = opk("m2m", W, dir, ind);
                 }
             }
-            add_gemm(probs, L.x, L.y, W == 1.0 ? lf_upeq : hf_upeq, hf_upeq, GEMM_ATOMIC, width_label("hf_m2m", W));
+            add_gemm(probs, L.x, L.y, W == 1.0 ? lf_upeq : hf_upeq, hf_upeq, GEMM_ATOMIC, width_label("hf_m2m", W),
+                     W == 1.0 ? &lf_dg : &up_dg, &m2m_i8[level]);
         }
+        if (up_i8.count(level)) add_digits(node_vecs(up, level, up_dg), hf_upeq, up_dg, "hf_digits_up");
     }
 
     phase("steps_hf_up");
@@ -1311,7 +1484,12 @@ void Session::build() {
                     if (!opctx_.empty()) opkey_[KP(M.fin)] = M.key;
                 }
             }
-            add_gemm(probs, m2l_x[level], m2l_y[level], hf_upeq, hf_dnchk, GEMM_ATOMIC, width_label("hf_m2l", W));
+            add_gemm(probs, m2l_x[level], m2l_y[level], hf_upeq, hf_dnchk, GEMM_ATOMIC, width_label("hf_m2l", W), &up_dg,
+                     &m2l_i8[level]);
+        }
+        if (dn_i8.count(level)) {
+            dn_dg.base = dn.v[dr.first].off;  // one level's digits at a time
+            add_digits(node_vecs(dn, level, dn_dg), hf_dnchk, dn_dg, "hf_digits_down");
         }
         // L2L into the children's (pdir) u, or LF dnchkval at W=1 (src/wave3d_eval.cpp:938-991),
         // one launch for the 8 child positions: a problem per (wedge, child)
@@ -1329,7 +1507,8 @@ void Session::build() {
                     if (!opctx_.empty()) opkey_[KP(M.fin[ind])] = opk("l2l", W, dir, ind);
                 }
             }
-            add_gemm(probs, L.x, L.y, hf_dnchk, W == 1.0 ? lf_dnchk : hf_dnchk, GEMM_ATOMIC, width_label("hf_l2l", W));
+            add_gemm(probs, L.x, L.y, hf_dnchk, W == 1.0 ? lf_dnchk : hf_dnchk, GEMM_ATOMIC, width_label("hf_l2l", W),
+                     &dn_dg, &l2l_i8[level]);
         }
     }
 
@@ -1569,6 +1748,8 @@ static const char* kernel_name(int kind, int tpi) {
         case 2: return "vlist_forward_kernel";
         case 3: return "vlist_group_kernel";
         case 6: return "vlist_inverse_kernel";
+        case 7: return "i8_slice_kernel";
+        case 8: return "i8_gemm_kernel";
         default: return "umma_cgemm_kernel";
     }
 }
@@ -1609,6 +1790,8 @@ void Session::launch_step(const Step& st, cudaStream_t s, double2* spec) {
             else
                 launch_vlist_inverse(st.v.L, st.v.trg, st.v.ntrg, st.v.tsp, st.v.dnchk, s);
             break;
+        case 7: launch_i8_slice(st.dg.vecs, st.dg.n, st.dg.X, st.dg.X8, st.dg.cx, s); break;
+        case 8: launch_i8_gemm(st.i8, d_err_, s); break;
         case 5: {
             const unsigned long long wait_ns = stall_wait_ns_;
             stall_wait_ns_ = 0;  // one launch only

@@ -122,15 +122,33 @@ private:
         void* p;
         size_t bytes;
     };
+    struct DigitsLaunch {
+        const I8Vec* vecs = nullptr;
+        int n = 0;
+        const double2* X = nullptr;
+        char* X8 = nullptr;
+        double* cx = nullptr;
+    };
+    // The digits of a GEMM launch's input array: element offset o of a vector is
+    // granule (o - base) / unit * gran of X8.
+    struct Digits {
+        char* X8 = nullptr;
+        double* cx = nullptr;
+        long long base = 0;
+        int unit = 16, gran = 1;
+    };
     // one step of the eval: exactly one of these is used
     struct Step {
-        int kind;  // 0 gemm, 1 pt, 2 vfwd, 3 V-list sums, 5 tcgen05 gemm, 6 V-list inverse
+        int kind;  // 0 gemm, 1 pt, 2 vfwd, 3 V-list sums, 5 tcgen05 gemm, 6 V-list inverse,
+                   // 7 digits of vectors, 8 int8 tcgen05 gemm
         const char* label;  // pass name for profiling
         double flops;       // algorithmic flops of the launch
         double bytes;       // algorithmic DRAM bytes of the launch
         GemmLaunch g;
         PtLaunch pt;
         VLaunch v;
+        I8Sub i8;
+        DigitsLaunch dg;
         // Position of the step in the pass structure, equal across sessions for steps
         // that play the same part (phase, width, step type, occurrence): a Batch
         // merges the steps of its sessions that share a key into one launch.
@@ -170,7 +188,11 @@ private:
     void dfree(const void* p);  // release one allocation made by dalloc / a large upload
     void add_gemm(std::vector<GemmProblem>& probs, std::vector<std::vector<long long> >& xo,
                   std::vector<std::vector<long long> >& yo, const double2* X, double2* Y, int mode,
-                  const char* label);
+                  const char* label, const Digits* dg = nullptr, const std::vector<char>* on_i8 = nullptr);
+    const Digits* i8_target_ = nullptr;  // set while add_gemm emits the int8 part of a launch
+    void add_i8(const std::vector<GemmProblem>& P, const long long* xs, const long long* ys, size_t ncols, double2* Y,
+                const Digits& dg, Step& st);
+    void add_digits(const std::vector<I8Vec>& vecs, const double2* X, const Digits& dg, const char* label);
     const float* packed_operator(const GemmProblem& q);
     void add_umma(const std::vector<GemmProblem>& P, const long long* xs, const long long* ys, size_t ncols,
                   const double2* X, double2* Y, int mode, Step& st);

@@ -162,6 +162,13 @@ int ddfmm_precompute_operators(int kernel, int accu, int wmax, int threads, cons
  * context stays usable.  DDFMM_EINVAL on other sessions. */
 int ddfmm_session_test_gemm_stall(ddfmm_session* s, double wait_s);
 
+/* Test entry point, no counterpart in the reference: Y += A X (A m x k, X k x
+ * ncol, Y m x ncol, column-major complex128 host arrays; m, k <= 400) on the
+ * current device through a translation kernel of the PLAIN_FP64 form -- path
+ * 0: the FP64 tensor path, 1: the int8 tensor path (exact integer products of
+ * digit planes).  Columns are gathered and scattered as an eval's are. */
+int ddfmm_test_gemm(const double* A, int m, int k, const double* X, int ncol, int path, double* Y);
+
 /* Host-only (no GPU): build the octree and interaction lists of
  * Wave3d::setup (src/wave3d_setup.cpp:100-299) and report, per level, what
  * Wave3d::eval prints about them (src/wave3d_eval.cpp:345-372): boxes with
