@@ -1322,21 +1322,25 @@ void Session::build() {
             items.push_back(itm);
         }
         add_pt(items, srcs, "lf_s2m");
-        // M2M from children (src/wave3d_eval.cpp:452-463)
-        if (L.has_children)
+        // M2M from children (src/wave3d_eval.cpp:452-463) and, further down, L2L to them:
+        // one launch for the 8 child positions, a problem each (an adaptive tree has many
+        // levels of few boxes: 8 launches a level were half of such an eval's)
+        if (L.has_children) {
+            std::vector<GemmProblem> probs;
+            std::vector<std::vector<long long> > x(8), y(8);
             for (int ind = 0; ind < 8; ++ind) {
-                std::vector<long long> x, y;
+                probs.push_back(GemmProblem{opm(L.ue2uc[ind], (size_t)nE * nE), nE, nE, nE, 0, 0});
                 for (int l : ids) {
                     int b = lfbox[l];
                     if (T.boxes[b].terminal()) continue;
                     int c = T.child(b, ind);
                     if (c < 0 || !T.boxes[c].has_pts()) continue;
-                    x.push_back((long long)lfidx[c] * nE);
-                    y.push_back((long long)l * nE);
+                    x[ind].push_back((long long)lfidx[c] * nE);
+                    y[ind].push_back((long long)l * nE);
                 }
-                single(GemmProblem{opm(L.ue2uc[ind], (size_t)nE * nE), nE, nE, nE, 0, 0}, x, y, lf_upeq, lf_upchk, GEMM_ADD,
-                       "lf_m2m");
             }
+            add_gemm(probs, x, y, lf_upeq, lf_upchk, GEMM_ATOMIC, "lf_m2m");  // siblings add into one parent
+        }
         // upeqnden = v * (1/sigma .* (U^H * upchk))   (src/wave3d_eval.cpp:466-478)
         std::vector<long long> a, b2;
         for (int l : ids) {
@@ -1686,20 +1690,22 @@ void Session::build() {
             add_pt(items, srcs, "lf_l2t");
         }
         // L2L to the children (src/wave3d_eval.cpp:562-579)
-        if (L.has_children)
+        if (L.has_children) {
+            std::vector<GemmProblem> probs;
+            std::vector<std::vector<long long> > x(8), y(8);
             for (int ind = 0; ind < 8; ++ind) {
-                std::vector<long long> x, y;
+                probs.push_back(GemmProblem{opm(L.de2dc[ind], (size_t)nE * nE), nE, nE, nE, 0, 0});
                 for (int l : ids) {
                     int b = lfbox[l];
                     if (T.boxes[b].terminal()) continue;
                     int c = T.child(b, ind);
                     if (c < 0 || !T.boxes[c].has_pts()) continue;
-                    x.push_back((long long)l * nE);
-                    y.push_back((long long)lfidx[c] * nE);
+                    x[ind].push_back((long long)l * nE);
+                    y[ind].push_back((long long)lfidx[c] * nE);
                 }
-                single(GemmProblem{opm(L.de2dc[ind], (size_t)nE * nE), nE, nE, nE, 0, 0}, x, y, lf_dneq, lf_dnchk, GEMM_ADD,
-                       "lf_l2l");
             }
+            add_gemm(probs, x, y, lf_dneq, lf_dnchk, GEMM_ADD, "lf_l2l");  // every child has one parent
+        }
     }
     phase("steps_lf_down");
     if (trace)
