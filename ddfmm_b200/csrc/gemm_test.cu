@@ -59,6 +59,14 @@ void test_gemm(const double2* A, int m, int k, const double2* X, int ncol, int p
         gemm_init();
         launch_gemm(P.put(std::vector<GemmProblem>(1, GemmProblem{dA, m, k, m, 0, ncol, nullptr})), P.put(tiles),
                     (int)tiles.size(), P.put(xo), dyo, dX, dY, GEMM_ATOMIC, nullptr);
+    } else if (path == 2) {
+        const int rows = m > 64 ? 128 : 64;
+        std::vector<GemmTile> tiles;
+        for (int r = 0; r < m; r += rows)
+            for (int c = 0; c < ncol; c += 8) tiles.push_back(GemmTile{0, r, c, 0});
+        gemm_init();
+        launch_gemm_narrow(P.put(std::vector<GemmProblem>(1, GemmProblem{dA, m, k, m, 0, ncol, nullptr})), P.put(tiles),
+                           (int)tiles.size(), P.put(xo), dyo, dX, dY, GEMM_ATOMIC, k, rows, nullptr);
     } else {
         const int nkb = (k + 15) / 16;
         char* B = P.put(std::vector<char>(i8_packed_bytes(m, k)));

@@ -328,14 +328,109 @@ __global__ void __launch_bounds__(256, DDFMM_ZGEMM_MINB) zgemm_kernel(const Gemm
         }
 }
 
-void gemm_init() {
-    cudaFuncSetAttribute(zgemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM);
-}
-
 void launch_gemm(const GemmProblem* probs, const GemmTile* tiles, int ntiles, const long long* xoff,
                  const long long* yoff, const double2* X, double2* Y, int mode, cudaStream_t s) {
     if (ntiles == 0) return;
     zgemm_kernel<<<ntiles, 256, GEMM_SMEM, s>>>(probs, tiles, xoff, yoff, X, Y, mode);
+}
+
+// Products with few columns: the operator is read once and hardly reused, so what
+// counts is bytes of it in flight.  zgemm_kernel stages it through shared memory
+// in 16-wide slices beside 64 columns, mostly zeros then, with a block barrier a
+// slice.  Here a tile is `blockDim / 2` operator rows x 8 columns; a warp owns 16
+// rows and reads its MMA fragments straight from memory into registers, one
+// 8-wide K step ahead (a fragment load is four 128-byte pieces of operator
+// columns), and 24 warps an SM keep the loads coming.  Only the gathered columns
+// go through shared memory, all of k at once, one barrier a block; they stand
+// kp = 8-multiple + 4 apart, which makes the fragment reads conflict-free as in
+// zgemm_kernel.  Column tiles of the same rows are adjacent and share the
+// operator in L2.  Measured, operators cold, 768 of 150 x 296 (546 MB): 8 columns
+// 258 -> 133 us (4.1 TB/s); deeper prefetch with fewer warps is slower (two steps
+// and 16 warps 195 us, four and 8 warps 317 us), and so are tiles of 16 columns
+// (registers).
+__global__ void __launch_bounds__(256, 3) zgemm_narrow_kernel(const GemmProblem* __restrict__ probs,
+                                                              const GemmTile* __restrict__ tiles,
+                                                              const long long* __restrict__ xoff,
+                                                              const long long* __restrict__ yoff,
+                                                              const double2* __restrict__ X, double2* Y, int mode) {
+    extern __shared__ double2 nsm[];
+    const GemmTile t = tiles[blockIdx.x];
+    const GemmProblem p = probs[t.prob];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tig = lane & 3;
+    const int ncol = min(8, p.ncol - t.col0);
+    const int ksteps = (p.k + 7) >> 3, kp = ksteps * 8 + 4;
+    const int row = t.row0 + warp * 16 + g;  // rows row and row + 8 of the operator
+    const bool r0 = row < p.m, r1 = row + 8 < p.m, work = t.row0 + warp * 16 < p.m;
+    const double2 zero = make_double2(0.0, 0.0);
+    double2 a[4];
+    auto load = [&](int step) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int k = step * 8 + tig + 4 * (q >> 1);
+            const bool ok = k < p.k && ((q & 1) ? r1 : r0);
+            a[q] = ok ? __ldg(p.A + (size_t)k * p.lda + row + 8 * (q & 1)) : zero;
+        }
+    };
+    if (work) load(0);
+    // the tile's columns, zeros past the last one and past k
+    for (int c = warp; c < 8; c += blockDim.x >> 5) {
+        const double2* x = c < ncol ? X + xoff[p.col0 + t.col0 + c] : nullptr;
+        for (int k = lane; k < ksteps * 8; k += 32) nsm[c * kp + k] = x && k < p.k ? x[k] : zero;
+    }
+    __syncthreads();
+    if (!work) return;
+    double cr[4] = {0.0, 0.0, 0.0, 0.0}, ci[4] = {0.0, 0.0, 0.0, 0.0}, cs[4] = {0.0, 0.0, 0.0, 0.0};
+    const double2* Xs = nsm + g * kp + tig;
+    for (int s = 0; s < ksteps; ++s) {
+        double ar[4], ai[4], as[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            ar[q] = a[q].x;
+            ai[q] = a[q].y;
+            as[q] = a[q].x + a[q].y;
+        }
+        load(s + 1);  // zeros past k
+        const double2 b0 = Xs[s * 8], b1 = Xs[s * 8 + 4];
+        const double br[2] = {b0.x, b1.x}, bi[2] = {b0.y, b1.y}, bs[2] = {b0.x + b0.y, b1.x + b1.y};
+        dmma16(cr, ar, br);
+        dmma16(ci, ai, bi);
+        dmma16(cs, as, bs);
+    }
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const int col = 2 * tig + e;
+        if (col >= ncol) continue;
+        double2* y = Y + yoff[p.col0 + t.col0 + col];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int rr = row + 8 * i, q = 2 * i + e;
+            if (rr >= p.m) continue;
+            const double2 v = make_double2(cr[q] - ci[q], cs[q] - cr[q] - ci[q]);
+            if (mode == GEMM_SET) {
+                y[rr] = v;
+            } else if (mode == GEMM_ADD) {
+                const double2 o = y[rr];
+                y[rr] = make_double2(o.x + v.x, o.y + v.y);
+            } else {
+                atomicAdd(&y[rr].x, v.x);
+                atomicAdd(&y[rr].y, v.y);
+            }
+        }
+    }
+}
+
+void gemm_init() {
+    cudaFuncSetAttribute(zgemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM);
+    cudaFuncSetAttribute(zgemm_narrow_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, NARROW_SMEM);
+}
+
+size_t narrow_smem(int k) { return sizeof(double2) * 8 * ((size_t)(k + 7) / 8 * 8 + 4); }
+
+void launch_gemm_narrow(const GemmProblem* probs, const GemmTile* tiles, int ntiles, const long long* xoff,
+                        const long long* yoff, const double2* X, double2* Y, int mode, int kmax, int rows,
+                        cudaStream_t s) {
+    if (ntiles == 0) return;
+    zgemm_narrow_kernel<<<ntiles, rows * 2, narrow_smem(kmax), s>>>(probs, tiles, xoff, yoff, X, Y, mode);
 }
 
 // ---------------------------------------------------------------- points

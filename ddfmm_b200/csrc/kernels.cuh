@@ -70,6 +70,13 @@ void launch_list_columns(const ColumnSpan* spans_dev, int nspans, long long ncol
 void launch_gemm(const GemmProblem* probs_dev, const GemmTile* tiles_dev, int ntiles,
                  const long long* xoff, const long long* yoff, const double2* X, double2* Y, int mode,
                  cudaStream_t s);
+// Products with few columns: tiles of `rows` (64 or 128) operator rows x 8 columns; kmax: the
+// launch's longest k, narrow_smem(kmax) <= NARROW_SMEM.
+constexpr int NARROW_SMEM = 72 << 10;
+size_t narrow_smem(int k);
+void launch_gemm_narrow(const GemmProblem* probs_dev, const GemmTile* tiles_dev, int ntiles, const long long* xoff,
+                        const long long* yoff, const double2* X, double2* Y, int mode, int kmax, int rows,
+                        cudaStream_t s);
 // tpi: the launch shape, chosen per step by the session's autotuner: 4, 8, 16 or
 // 32 threads per item, each thread taking targets and walking the sources in
 // global memory; or one warp per item with the item's sources staged in

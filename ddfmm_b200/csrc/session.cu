@@ -222,6 +222,43 @@ void Session::add_gemm(std::vector<GemmProblem>& probs, std::vector<std::vector<
         std::chrono::steady_clock::time_point t0 = std::chrono::steady_clock::now();
         ~Clock() { acc += std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count(); }
     } clock{t_emit_gemm_};
+    // zgemm_narrow_kernel for launches of products with up to 40 columns (operators cold:
+    // 8 columns 0.44-0.6 of zgemm_kernel's time, 24 columns 0.7-0.8, 32 columns 0.8-0.95,
+    // 48 columns 0.95-1.1), for launches whose 64-column tiles would not give every SM a
+    // block (150 columns of 56 x 56: 18 -> 11 us), and for a launch's products of up to
+    // 24 columns where they are enough for a launch of their own
+    bool narrow = narrow_;
+    int kmax = 0, mmax = 0;
+    if (!mixed() && !i8_target_ && !narrow_) {
+        size_t tiles64 = 0, few = 0, many = 0;
+        for (size_t i = 0; i < probs.size(); ++i) {
+            tiles64 += (size_t)((probs[i].m + GEMM_TILE_M - 1) / GEMM_TILE_M) * ((xo[i].size() + GEMM_TILE_N - 1) / GEMM_TILE_N);
+            if (xo[i].size() > 40) ++many;
+            if (!xo[i].empty() && xo[i].size() <= 24) ++few;
+        }
+        if (tiles64 < 148 || many == 0) {
+            narrow = true;
+        } else if (few >= 148) {  // enough for a launch of their own
+            std::vector<GemmProblem> big, small;
+            std::vector<std::vector<long long> > bx, by, sx, sy;
+            for (size_t i = 0; i < probs.size(); ++i) {
+                const bool b = xo[i].size() > 24;
+                (b ? big : small).push_back(probs[i]);
+                (b ? bx : sx).push_back(std::move(xo[i]));
+                (b ? by : sy).push_back(std::move(yo[i]));
+            }
+            narrow_ = true;
+            add_gemm(small, sx, sy, X, Y, mode, label);
+            narrow_ = false;
+            add_gemm(big, bx, by, X, Y, mode, label);
+            return;
+        }
+    }
+    for (size_t i = 0; i < probs.size(); ++i) {
+        kmax = std::max(kmax, probs[i].k);
+        mmax = std::max(mmax, probs[i].m);
+    }
+    const int tile_m = narrow && mmax > 64 ? 128 : GEMM_TILE_M, tile_n = narrow ? 8 : GEMM_TILE_N;
     double flops = 0, bytes = 0;
     std::vector<GemmProblem> P;
     std::vector<size_t> from;  // the caller's problem of each P
@@ -237,8 +274,8 @@ void Session::add_gemm(std::vector<GemmProblem>& probs, std::vector<std::vector<
         P.push_back(q);
         from.push_back(i);
         ncols += (size_t)q.ncol;
-        for (int r0 = 0; r0 < q.m; r0 += GEMM_TILE_M)
-            for (int c0 = 0; c0 < q.ncol; c0 += GEMM_TILE_N) tiles.push_back(GemmTile{pid, r0, c0, 0});
+        for (int r0 = 0; r0 < q.m; r0 += tile_m)
+            for (int c0 = 0; c0 < q.ncol; c0 += tile_n) tiles.push_back(GemmTile{pid, r0, c0, 0});
         flops += 8.0 * q.m * q.k * (double)q.ncol;
         // operator once, each input and output column once (read-modify-write for += modes)
         bytes += 16.0 * ((double)q.m * q.k + (double)q.k * q.ncol + (mode == GEMM_SET ? 1.0 : 2.0) * q.m * q.ncol);
@@ -267,6 +304,7 @@ void Session::add_gemm(std::vector<GemmProblem>& probs, std::vector<std::vector<
     st.flops = flops;
     st.bytes = bytes;
     if (i8_target_) {
+        // a label of its own, so that profiles show the two kernels apart
         st.label = width_label((std::string(label).substr(0, std::string(label).rfind("_w")) + "_i8").c_str(),
                                std::atof(label + std::string(label).rfind("_w") + 2));
         add_i8(P, xs.get(), ys.get(), ncols, Y, *i8_target_, st);
@@ -288,6 +326,8 @@ void Session::add_gemm(std::vector<GemmProblem>& probs, std::vector<std::vector<
     st.g.X = X;
     st.g.Y = Y;
     st.g.mode = mode;
+    st.g.kmax = kmax;
+    st.g.rows = narrow ? tile_m : 0;
     push_step(st);
     stats_.gemm_launches++;
 }
@@ -1737,9 +1777,9 @@ void Session::build() {
     stats_.kernel_launches = (long long)steps_.size() + 2;
 }
 
-static const char* kernel_name(int kind, int tpi) {
+static const char* kernel_name(int kind, int tpi, bool narrow) {
     switch (kind) {
-        case 0: return "zgemm_kernel";
+        case 0: return narrow ? "zgemm_narrow_kernel" : "zgemm_kernel";
         case 1:
             switch (tpi) {  // the launch shape the autotuner chose
                 case 4: return "pt_kernel<4>";
@@ -1766,6 +1806,9 @@ void Session::launch_step(const Step& st, cudaStream_t s, double2* spec) {
         case 0:
             if (m)
                 launch_cgemm(st.g.probs, st.g.tiles, st.g.ntiles, st.g.xoff, st.g.yoff, st.g.X, st.g.Y, st.g.mode, s);
+            else if (st.g.rows)
+                launch_gemm_narrow(st.g.probs, st.g.tiles, st.g.ntiles, st.g.xoff, st.g.yoff, st.g.X, st.g.Y, st.g.mode,
+                                   st.g.kmax, st.g.rows, s);
             else
                 launch_gemm(st.g.probs, st.g.tiles, st.g.ntiles, st.g.xoff, st.g.yoff, st.g.X, st.g.Y, st.g.mode, s);
             break;
@@ -1881,7 +1924,7 @@ std::vector<Session::ProfileEntry> Session::profile_read() {
         const Step& st = steps_[pe.first];
         ProfileEntry& e = prof_[st.label];
         e.label = st.label;
-        e.kernel = kernel_name(st.kind, st.tpi);
+        e.kernel = kernel_name(st.kind, st.tpi, st.g.rows > 0);
         e.launches += 1;
         e.ms += ms;
         e.flops += st.flops;

@@ -100,6 +100,7 @@ private:
         const double2* X = nullptr;
         double2* Y = nullptr;
         int mode = 0;
+        int kmax = 0, rows = 0;  // few columns (launch_gemm_narrow) where rows > 0
     };
     struct PtLaunch {
         PtItem* items = nullptr;
@@ -190,6 +191,7 @@ private:
                   std::vector<std::vector<long long> >& yo, const double2* X, double2* Y, int mode,
                   const char* label, const Digits* dg = nullptr, const std::vector<char>* on_i8 = nullptr);
     const Digits* i8_target_ = nullptr;  // set while add_gemm emits the int8 part of a launch
+    bool narrow_ = false;                // set while it emits the products with few columns
     void add_i8(const std::vector<GemmProblem>& P, const long long* xs, const long long* ys, size_t ncols, double2* Y,
                 const Digits& dg, Step& st);
     void add_digits(const std::vector<I8Vec>& vecs, const double2* X, const Digits& dg, const char* label);

@@ -1,5 +1,5 @@
-"""The plain form's two translation kernels on one complex product: the FP64
-tensor path and the int8 tensor path (seven balanced base-256 digits a number,
+"""The plain form's translation kernels on one complex product: the FP64
+tensor path (64-column tiles, and the one for few columns) and the int8 tensor path (seven balanced base-256 digits a number,
 54 bits below the largest component of a vector or operator row, all sums
 exact) against a long-double product.
 
@@ -18,7 +18,7 @@ import pytest
 from ddfmm_b200 import _lib
 
 pytestmark = pytest.mark.gpu
-EDGES = [(1, 1, 1), (8, 15, 127), (53, 56, 128), (55, 16, 129), (56, 17, 33), (57, 152, 300), (64, 31, 5),
+EDGES = [(1, 1, 1), (17, 9, 7), (64, 296, 8), (129, 33, 17), (8, 15, 127), (53, 56, 128), (55, 16, 129), (56, 17, 33), (57, 152, 300), (64, 31, 5),
          (106, 95, 257), (112, 112, 640), (113, 90, 48), (152, 110, 129), (296, 174, 70), (400, 400, 131)]
 
 
@@ -48,9 +48,10 @@ def part_max(v, axis):
 def test_paths_against_long_double(m, k, n, spread):
     A, X = mats(m, k, n, spread)
     want = A.astype(np.clongdouble) @ X.astype(np.clongdouble)
-    err = {p: np.abs((product(A, X, p) - want).astype(np.complex128)) for p in (0, 1)}
+    err = {p: np.abs((product(A, X, p) - want).astype(np.complex128)) for p in (0, 1, 2)}
     assert np.all(err[1] <= 2.0 ** -51 * (k * part_max(A, 1) * part_max(X, 0) + np.abs(want).astype(float)))
-    assert np.all(err[0] <= 4 * k * 2.0 ** -52 * (np.abs(A) @ np.abs(X)))
+    for p in (0, 2):
+        assert np.all(err[p] <= 4 * k * 2.0 ** -52 * (np.abs(A) @ np.abs(X)))
     if k >= 16 and spread == 0.0:  # no further off than the FP64 path, column by column norms apart
         assert np.linalg.norm(err[1]) <= np.linalg.norm(err[0])
 
