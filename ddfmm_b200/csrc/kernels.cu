@@ -731,6 +731,49 @@ __global__ void __launch_bounds__(256) vlist_group_kernel(const int* __restrict_
     }
 }
 
+// The same sums for few groups (VGROUP_SPLIT): block (group, frequency chunk), warp
+// w takes entries w, w + 8, ..., 32 of them read at once and handed round by
+// shuffles; the warps' partial sums meet in shared memory.
+template <int G>
+__global__ void __launch_bounds__(256) vlist_split_kernel(const int* __restrict__ gptr, const int2* __restrict__ gsrc,
+                                                          const int* __restrict__ gtrg,
+                                                          const double2* __restrict__ spec,
+                                                          const double2* __restrict__ tns, double2* __restrict__ tsp) {
+    constexpr int G3 = G * G * G;
+    __shared__ double2 part[VGROUP_WARPS][8][32];
+    const int grp = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int f = blockIdx.y * 32 + lane;
+    double2 acc[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) acc[c] = make_double2(0.0, 0.0);
+    const int e1 = __ldg(gptr + grp + 1);
+    for (int e0 = __ldg(gptr + grp) + warp; e0 < e1; e0 += 32 * VGROUP_WARPS) {
+        const int mine = e0 + lane * VGROUP_WARPS;
+        const int2 my = mine < e1 ? __ldg(gsrc + mine) : make_int2(0, 0);
+        const int n = min(32, (e1 - e0 + VGROUP_WARPS - 1) / VGROUP_WARPS);
+        for (int i = 0; i < n; ++i) {
+            const int row = __shfl_sync(0xffffffffu, my.x, i), tm = __shfl_sync(0xffffffffu, my.y, i);
+            const double2 S = __ldg(spec + (size_t)row * G3 + f);
+            const double2* tb = tns + (size_t)(tm >> 8) * G3 + f;
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+                if (tm & (1 << c)) cfma(acc[c], __ldg(tb + (size_t)child_voff(c) * G3), S);
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 8; ++c) part[warp][c][lane] = acc[c];
+    __syncthreads();
+    const int t = __ldg(gtrg + 8 * grp + warp);  // warp w sums child position w
+    if (t < 0) return;
+    double2 v = part[0][warp][lane];
+#pragma unroll
+    for (int w = 1; w < VGROUP_WARPS; ++w) {
+        v.x += part[w][warp][lane].x;
+        v.y += part[w][warp][lane].y;
+    }
+    tsp[(size_t)t * G3 + f] = v;
+}
+
 // Pruned inverse DFT of one target's summed spectrum per block: P outputs
 // of G-term sums along z (each thread one (ka, kb) line, its G inputs read
 // straight from the summed spectrum), then y, then x; the corner-cube nodes
@@ -831,6 +874,16 @@ void launch_vlist_forward(const VlistLevel& L, const int* boxes, int nbox, const
 void launch_vlist_group(const VlistLevel& L, const VlistGroups& V, const double2* spec, double2* tsp,
                         cudaStream_t s) {
     if (V.ngroups == 0) return;
+    if ((long long)V.ngroups * (L.G * L.G * L.G / 32) < VGROUP_SPLIT) {
+        const dim3 sgrid(V.ngroups, L.G * L.G * L.G / 32);
+        switch (L.G) {
+            case 8: vlist_split_kernel<8><<<sgrid, 256, 0, s>>>(V.gptr, V.gsrc, V.gtrg, spec, L.tns, tsp); break;
+            case 12: vlist_split_kernel<12><<<sgrid, 256, 0, s>>>(V.gptr, V.gsrc, V.gtrg, spec, L.tns, tsp); break;
+            case 16: vlist_split_kernel<16><<<sgrid, 256, 0, s>>>(V.gptr, V.gsrc, V.gtrg, spec, L.tns, tsp); break;
+            default: break;
+        }
+        return;
+    }
     const dim3 grid((V.ngroups + VGROUP_WARPS - 1) / VGROUP_WARPS, L.G * L.G * L.G / 32);
     switch (L.G) {
         case 8: vlist_group_kernel<8><<<grid, 32 * VGROUP_WARPS, 0, s>>>(V.gptr, V.gsrc, V.gtrg, V.ngroups, spec, L.tns, tsp); break;

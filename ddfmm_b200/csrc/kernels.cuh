@@ -115,6 +115,13 @@ void launch_vlist_forward(const VlistLevel& L, const int* boxes, int nbox, const
 // tsp[t] (G^3 per target, rows in group order) receives the summed spectrum
 // of target t, overwritten each eval.
 constexpr int VGROUP_WARPS = 8;  // target parents per block of the sums
+// Launches with fewer (group, 32-frequency chunk) pairs than this give a pair a
+// whole block, its entries dealt to the 8 warps: a warp alone walks 40 to 190
+// entries of two dependent loads each, and so few warps do not fill the SMs.
+// Measured: K = 4, P = 4 (800 pairs) 86 -> 80 us a matvec, a K = 8 adaptive cluster
+// (five levels) 681 -> 643 us, but K = 8, P = 4 (2900 pairs) 399 -> 409 us: the line
+// lies at 12 warps an SM.
+constexpr long long VGROUP_SPLIT = 148 * 12;
 struct VlistGroups {
     const int* gptr;   // ngroups + 1: the source entries of each group
     const int2* gsrc;  // the source entries

@@ -569,6 +569,48 @@ __global__ void __launch_bounds__(256) vlist_group32_kernel(const VaSub one, con
     }
 }
 
+// vlist_split_kernel of kernels.cu in complex FP32: one instance with few groups.
+template <int G>
+__global__ void __launch_bounds__(256) vlist_split32_kernel(const VaSub S, const int* __restrict__ active,
+                                                            const float2* spec_override) {
+    constexpr int G3 = G * G * G;
+    __shared__ float2 part[VGROUP_WARPS][8][32];
+    if (active && !active[S.inst]) return;
+    const float2* __restrict__ spec = spec_override ? spec_override : S.spec;
+    const float2* __restrict__ tns = reinterpret_cast<const float2*>(S.L.tns);
+    const int grp = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int f = blockIdx.y * 32 + lane;
+    float2 acc[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) acc[c] = make_float2(0.f, 0.f);
+    const int e1 = __ldg(S.gptr + grp + 1);
+    for (int e0 = __ldg(S.gptr + grp) + warp; e0 < e1; e0 += 32 * VGROUP_WARPS) {
+        const int mine = e0 + lane * VGROUP_WARPS;
+        const int2 my = mine < e1 ? __ldg(S.gsrc + mine) : make_int2(0, 0);
+        const int n = min(32, (e1 - e0 + VGROUP_WARPS - 1) / VGROUP_WARPS);
+        for (int i = 0; i < n; ++i) {
+            const int row = __shfl_sync(0xffffffffu, my.x, i), tm = __shfl_sync(0xffffffffu, my.y, i);
+            const float2 sv = __ldg(spec + (size_t)row * G3 + f);
+            const float2* tb = tns + (size_t)(tm >> 8) * G3 + f;
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+                if (tm & (1 << c)) cfma32(acc[c], __ldg(tb + (size_t)child_voff32(c) * G3), sv);
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 8; ++c) part[warp][c][lane] = acc[c];
+    __syncthreads();
+    const int t = __ldg(S.gtrg + 8 * grp + warp);  // warp w sums child position w
+    if (t < 0) return;
+    float2 v = part[0][warp][lane];
+#pragma unroll
+    for (int w = 1; w < VGROUP_WARPS; ++w) {
+        v.x += part[w][warp][lane].x;
+        v.y += part[w][warp][lane].y;
+    }
+    S.tsp[(size_t)t * G3 + f] = v;
+}
+
 // The inverse transform of kernels.cu (vlist_inverse_kernel) in complex FP32,
 // one block per target.
 template <int G>
@@ -703,6 +745,16 @@ void launch_vlist_group32(const VaSub* subs, const int* prefix, int nsub, int ng
         o = *one;
     }
     const float2* so = static_cast<const float2*>(spec_override);
+    if (nsub == 1 && (long long)ngroups * (G * G * G / 32) < VGROUP_SPLIT) {
+        const dim3 sgrid(ngroups, G * G * G / 32);
+        switch (G) {
+            case 8: vlist_split32_kernel<8><<<sgrid, 256, 0, s>>>(o, active, so); break;
+            case 12: vlist_split32_kernel<12><<<sgrid, 256, 0, s>>>(o, active, so); break;
+            case 16: vlist_split32_kernel<16><<<sgrid, 256, 0, s>>>(o, active, so); break;
+            default: break;
+        }
+        return;
+    }
     const dim3 grid((ngroups + VGROUP_WARPS - 1) / VGROUP_WARPS, G * G * G / 32);
 #define DDFMM_VGRP(g)                                                                                             \
     if (nsub == 1)                                                                                                \
