@@ -199,7 +199,8 @@ private:
     void add_umma(const std::vector<GemmProblem>& P, const long long* xs, const long long* ys, size_t ncols,
                   const double2* X, double2* Y, int mode, Step& st);
     void flush_packs();
-    void add_pt(const std::vector<PtItem>& items, const std::vector<PtSrc>& srcs, const char* label);
+    static constexpr size_t kPtItems = 148 * 16;  // items a point-interaction step should have: 16 warps an SM
+    void add_pt(std::vector<PtItem> items, const std::vector<PtSrc>& srcs, const char* label);
     template <class Sub>
     void set_multi(Step& st, const Sub& sub, int total);
     void begin_block(int phase, double W);
