@@ -196,6 +196,9 @@ Session::~Session() {
     stage_release();
     for (cudaEvent_t e : ev_) cudaEventDestroy(e);
     for (void* p : allocs_) cudaFree(p);
+    for (cudaEvent_t e : {fork_, lf_up_, join_})
+        if (e) cudaEventDestroy(e);
+    if (side_) cudaStreamDestroy(side_);
     if (stream_) cudaStreamDestroy(stream_);
 }
 
@@ -506,6 +509,7 @@ void Session::push_step(Step st) {
     for (size_t i = 0; i < sizeof(order) / sizeof(order[0]); ++i)
         if (base == order[i]) rank = (long long)i;
     const long long occ = block_counts_[base]++;
+    st.lane = lane_;
     st.key = ((long long)cur_phase_ << 48) | (cur_wkey_ << 32) | (rank << 16) | occ;
     steps_.push_back(st);
 }
@@ -1577,6 +1581,14 @@ void Session::build() {
     }
 
     phase("steps_hf_down");
+    // Small instances do not fill the GPU in any pass: their V-list sums and near field
+    // run beside the high-frequency passes (run_steps).  The line is the size of the
+    // summed target spectra, which then need memory of their own.
+    overlap_ = !hflevels.empty() && (size_t)nLF * G3 * es <= ((size_t)128 << 20);
+    if (overlap_) {
+        CK(cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking));
+        for (cudaEvent_t* e : {&fork_, &lf_up_, &join_}) CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+    }
     // ---------------------------------------------------------------- steps: LF downward
     for (auto& kv : lflevels) {  // levels ascending = widths descending
         int level = kv.first;
@@ -1612,13 +1624,16 @@ void Session::build() {
                                   reinterpret_cast<float2*>(lf_spec), f.v.nsrc, 0};
                     set_multi(f, f.hvf, f.v.nsrc);
                 }
+                lane_ = Step::SIDE_LATE;
                 push_step(f);
-                // summed target spectra: a high-frequency buffer when one is large enough
+                // summed target spectra, of their own where the sums may overlap the
+                // high-frequency passes; else a high-frequency buffer when one is large enough
                 // (every high-frequency pass has run before this low-frequency downward
                 // step, so the outgoing densities and the incoming check values are free
                 // by then), else a buffer of their own
                 const size_t tsp_elems = trg.size() * (size_t)G3;
-                double2* tsp = tsp_elems <= (size_t)upeq_total    ? hf_upeq
+                double2* tsp = overlap_                           ? salloc(tsp_elems)
+                               : tsp_elems <= (size_t)upeq_total  ? hf_upeq
                                : tsp_elems <= (size_t)dnchk_total ? hf_dnchk
                                                                   : salloc(tsp_elems);
                 const int ngroups = (int)vg.gptr.size() - 1;
@@ -1640,6 +1655,7 @@ void Session::build() {
                     set_multi(a, a.hva, ngroups);
                 }
                 push_step(a);
+                lane_ = Step::MAIN;
                 Step iv{};
                 iv.kind = 6;
                 iv.label = "lf_vlist_inv";
@@ -1679,7 +1695,9 @@ void Session::build() {
                 itm.src_end = (int)S.size();
                 (direct ? itemsA : itemsB).push_back(itm);
             }
+            lane_ = Step::SIDE_EARLY;
             add_pt(itemsA, srcsA, "lf_xlist");
+            lane_ = Step::MAIN;
             add_pt(itemsB, srcsB, "lf_xlist");
         }
         // U list (src/wave3d_eval.cpp:585-600) and W list (:688-718) into extval
@@ -1722,8 +1740,11 @@ void Session::build() {
                     witems.push_back(itm);
                 }
             }
+            lane_ = Step::SIDE_EARLY;
             add_pt(items, srcs, "lf_ulist");
+            lane_ = Step::SIDE_LATE;
             add_pt(witems, wsrcs, "lf_wlist");
+            lane_ = Step::MAIN;
         }
         // dneqnden = up^T (1/sigma .* (v^T dnchk))   (src/wave3d_eval.cpp:536-547, src/mlib3d.cpp:147-152)
         std::vector<long long> a;
@@ -1920,6 +1941,10 @@ void Session::run_steps(cudaStream_t s) {
         for (size_t i = have; i < ev_.size(); ++i) CK(cudaEventCreate(&ev_[i]));
     }
     if (profiling_ && !ev_pending_.empty()) profile_read();  // keep one eval of events in flight at most
+    if (overlap_ && !profiling_) {
+        run_overlapped(s);
+        return;
+    }
     for (size_t i = 0; i < steps_.size(); ++i) {
         const Step& st = steps_[i];
         if (profiling_) CK(cudaEventRecord(ev_[2 * i], s));
@@ -1929,6 +1954,30 @@ void Session::run_steps(cudaStream_t s) {
             ev_pending_.push_back(std::make_pair((int)i, (int)(2 * i)));
         }
     }
+}
+
+// The steps on two streams.  Side stream: U and direct X lists at once, V-list
+// transforms and sums and W lists once the upward low-frequency passes are done
+// (they only read points, densities and outgoing LF densities); each adds into
+// values that nothing on the caller's stream touches before the join, where the
+// downward low-frequency passes begin.  Works on a capturing stream: the side
+// stream joins the capture at the fork and leaves it at the join.
+void Session::run_overlapped(cudaStream_t s) {
+    CK(cudaEventRecord(fork_, s));
+    CK(cudaStreamWaitEvent(side_, fork_, 0));
+    for (const Step& st : steps_)
+        if (st.lane == Step::SIDE_EARLY) launch_step(st, side_, st.v.spec);
+    size_t i = 0;
+    for (; i < steps_.size() && (steps_[i].key >> 48) == 0; ++i) launch_step(steps_[i], s, steps_[i].v.spec);
+    CK(cudaEventRecord(lf_up_, s));
+    CK(cudaStreamWaitEvent(side_, lf_up_, 0));
+    for (const Step& st : steps_)
+        if (st.lane == Step::SIDE_LATE) launch_step(st, side_, st.v.spec);
+    CK(cudaEventRecord(join_, side_));
+    for (; i < steps_.size() && (steps_[i].key >> 48) < 3; ++i) launch_step(steps_[i], s, steps_[i].v.spec);
+    CK(cudaStreamWaitEvent(s, join_, 0));
+    for (; i < steps_.size(); ++i)
+        if (steps_[i].lane == Step::MAIN) launch_step(steps_[i], s, steps_[i].v.spec);
 }
 
 void Session::profile_enable(bool on) {

@@ -154,6 +154,9 @@ private:
         // that play the same part (phase, width, step type, occurrence): a Batch
         // merges the steps of its sessions that share a key into one launch.
         long long key;
+        // Stream of the step when an eval overlaps its passes (run_steps): the caller's, or
+        // the side stream from the eval's start or from the end of the upward LF passes
+        enum Lane { MAIN = 0, SIDE_EARLY = 1, SIDE_LATE = 2 } lane;
         int tpi;  // point interactions: launch shape (launch_pt; 0 = 32 threads per item), set by autotune()
         // mixed form: the step as a one-instance launch (device sub-launch array and
         // prefix sums) and the host copy of its sub-launch
@@ -210,6 +213,7 @@ private:
     // and keeps the fastest (point interactions: threads per item).
     void autotune();
     void run_steps(cudaStream_t s);
+    void run_overlapped(cudaStream_t s);
     void run_steps_spec(cudaStream_t s, double2* spec);
     void launch_step(const Step& st, cudaStream_t s, double2* spec);
 
@@ -245,6 +249,10 @@ private:
     void stage_copy(void* dst, const void* src, size_t bytes);
     void stage_release();  // after a stream sync
     std::vector<Step> steps_;
+    Step::Lane lane_ = Step::MAIN;  // of the steps being emitted
+    bool overlap_ = false;          // small instance: passes overlap on two streams
+    cudaStream_t side_ = nullptr;
+    cudaEvent_t fork_ = nullptr, lf_up_ = nullptr, join_ = nullptr;
     cudaStream_t stream_ = nullptr;
     SessionStats stats_;
 
