@@ -214,6 +214,7 @@ private:
     void autotune();
     void run_steps(cudaStream_t s);
     void run_overlapped(cudaStream_t s);
+    void build_graph();
     void run_steps_spec(cudaStream_t s, double2* spec);
     void launch_step(const Step& st, cudaStream_t s, double2* spec);
 
@@ -253,6 +254,7 @@ private:
     bool overlap_ = false;          // small instance: passes overlap on two streams
     cudaStream_t side_ = nullptr;
     cudaEvent_t fork_ = nullptr, lf_up_ = nullptr, join_ = nullptr;
+    cudaGraphExec_t graph_ = nullptr;  // run_steps of a small instance, instantiated at setup
     cudaStream_t stream_ = nullptr;
     SessionStats stats_;
 
