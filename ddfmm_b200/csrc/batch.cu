@@ -43,6 +43,28 @@ void Batch::add(Kind kind, const std::vector<Sub>& subs, const std::vector<Pre>&
     if (L.total > 0) launches_.push_back(L);
 }
 
+// Tile order of the GEMM launch just added.  Instances share packed operators (the
+// process-wide cache): tiles that read one operator block run next to each other
+// across instances, so the block comes from DRAM once while the blocks in flight
+// share it in L2, instead of once per instance.  Within an operator, instance order
+// and each instance's tile order are kept.
+void Batch::by_operator(const std::vector<std::pair<int, const Session::Step*> >& steps) {
+    if (steps.size() < 2 || steps.size() >= 256) return;
+    std::vector<std::pair<const float*, int> > key;
+    for (size_t j = 0; j < steps.size(); ++j) {
+        const std::vector<const float*>& op = steps[j].second->uop;
+        if (op.size() >= (1u << 24)) return;
+        for (size_t t = 0; t < op.size(); ++t) key.push_back(std::make_pair(op[t], (int)((j << 24) | t)));
+    }
+    std::stable_sort(key.begin(), key.end(),
+                     [](const std::pair<const float*, int>& a, const std::pair<const float*, int>& b) {
+                         return a.first < b.first;
+                     });
+    std::vector<int> order(key.size());
+    for (size_t i = 0; i < key.size(); ++i) order[i] = key[i].second;
+    launches_.back().order = upload_bytes(order.data(), sizeof(int) * order.size());
+}
+
 Batch::Batch(const std::vector<Session*>& sessions) : sessions_(sessions) {
     if (sessions_.empty()) throw std::invalid_argument("a batch needs at least one session");
     device_ = sessions_[0]->device();
@@ -98,30 +120,30 @@ Batch::Batch(const std::vector<Session*>& sessions) : sessions_(sessions) {
                     tiles += u.ntiles;
                 }
                 add(GEMM, subs, n);
-                // Instances share packed operators (the process-wide cache): tiles that
-                // read one operator block run next to each other across instances, so
-                // the block comes from DRAM once while the blocks in flight share it in
-                // L2, instead of once per instance.  Within an operator, instance order
-                // and each instance's tile order are kept.
-                if (subs.size() > 1 && tiles > 0 && subs.size() < 256) {  // add() appended this launch
-                    std::vector<std::pair<const float*, int> > key;
-                    bool fits = true;
-                    for (size_t j = 0; j < kk.second.size(); ++j) {
-                        const std::vector<const float*>& op = kk.second[j].second->uop;
-                        if ((int)op.size() != n[j] || op.size() >= (1u << 24)) fits = false;
-                        for (size_t t = 0; fits && t < op.size(); ++t)
-                            key.push_back(std::make_pair(op[t], (int)((j << 24) | t)));
-                    }
-                    if (fits) {
-                        std::stable_sort(key.begin(), key.end(),
-                                         [](const std::pair<const float*, int>& a, const std::pair<const float*, int>& b) {
-                                             return a.first < b.first;
-                                         });
-                        std::vector<int> order(key.size());
-                        for (size_t i = 0; i < key.size(); ++i) order[i] = key[i].second;
-                        launches_.back().order = upload_bytes(order.data(), sizeof(int) * order.size());
-                    }
+                if (tiles > 0) by_operator(kk.second);
+            } else if (kind == 10) {
+                std::vector<HSub> subs;
+                std::vector<int> n;
+                long long tiles = 0;
+                for (auto& e : kk.second) {
+                    HSub u = e.second->hh;
+                    u.inst = e.first;
+                    subs.push_back(u);
+                    n.push_back(u.ntiles);
+                    tiles += u.ntiles;
                 }
+                add(GEMM16, subs, n);
+                if (tiles > 0) by_operator(kk.second);
+            } else if (kind == 9) {
+                std::vector<HSliceSub> subs;
+                std::vector<int> n;
+                for (auto& e : kk.second) {
+                    HSliceSub u = e.second->hs;
+                    u.inst = e.first;
+                    subs.push_back(u);
+                    n.push_back(u.n);
+                }
+                add(SPLIT16, subs, n);
             } else if (kind == 1) {
                 std::vector<PtSub> subs;
                 std::vector<int> n;
@@ -226,6 +248,15 @@ void Batch::run(const int* active, cudaStream_t s) {
                                   (int)L.total, active, d_err_, s,
                                   L.nsub == 1 ? reinterpret_cast<const UmmaSub*>(L.one) : nullptr, 0, 0,
                                   static_cast<const int*>(L.order));
+                break;
+            case SPLIT16:
+                launch_h16_slice(static_cast<const HSliceSub*>(L.subs), static_cast<const int*>(L.prefix), L.nsub,
+                                 (int)L.total, active, s, *reinterpret_cast<const HSliceSub*>(L.one));
+                break;
+            case GEMM16:
+                launch_h16_gemm(static_cast<const HSub*>(L.subs), static_cast<const int*>(L.prefix), L.nsub, (int)L.total,
+                                active, d_err_, s, *reinterpret_cast<const HSub*>(L.one),
+                                static_cast<const int*>(L.order));
                 break;
             case PT:
                 launch_pt32(static_cast<const PtSub*>(L.subs), static_cast<const int*>(L.prefix), L.nsub, (int)L.total,

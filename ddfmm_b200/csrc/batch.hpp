@@ -43,7 +43,7 @@ public:
     void check_error(cudaStream_t s);
 
 private:
-    enum Kind { ZERO, GATHER, SCATTER, GEMM, PT, VFWD, VACC, VINV };
+    enum Kind { ZERO, GATHER, SCATTER, GEMM, SPLIT16, GEMM16, PT, VFWD, VACC, VINV };
     struct Launch {
         Kind kind;
         void* subs;
@@ -57,6 +57,7 @@ private:
     };
     template <class Sub, class Pre>
     void add(Kind kind, const std::vector<Sub>& subs, const std::vector<Pre>& counts, int G = 0);
+    void by_operator(const std::vector<std::pair<int, const Session::Step*> >& steps);
     void* upload_bytes(const void* p, size_t bytes);
 
     std::vector<Session*> sessions_;

@@ -67,6 +67,50 @@ void test_gemm(const double2* A, int m, int k, const double2* X, int ncol, int p
         gemm_init();
         launch_gemm_narrow(P.put(std::vector<GemmProblem>(1, GemmProblem{dA, m, k, m, 0, ncol, nullptr})), P.put(tiles),
                            (int)tiles.size(), P.put(xo), dyo, dX, dY, GEMM_ATOMIC, k, rows, nullptr);
+    } else if (path >= 3) {  // mixed form, on FP32 copies: 3 FP16 planes, 4 split TF32
+        auto narrow = [](const std::vector<double2>& v) {
+            std::vector<float2> r;
+            for (const double2& a : v) r.push_back(make_float2((float)a.x, (float)a.y));
+            return r;
+        };
+        const float2* fA = P.put(narrow(std::vector<double2>(A, A + (size_t)m * k)));
+        const float2* fX = P.put(narrow(hx));
+        std::vector<float2> fy = narrow(hy);
+        float2* fY = P.put(fy);
+        int* err = P.put(std::vector<int>(1, 0));
+        if (path == 3) {
+            float* B = P.put(std::vector<float>(h16_packed_floats(m, k)));
+            char* X16 = P.put(std::vector<char>((size_t)ncol * (sx / 16) * H16_GRANULE));
+            float* cx = P.put(std::vector<float>((size_t)ncol * (sx / 16)));
+            std::vector<H16Tile> tiles;
+            h16_tiles(B, m, k, 0, ncol, tiles);
+            h16_init();
+            launch_h16_pack(P.put(std::vector<H16PackJob>(1, H16PackJob{fA, B, const_cast<float*>(h16_scales(B, m, k)), m, k,
+                                                                        m, h16_tile_rows(m)})),
+                            1, h16_row_tiles(m), nullptr);
+            launch_h16_slice(nullptr, nullptr, 1, ncol, nullptr, nullptr, HSliceSub{P.put(vecs), fX, X16, cx, ncol, 0});
+            launch_h16_gemm(nullptr, nullptr, 1, (int)tiles.size(), nullptr, err, nullptr,
+                            HSub{P.put(tiles), P.put(xg), dyo, X16, cx, fY, (int)tiles.size(), 0});
+        } else {
+            float* B = P.put(std::vector<float>(umma_packed_floats(m, k)));
+            std::vector<UmmaTile> tiles;
+            for (int r = 0; r * 128 < m; ++r)
+                for (int c = 0; c < ncol; c += 128) tiles.push_back(UmmaTile{0, r, r * 128, m - r * 128 < 128 ? m - r * 128 : 128, c, 0});
+            umma_init();
+            launch_umma_pack(P.put(std::vector<UmmaPackJob>(1, UmmaPackJob{fA, B, umma_tile_stride(k), m, k, m, umma_nkb(k)})),
+                             1, nullptr);
+            const UmmaSub one{P.put(std::vector<UmmaProblem>(1, UmmaProblem{B, umma_tile_stride(k), m, k, umma_nkb(k), 0, ncol})),
+                              P.put(tiles), P.put(xo), dyo, fX, fY, (int)tiles.size(), GEMM_ATOMIC, 0, 0};
+            launch_umma_cgemm(nullptr, nullptr, 1, (int)tiles.size(), nullptr, err, nullptr, &one);
+        }
+        int h = 0;
+        ck(cudaMemcpy(&h, err, sizeof(int), cudaMemcpyDeviceToHost));
+        if (h) throw std::runtime_error("CUDA error: a tensor-core GEMM timed out waiting on its pipeline");
+        ck(cudaGetLastError());
+        ck(cudaMemcpy(fy.data(), fY, sizeof(float2) * fy.size(), cudaMemcpyDeviceToHost));
+        for (int c = 0; c < ncol; ++c)
+            for (int i = 0; i < m; ++i) Y[(size_t)c * m + i] = make_double2(fy[yo[c] + i].x, fy[yo[c] + i].y);
+        return;
     } else {
         const int nkb = (k + 15) / 16;
         char* B = P.put(std::vector<char>(i8_packed_bytes(m, k)));

@@ -306,8 +306,56 @@ void i8_tiles(const char* B, const double* ra, int m, int k, int col0, int ncol,
 void launch_i8_pack(const I8PackJob* jobs_dev, int njobs, int max_tiles, cudaStream_t s);
 // *err is set when a block gave up waiting on its pipeline
 void launch_i8_gemm(const I8Sub& sub, int* err, cudaStream_t s);
-// gemm_test.cu: Y += A X through a GEMM kernel of the plain form (0: FP64, 1: int8 tensor path)
+// gemm_test.cu: Y += A X through one of the GEMM kernels (paths as in ddfmm.h)
 void test_gemm(const double2* A, int m, int k, const double2* X, int ncol, int path, double2* Y);
+
+// Mixed-form high-frequency GEMM on the FP16 tensor cores (kernels_h16.cu): 128
+// gathered columns x up to H16_TILE_ROWS complex operator rows per tile; both
+// operands as two FP16 planes under a power-of-two scale per vector / operator row.
+constexpr int H16_TILE_ROWS = 112;
+constexpr int H16_GRANULE = 128;  // bytes of the planes of 16 complex numbers: 64 of hi, 64 of lo
+struct HSliceSub {  // one instance's vectors to write as planes
+    const I8Vec* vecs;
+    const float2* X;
+    char* X16;
+    float* cx;  // output scale of the vector that starts at a granule
+    int n;
+    int inst;
+};
+struct alignas(16) H16Tile {  // everything about a tile, so that its next one can be read ahead
+    const float* B;           // the row tile's packed operator (h16_pack_kernel)
+    const float* ra;          // output scales of its rows
+    int col, row0;            // first column (of xgran, yoff), first operator row
+    unsigned short ncol, rows, n, k;  // columns, valid complex rows, real rows, complex K
+};
+struct HSub {
+    const H16Tile* tiles;
+    const int* xgran;       // first granule of each column's vector
+    const long long* yoff;  // element of Y each column adds into
+    const char* X16;
+    const float* cx;
+    float2* Y;
+    int ntiles;
+    int inst;
+};
+struct H16PackJob {
+    const float2* A;  // complex FP32 operator, column-major
+    float* dst;
+    float* ra;
+    int m, k, lda, rows_t;
+};
+void h16_init();
+int h16_row_tiles(int m);
+int h16_tile_rows(int m);
+size_t h16_packed_floats(int m, int k);
+const float* h16_scales(const float* packed, int m, int k);  // the row scales of a packed operator
+void h16_tiles(const float* packed, int m, int k, int col0, int ncol, std::vector<H16Tile>& out);
+void launch_h16_pack(const H16PackJob* jobs_dev, int njobs, int max_tiles, cudaStream_t s);
+// nsub == 1: `one` is that sub-launch (sent as a kernel parameter); order as in launch_umma_cgemm
+void launch_h16_slice(const HSliceSub* subs, const int* prefix, int nsub, int n, const int* active, cudaStream_t s,
+                      const HSliceSub& one);
+void launch_h16_gemm(const HSub* subs, const int* prefix, int nsub, int ntiles, const int* active, int* err,
+                     cudaStream_t s, const HSub& one, const int* order = nullptr);
 
 // gather/scatter helpers
 void launch_gather_den(const double2* den, const int* perm, double2* out, int n, cudaStream_t s);

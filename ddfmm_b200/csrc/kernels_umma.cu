@@ -49,6 +49,7 @@
 #include <cstdint>
 
 #include "kernels.cuh"
+#include "umma.cuh"
 
 namespace ddfmm {
 
@@ -65,9 +66,6 @@ constexpr int UNMAX = 256;   // max real rows per tile (MMA N)
 #endif
 #ifndef DDFMM_UMMA_PREF
 #define DDFMM_UMMA_PREF (UBK == 16 ? 4 : 8)
-#endif
-#ifndef DDFMM_UMMA_PCH
-#define DDFMM_UMMA_PCH 32
 #endif
 constexpr int USTAGES = DDFMM_UMMA_STAGES;  // ring depth
 constexpr int UPREF = DDFMM_UMMA_PREF;      // gathered-column blocks prefetched into registers
@@ -90,17 +88,11 @@ constexpr int U_EMPTY_ACC_COUNT = (UELECT ? 4 : UM) * UEPI;  // epilogue arrival
 constexpr int U_A_BYTES = UM * UBK * 4;
 constexpr int U_B_BYTES = UNMAX * UBK * 4;
 constexpr int U_STAGE_BYTES = 2 * U_A_BYTES + 2 * U_B_BYTES;
-constexpr int PCH = DDFMM_UMMA_PCH;  // epilogue chunk: complex rows parked per column
-static_assert(PCH == 32, "epilogue chunk of 32 rows");
-constexpr int UPS = PCH + 2;  // parking-area row stride (complex): 16-byte rows, conflict-free 16-byte accesses
 constexpr int U_PARK_BYTES = 4 * UEPI * 32 * UPS * 8;  // 32 columns x PCH complex (+2 pad) per warp
 // ring + parking area + alignment slack: one block per SM (also what the 512
 // TMEM columns need)
 constexpr int UGEMM_SMEM = USTAGES * U_STAGE_BYTES + U_PARK_BYTES + 1024;
 static_assert(UGEMM_SMEM + 4096 <= 232448, "shared memory per block");
-constexpr unsigned long long U_WAIT_NS = 1000000000ull;  // 1 s
-constexpr uint32_t U_WAIT_ITERS = 1u << 26;
-
 // byte offset of element (r, kk), kk < UBK, of a K block in the core-matrix layout
 __host__ __device__ __forceinline__ int core_off(int r, int kk) {
     return (r >> 3) * (UBK * 32) + (kk >> 2) * 128 + (r & 7) * 16 + (kk & 3) * 4;
@@ -116,8 +108,6 @@ __host__ __device__ __forceinline__ int core_off_a(int r, int kk) {
     const int row = (r >> 3) * (8 * U_ARB) + (r & 7) * U_ARB;
     return row + ((((kk >> 2) ^ ((((r & 7) * U_ARB) >> 7) & (U_ARB / 16 - 1)))) << 4) + (kk & 3) * 4;
 }
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 // descriptor of a gathered-column block in the swizzled layout: 8-row groups
 // 8 U_ARB bytes apart (SBO), leading offset unused (one swizzle row spans the
@@ -148,61 +138,6 @@ __device__ __forceinline__ uint32_t idesc_tf32(int n) {
     return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(UM >> 4) << 24);
 }
 
-__device__ __forceinline__ unsigned long long gtimer() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;\n" : "=l"(t));
-    return t;
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-
-// Wait for the phase of parity `parity`; false after limit_ns, 2^26 polls, or
-// once *failed is set by another role.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* failed,
-                                          unsigned long long limit_ns) {
-    const uint32_t addr = smem_u32(bar);
-    unsigned long long t0 = 0;
-    for (uint32_t it = 0; it < U_WAIT_ITERS; ++it) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}\n"
-            : "=r"(done)
-            : "r"(addr), "r"(parity)
-            : "memory");
-        if (done) return true;
-        if ((it & 255) == 255) {
-            if (failed && *failed) return false;
-            const unsigned long long t = gtimer();
-            if (t0 == 0)
-                t0 = t;
-            else if (t - t0 > limit_ns)
-                return false;
-        }
-    }
-    return false;
-}
-
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(bar)) : "memory");
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%1], %0;\n" ::"r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
-}
-
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
-            smem_u32(dst)),
-        "l"(src), "r"(bytes), "r"(smem_u32(bar))
-        : "memory");
-}
-
 __device__ __forceinline__ void umma_tf32(uint32_t dtmem, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -210,12 +145,6 @@ __device__ __forceinline__ void umma_tf32(uint32_t dtmem, uint64_t da, uint64_t 
         "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}\n" ::"r"(dtmem),
         "l"(da), "l"(db), "r"(idesc), "r"(acc), "r"(0u)
         : "memory");
-}
-
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                     smem_u32(bar))
-                 : "memory");
 }
 
 __device__ __forceinline__ uint32_t tf32_bits(float x) {
@@ -296,51 +225,6 @@ size_t umma_packed_floats(int m, int k) {
 }
 
 // ---------------------------------------------------------------- GEMM
-// Epilogue stores of one parked chunk (PCH complex rows from row0 on, 32 columns):
-// two columns per instruction, each lane two consecutive rows of one column, as
-// one 16-byte store or vector atomic where the output is 16-byte aligned (two
-// 8-byte ones otherwise, or one at an odd last row).  Column c of the warp's 32
-// writes at Y + (c's yoff) + row.
-template <int MODE>
-__device__ __forceinline__ void store_one(float2* y, float2 v) {
-    if (MODE == GEMM_SET) {
-        *y = v;
-    } else if (MODE == GEMM_ADD) {
-        const float2 o = *y;
-        *y = make_float2(o.x + v.x, o.y + v.y);
-    } else {
-        atomicAdd(y, v);
-    }
-}
-template <int MODE>
-__device__ __forceinline__ void store_chunk(const float2* park, float2* Y, long long my_yo, int col_base, int ncol,
-                                            int row0, int rows, int lane) {
-    const int sub = lane >> 4, r2 = 2 * (lane & 15), i = row0 + r2;
-    for (int cc = 0; cc < 32; cc += 2) {
-        const int col = cc + sub;
-        const long long yb = __shfl_sync(0xffffffffu, my_yo, col);
-        if (col_base + cc >= ncol) break;
-        if (i >= rows || col_base + col >= ncol) continue;
-        const float4 v = *reinterpret_cast<const float4*>(park + col * UPS + r2);
-        float2* y = Y + yb + i;
-        const bool two = i + 1 < rows;
-        if (two && (reinterpret_cast<uintptr_t>(y) & 15) == 0) {
-            float4* y4 = reinterpret_cast<float4*>(y);
-            if (MODE == GEMM_SET) {
-                *y4 = v;
-            } else if (MODE == GEMM_ADD) {
-                const float4 o = *y4;
-                *y4 = make_float4(o.x + v.x, o.y + v.y, o.z + v.z, o.w + v.w);
-            } else {
-                atomicAdd(y4, v);
-            }
-        } else {
-            store_one<MODE>(y, make_float2(v.x, v.y));
-            if (two) store_one<MODE>(y + 1, make_float2(v.z, v.w));
-        }
-    }
-}
-
 // Tile ti of a launch: its sub-launch (prefix[j] <= ti < prefix[j+1], or
 // order[ti] = j << 24 | tile of sub-launch j where the launch gives an order),
 // tile and problem; `on` is false when the sub-launch's instance is inactive.

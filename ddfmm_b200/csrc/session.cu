@@ -207,6 +207,12 @@ Session::~Session() {
 void Session::add_gemm(std::vector<GemmProblem>& probs, std::vector<std::vector<long long> >& xo,
                        std::vector<std::vector<long long> >& yo, const double2* X, double2* Y, int mode,
                        const char* label, const Digits* dg, const std::vector<char>* on_i8) {
+    if (on_i8 && !on_i8->empty() && umma()) {  // all problems
+        i8_target_ = dg;
+        add_gemm(probs, xo, yo, X, Y, mode, label);
+        i8_target_ = nullptr;
+        return;
+    }
     if (on_i8 && !on_i8->empty()) {  // the problems chosen for the int8 path, then the others
         std::vector<GemmProblem> big, small;
         std::vector<std::vector<long long> > bx, by, sx, sy;
@@ -309,10 +315,14 @@ void Session::add_gemm(std::vector<GemmProblem>& probs, std::vector<std::vector<
     st.flops = flops;
     st.bytes = bytes;
     if (i8_target_) {
-        // a label of its own, so that profiles show the two kernels apart
-        st.label = width_label((std::string(label).substr(0, std::string(label).rfind("_w")) + "_i8").c_str(),
-                               std::atof(label + std::string(label).rfind("_w") + 2));
-        add_i8(P, xs.get(), ys.get(), ncols, Y, *i8_target_, st);
+        if (umma()) {
+            add_h16(P, xs.get(), ys.get(), ncols, Y, *i8_target_, st);
+        } else {
+            // a label of its own, so that profiles show the two kernels apart
+            st.label = width_label((std::string(label).substr(0, std::string(label).rfind("_w")) + "_i8").c_str(),
+                                   std::atof(label + std::string(label).rfind("_w") + 2));
+            add_i8(P, xs.get(), ys.get(), ncols, Y, *i8_target_, st);
+        }
         push_step(st);
         stats_.gemm_launches++;
         return;
@@ -345,7 +355,7 @@ const float* Session::cached_op(const std::string& key) {
     return e->p;
 }
 
-const float* Session::packed_operator(const GemmProblem& q) {
+const float* Session::packed_operator(const GemmProblem& q, bool h16) {
     if (q.packed) return q.packed;  // shared copy from the cache
     struct Clock {
         double& acc;
@@ -357,7 +367,7 @@ const float* Session::packed_operator(const GemmProblem& q) {
     if (it != packed_.end()) return it->second;
     // packed operators are sub-allocated from device chunks (256-byte aligned; cp.async.bulk
     // needs 16), the unit the operator cache frees; one larger than a chunk gets its own
-    const size_t nf = (umma_packed_floats(q.m, q.k) + 63) & ~(size_t)63;
+    const size_t nf = ((h16 ? h16_packed_floats(q.m, q.k) : umma_packed_floats(q.m, q.k)) + 63) & ~(size_t)63;
     if (nf > chunk_left_) {
         Clock ca{t_pack_alloc_};
         // chunks of 16 MiB doubling to 128 MiB: small sessions stay small, large
@@ -377,7 +387,11 @@ const float* Session::packed_operator(const GemmProblem& q) {
     held_.push_back(op);
     auto k = opkey_.find((const void*)q.A);
     if (k != opkey_.end()) to_publish_.push_back(std::make_pair(opctx_ + "|" + k->second, op));
-    pack_jobs_.push_back(UmmaPackJob{(const float2*)q.A, d, umma_tile_stride(q.k), q.m, q.k, q.lda, umma_nkb(q.k)});
+    if (h16)
+        h16_jobs_.push_back(H16PackJob{(const float2*)q.A, d, const_cast<float*>(h16_scales(d, q.m, q.k)), q.m, q.k, q.lda,
+                                       h16_tile_rows(q.m)});
+    else
+        pack_jobs_.push_back(UmmaPackJob{(const float2*)q.A, d, umma_tile_stride(q.k), q.m, q.k, q.lda, umma_nkb(q.k)});
     return packed_[key] = d;
 }
 
@@ -390,7 +404,7 @@ void Session::add_umma(const std::vector<GemmProblem>& P, const long long* xs, c
     std::vector<UmmaTile> tiles;
     for (size_t i = 0; i < P.size(); ++i) {
         const GemmProblem& q = P[i];
-        U.push_back(UmmaProblem{packed_operator(q), umma_tile_stride(q.k), q.m, q.k, umma_nkb(q.k), q.col0, q.ncol});
+        U.push_back(UmmaProblem{packed_operator(q, false), umma_tile_stride(q.k), q.m, q.k, umma_nkb(q.k), q.col0, q.ncol});
         for (int rt = 0; rt * 128 < q.m; ++rt)
             for (int c0 = 0; c0 < q.ncol; c0 += 128) {
                 tiles.push_back(UmmaTile{(int)i, rt, rt * 128, std::min(128, q.m - rt * 128), c0, 0});
@@ -428,6 +442,15 @@ static std::vector<char> i8_choose(const std::vector<std::array<int, 3> >& shape
     return on;
 }
 
+// first granule of each gathered column's vector (Digits)
+static std::vector<int> granules(const long long* xs, size_t ncols, long long base, int unit, int gran) {
+    std::vector<int> xg(ncols);
+    host_parallel_for((ncols + 65535) / 65536, [&](size_t c) {
+        for (size_t j = c * 65536; j < std::min(ncols, (c + 1) * 65536); ++j) xg[j] = (int)((xs[j] - base) / unit) * gran;
+    });
+    return xg;
+}
+
 // int8 form of one grouped GEMM launch: the operators packed as digits (now: they
 // are on the device).
 void Session::add_i8(const std::vector<GemmProblem>& P, const long long* xs, const long long* ys, size_t ncols,
@@ -450,11 +473,7 @@ void Session::add_i8(const std::vector<GemmProblem>& P, const long long* xs, con
         B += i8_packed_bytes(q.m, q.k);
         ra += q.m;
     }
-    std::vector<int> xg(ncols);
-    host_parallel_for((ncols + 65535) / 65536, [&](size_t c) {
-        for (size_t j = c * 65536; j < std::min(ncols, (c + 1) * 65536); ++j)
-            xg[j] = (int)((xs[j] - dg.base) / dg.unit) * dg.gran;
-    });
+    const std::vector<int> xg = granules(xs, ncols, dg.base, dg.unit, dg.gran);
     if (!d_err_) {
         d_err_ = dalloc<int>(1);
         CK(cudaMemsetAsync(d_err_, 0, sizeof(int), stream_));
@@ -464,20 +483,40 @@ void Session::add_i8(const std::vector<GemmProblem>& P, const long long* xs, con
     launch_i8_pack(dj, (int)jobs.size(), max_tiles, stream_);
     CK(cudaGetLastError());
     st.kind = 8;
-    st.i8 = I8Sub{upload(tiles), upload(xg), upload_n(ys, ncols), dg.X8, dg.cx, Y, (int)tiles.size()};
+    st.i8 = I8Sub{upload(tiles), upload(xg), upload_n(ys, ncols), dg.X8, (const double*)dg.cx, Y, (int)tiles.size()};
 }
 
-// The digits of the given vectors of X, for the int8 GEMMs that gather them.
+// FP16 form of one grouped GEMM launch of the mixed form's high-frequency passes
+// (kernels_h16.cu), tiles of one problem adjacent as in add_umma.
+void Session::add_h16(const std::vector<GemmProblem>& P, const long long* xs, const long long* ys, size_t ncols,
+                      double2* Y, const Digits& dg, Step& st) {
+    std::vector<H16Tile> tiles;
+    for (const GemmProblem& q : P) h16_tiles(packed_operator(q, true), q.m, q.k, q.col0, q.ncol, tiles);
+    for (const H16Tile& t : tiles) st.uop.push_back(t.B);
+    st.kind = 10;
+    st.hh = HSub{upload(tiles), upload(granules(xs, ncols, dg.base, dg.unit, dg.gran)), upload_n(ys, ncols), dg.X8,
+                 (const float*)dg.cx, reinterpret_cast<float2*>(Y), (int)tiles.size(), 0};
+    set_multi(st, st.hh, (int)tiles.size());
+}
+
+// The digits (mixed form: FP16 planes) of the given vectors of X, for the GEMMs that gather them.
 void Session::add_digits(const std::vector<I8Vec>& vecs, const double2* X, const Digits& dg, const char* label) {
     Step st{};
     st.kind = 7;
     st.label = label;
-    for (const I8Vec& v : vecs) st.bytes += 30.0 * v.len;
+    for (const I8Vec& v : vecs) st.bytes += (umma() ? 16.0 : 30.0) * v.len;
+    if (umma()) {
+        st.kind = 9;
+        st.hs = HSliceSub{upload(vecs), reinterpret_cast<const float2*>(X), dg.X8, (float*)dg.cx, (int)vecs.size(), 0};
+        set_multi(st, st.hs, st.hs.n);
+        push_step(st);
+        return;
+    }
     st.dg.vecs = upload(vecs);
     st.dg.n = (int)vecs.size();
     st.dg.X = X;
     st.dg.X8 = dg.X8;
-    st.dg.cx = dg.cx;
+    st.dg.cx = (double*)dg.cx;
     push_step(st);
 }
 
@@ -499,8 +538,8 @@ void Session::begin_block(int phase, double W) {
 
 void Session::push_step(Step st) {
     // step types in the order the blocks emit them
-    static const char* const order[] = {"lf_s2m",       "lf_m2m",       "lf_uc2ue", "hf_m2m",   "hf_m2l",
-                                        "hf_l2l",       "lf_vlist_fft", "lf_vlist_m2l", "lf_vlist_inv",
+    static const char* const order[] = {"lf_s2m",       "lf_m2m",       "lf_uc2ue", "lf_digits", "hf_m2m",
+                                        "hf_digits_up", "hf_m2l",       "hf_digits_down", "hf_l2l", "lf_vlist_fft", "lf_vlist_m2l", "lf_vlist_inv",
                                         "lf_xlist",     "lf_ulist",     "lf_wlist", "lf_dc2de", "lf_l2t", "lf_l2l"};
     std::string base(st.label);
     const size_t u = base.rfind("_w");
@@ -518,16 +557,25 @@ void Session::push_step(Step st) {
 
 void Session::flush_packs() {
     flush_uploads();
-    if (pack_jobs_.empty()) return;
-    UmmaPackJob* d = nullptr;
-    CK(cudaMalloc(&d, sizeof(UmmaPackJob) * pack_jobs_.size()));
-    CK(cudaMemcpyAsync(d, pack_jobs_.data(), sizeof(UmmaPackJob) * pack_jobs_.size(), cudaMemcpyHostToDevice,
-                       stream_));
-    launch_umma_pack(d, (int)pack_jobs_.size(), stream_);
+    if (pack_jobs_.empty() && h16_jobs_.empty()) return;
+    auto to_device = [&](const void* p, size_t bytes) {
+        void* d = nullptr;
+        CK(cudaMalloc(&d, std::max<size_t>(bytes, 16)));
+        if (bytes) CK(cudaMemcpyAsync(d, p, bytes, cudaMemcpyHostToDevice, stream_));
+        return d;
+    };
+    void* d = to_device(pack_jobs_.data(), sizeof(UmmaPackJob) * pack_jobs_.size());
+    launch_umma_pack(static_cast<const UmmaPackJob*>(d), (int)pack_jobs_.size(), stream_);
+    void* dh = to_device(h16_jobs_.data(), sizeof(H16PackJob) * h16_jobs_.size());
+    int max_tiles = 1;
+    for (const H16PackJob& j : h16_jobs_) max_tiles = std::max(max_tiles, h16_row_tiles(j.m));
+    launch_h16_pack(static_cast<const H16PackJob*>(dh), (int)h16_jobs_.size(), max_tiles, stream_);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(stream_));
     CK(cudaFree(d));
+    CK(cudaFree(dh));
     pack_jobs_.clear();
+    h16_jobs_.clear();
     // packed and complete: other sessions may use them from now on
     for (auto& kp : to_publish_) OpCache::publish(kp.first, kp.second);
     to_publish_.clear();
@@ -805,6 +853,7 @@ void Session::build() {
     cgemm_init();
     if (umma()) {
         umma_init();
+        h16_init();
         d_err_ = dalloc<int>(1);
         CK(cudaMemsetAsync(d_err_, 0, sizeof(int), stream_));
     }
@@ -1435,19 +1484,24 @@ void Session::build() {
     HfColumns cols = hf_columns(T, up, dn, kids, lf_off, dirpts.size(), hfcanon.size(), false);
     phase("hf_columns");
     // ---------------------------------------------------------------- digits of the HF inputs
-    // (plain form) of the launches with problems large enough for the int8 path
+    // plain form: of the launches with problems large enough for the int8 path; tcgen05
+    // form: FP16 planes, of all
     Digits lf_dg, up_dg, dn_dg;
     std::map<int, std::vector<char> > m2m_i8, m2l_i8, l2l_i8;  // level -> problems on the int8 path
     std::set<int> up_i8, dn_i8;  // levels whose outgoing / incoming vectors are written as digits
     bool lf_i8 = false;
-    if (!mixed) {
+    if (!mixed || umma()) {
+        auto choose = [&](const std::vector<std::array<int, 3> >& shapes) {
+            return umma() ? std::vector<char>(shapes.size(), 1) : i8_choose(shapes);
+        };
         long long dn_most = 0;
         for (auto& kv : hflevels) {
             const int level = kv.first;
             const double W = T.width(level);
             auto shapes = [&](const ColLists& L, const std::map<std::pair<double, Idx3>, DirMats>& mats) {
                 std::vector<std::array<int, 3> > v;
-                for (size_t i = 0; i < L.key.size(); ++i) {
+                if (umma()) v.resize(L.key.size());  // all of them
+                for (size_t i = v.size(); i < L.key.size(); ++i) {
                     const DirMats& M = mats.at(std::make_pair(W, did_wedge[L.key[i] / 8].second));
                     v.push_back({{M.mrows, M.mcols, (int)L.x[i].size()}});
                 }
@@ -1458,9 +1512,9 @@ void Session::build() {
                 const int r1 = m2l_mats[m2l_probs[level][i]].r1;
                 far.push_back({{r1, r1, (int)m2l_x[level][i].size()}});
             }
-            m2m_i8[level] = i8_choose(shapes(cols.m2m.at(level), m2m_mats));
-            m2l_i8[level] = i8_choose(far);
-            l2l_i8[level] = i8_choose(shapes(cols.l2l.at(level), l2l_mats));
+            m2m_i8[level] = choose(shapes(cols.m2m.at(level), m2m_mats));
+            m2l_i8[level] = choose(far);
+            l2l_i8[level] = choose(shapes(cols.l2l.at(level), l2l_mats));
             if (!m2m_i8[level].empty()) {
                 if (W == 1.0)
                     lf_i8 = true;
@@ -1475,7 +1529,7 @@ void Session::build() {
             }
         }
         auto room = [&](Digits& d, size_t granules) {
-            d.X8 = dalloc<char>(granules * I8_GRANULE);
+            d.X8 = dalloc<char>(granules * (umma() ? H16_GRANULE : I8_GRANULE));
             d.cx = dalloc<double>(granules);
         };
         lf_dg.unit = nE;
@@ -1483,7 +1537,7 @@ void Session::build() {
         if (lf_i8) room(lf_dg, (size_t)nLF * lf_dg.gran);
         if (!up_i8.empty()) room(up_dg, (size_t)upeq_total / 16);
         if (!dn_i8.empty()) room(dn_dg, (size_t)dn_most / 16);
-        if (lf_i8 || !up_i8.empty() || !dn_i8.empty()) i8_init();
+        if (!mixed && (lf_i8 || !up_i8.empty() || !dn_i8.empty())) i8_init();
     }
     auto node_vecs = [&](const HfNodes& N, int level, const Digits& d) {
         const auto r = N.range.at(level);
@@ -1838,6 +1892,8 @@ static const char* kernel_name(int kind, int tpi, bool narrow) {
         case 6: return "vlist_inverse_kernel";
         case 7: return "i8_slice_kernel";
         case 8: return "i8_gemm_kernel";
+        case 9: return "h16_slice_kernel";
+        case 10: return "h16_gemm_kernel";
         default: return "umma_cgemm_kernel";
     }
 }
@@ -1883,6 +1939,12 @@ void Session::launch_step(const Step& st, cudaStream_t s, double2* spec) {
             break;
         case 7: launch_i8_slice(st.dg.vecs, st.dg.n, st.dg.X, st.dg.X8, st.dg.cx, s); break;
         case 8: launch_i8_gemm(st.i8, d_err_, s); break;
+        case 9:
+            launch_h16_slice(static_cast<const HSliceSub*>(st.msubs), st.mpre, 1, st.mtotal, nullptr, s, st.hs);
+            break;
+        case 10:
+            launch_h16_gemm(static_cast<const HSub*>(st.msubs), st.mpre, 1, st.mtotal, nullptr, d_err_, s, st.hh);
+            break;
         case 5: {
             const unsigned long long wait_ns = stall_wait_ns_;
             stall_wait_ns_ = 0;  // one launch only

@@ -130,18 +130,19 @@ private:
         char* X8 = nullptr;
         double* cx = nullptr;
     };
-    // The digits of a GEMM launch's input array: element offset o of a vector is
-    // granule (o - base) / unit * gran of X8.
+    // The digits (plain form) or FP16 planes (mixed form) of a GEMM launch's input
+    // array: element offset o of a vector is granule (o - base) / unit * gran of X8.
     struct Digits {
         char* X8 = nullptr;
-        double* cx = nullptr;
+        void* cx = nullptr;  // double or float per granule
         long long base = 0;
         int unit = 16, gran = 1;
     };
     // one step of the eval: exactly one of these is used
     struct Step {
         int kind;  // 0 gemm, 1 pt, 2 vfwd, 3 V-list sums, 5 tcgen05 gemm, 6 V-list inverse,
-                   // 7 digits of vectors, 8 int8 tcgen05 gemm
+                   // 7 digits of vectors, 8 int8 tcgen05 gemm, 9 FP16 planes of vectors,
+                   // 10 FP16 tcgen05 gemm
         const char* label;  // pass name for profiling
         double flops;       // algorithmic flops of the launch
         double bytes;       // algorithmic DRAM bytes of the launch
@@ -164,6 +165,8 @@ private:
         int* mpre;
         int mtotal;
         UmmaSub hu;
+        HSliceSub hs;
+        HSub hh;
         std::vector<const float*> uop;  // tcgen05 GEMM: each tile's packed operator block (batch tile order)
         PtSub hp;
         VfSub hvf;
@@ -193,12 +196,14 @@ private:
     void add_gemm(std::vector<GemmProblem>& probs, std::vector<std::vector<long long> >& xo,
                   std::vector<std::vector<long long> >& yo, const double2* X, double2* Y, int mode,
                   const char* label, const Digits* dg = nullptr, const std::vector<char>* on_i8 = nullptr);
-    const Digits* i8_target_ = nullptr;  // set while add_gemm emits the int8 part of a launch
+    const Digits* i8_target_ = nullptr;  // set while add_gemm emits the int8 (mixed form: FP16) part of a launch
     bool narrow_ = false;                // set while it emits the products with few columns
     void add_i8(const std::vector<GemmProblem>& P, const long long* xs, const long long* ys, size_t ncols, double2* Y,
                 const Digits& dg, Step& st);
     void add_digits(const std::vector<I8Vec>& vecs, const double2* X, const Digits& dg, const char* label);
-    const float* packed_operator(const GemmProblem& q);
+    void add_h16(const std::vector<GemmProblem>& P, const long long* xs, const long long* ys, size_t ncols, double2* Y,
+                 const Digits& dg, Step& st);
+    const float* packed_operator(const GemmProblem& q, bool h16);
     void add_umma(const std::vector<GemmProblem>& P, const long long* xs, const long long* ys, size_t ncols,
                   const double2* X, double2* Y, int mode, Step& st);
     void flush_packs();
@@ -271,6 +276,7 @@ private:
     unsigned long long stall_wait_ns_ = 0;  // armed failure-path hook (0: none)
     std::map<std::pair<const void*, long long>, const float*> packed_;  // (operator, m k) -> packed copy
     std::vector<UmmaPackJob> pack_jobs_;
+    std::vector<H16PackJob> h16_jobs_;
     // setup trace: host seconds in add_gemm, vlist_groups, uploads above kArenaMax,
     // packed_operator, and of that in packed-operator chunk allocations
     double t_emit_gemm_ = 0, t_emit_vgroups_ = 0, t_big_uploads_ = 0, t_pack_ = 0, t_pack_alloc_ = 0;

@@ -164,10 +164,11 @@ int ddfmm_session_test_gemm_stall(ddfmm_session* s, double wait_s);
 
 /* Test entry point, no counterpart in the reference: Y += A X (A m x k, X k x
  * ncol, Y m x ncol, column-major complex128 host arrays; m, k <= 400) on the
- * current device through a translation kernel of the PLAIN_FP64 form -- path
- * 0: the FP64 tensor path, 1: the int8 tensor path (exact integer products of
- * digit planes), 2: the FP64 tensor path for few columns.  Columns are gathered
- * and scattered as an eval's are. */
+ * current device through a translation kernel -- path 0: the FP64 tensor path,
+ * 1: the int8 tensor path (exact integer products of digit planes), 2: the FP64
+ * tensor path for few columns (PLAIN_FP64 form); 3: the FP16 tensor path (two
+ * planes per number), 4: split TF32 (MIXED form, on FP32 copies).  Columns are
+ * gathered and scattered as an eval's are. */
 int ddfmm_test_gemm(const double* A, int m, int k, const double* X, int ncol, int path, double* Y);
 
 /* Host-only (no GPU): build the octree and interaction lists of
