@@ -272,8 +272,9 @@ def gemm_traffic(kernel, algorithmic_bytes):
 
 def measure_mixed(w, wave_args, steps, warmup, dev, chk, ws, profile_json=None, precision=None):
     """The mixed-precision form on the same workload: complex64 densities on
-    the device, 3xTF32 translations (tcgen05 by default, or the mma.sync
-    path); reports matvec/s, its error vs the FP64 direct sum and latency
+    the device, split-product translations (tcgen05 by default: two FP16 planes a
+    number in the high-frequency passes, 3xTF32 in the others; or the mma.sync
+    3xTF32 path); reports matvec/s, its error vs the FP64 direct sum and latency
     percentiles."""
     import torch
     from ddfmm_b200 import _lib, wave3d
@@ -326,7 +327,7 @@ def measure_mixed(w, wave_args, steps, warmup, dev, chk, ws, profile_json=None, 
     m.profile(False)
     gk = {"launches": 0, "ms": 0.0, "flops": 0.0, "bytes": 0.0}
     for e in prof.values():
-        if e["kernel"] in ("umma_cgemm_kernel", "zgemm_kernel"):
+        if e["kernel"] == ("h16_gemm_kernel" if precision == _lib.MIXED else "zgemm_kernel"):
             gk["launches"] += e["launches"]
             gk["ms"] += e["ms"]
             gk["flops"] += e["flops"]
@@ -335,12 +336,14 @@ def measure_mixed(w, wave_args, steps, warmup, dev, chk, ws, profile_json=None, 
     if gk["ms"] > 0:
         peaks = measured_peaks()
         algo = gk["flops"] / (gk["ms"] * 1e-3) / 1e12  # complex flops (8 per complex MAC) / s
-        executed = 3.0 * algo  # 3xTF32: three TF32 products per complex product
-        if "bf16_tflops_sustained" in peaks:
-            peak, src = peaks["bf16_tflops_sustained"] / 2, "MEASURED_PEAKS.json bf16_tflops_sustained / 2"
-        else:
-            peak, src = 1400.0 / 2, "fallback 1.4 PFLOP/s bf16 sustained / 2"
-        kname = "umma_cgemm_kernel" if precision == _lib.MIXED else "cgemm_kernel"
+        executed = 3.0 * algo  # three FP16 (mma.sync: TF32) products per product
+        h16 = precision == _lib.MIXED
+        peak, src = peaks.get("bf16_tflops_sustained"), "MEASURED_PEAKS.json bf16_tflops_sustained"
+        if peak is None:
+            peak, src = 1400.0, "fallback 1.4 PFLOP/s bf16 sustained"
+        if not h16:
+            peak, src = peak / 2, src + " / 2"
+        kname = "h16_gemm_kernel" if h16 else "cgemm_kernel"
         roof = {"bound": "tensor", "kernel": kname,
                 "achieved": executed, "peak": peak, "unit": "TFLOP/s", "frac": executed / peak,
                 "traffic": gemm_traffic(kname, 0.5 * gk["bytes"] / max(1, gk["launches"])),
@@ -350,14 +353,15 @@ def measure_mixed(w, wave_args, steps, warmup, dev, chk, ws, profile_json=None, 
                                 "(profiles/gemm_dram_traffic_sphere_K16_P6.txt)",
                 "algorithmic_bytes": 0.5 * gk["bytes"] / max(1, gk["launches"]),
                 "algorithmic_complex_tflops": algo, "launches": gk["launches"] // 3,
-                "peak_source": src + " (dense TF32 runs at half the BF16 rate on B200's tensor cores)",
-                "note": "executed = 3 x algorithmic (hi*hi + lo*hi + hi*lo TF32 products)"}
+                "peak_source": src + (" (dense FP16 runs at the BF16 rate)" if h16 else
+                                      " (dense TF32 runs at half the BF16 rate on B200's tensor cores)"),
+                "note": "executed = 3 x algorithmic (hi*hi + lo*hi + hi*lo products)"}
     m.close()
     gemm = "tcgen05" if precision == _lib.MIXED else "mma.sync"
     passes = {lab: {"ms_per_step": e["ms"] / 3, "launches_per_step": e["launches"] / 3, "kernel": e["kernel"]}
               for lab, e in sorted(prof.items(), key=lambda kv: -kv[1]["ms"])}
     return {"value": whole_job_rate(ms, ws), "unit": "matvec/s", "ms_per_step": ms,
-            "dtype": "c64 (3xTF32 translations on %s)" % gemm,
+            "dtype": "c64 (%s translations on %s)" % ("2 x FP16 plane" if precision == _lib.MIXED else "3xTF32", gemm),
             "relerr_vs_fp64_direct": relerr, "setup_s": setup_s, "roofline": roof,
             "latency_ms": {"p50": float(np.percentile(lat, 50)), "p99": float(np.percentile(lat, 99))},
             "passes": passes}
@@ -726,6 +730,7 @@ def run_ours(args):
         algo = dk["flops"] / (dk["ms"] * 1e-3) / 1e12
         roof = {"bound": "tensor", "pipe": "int8 (tcgen05.mma kind::i8)", "kernel": dom, "achieved": 34 * algo,
                 "peak": peak, "unit": "TOP/s", "frac": 34 * algo / peak, "algorithmic_fp64_tflops": algo,
+                "traffic": gemm_traffic(dom, dk["bytes"] / max(1, dk["launches"])),
                 "algorithmic_bytes": dk["bytes"] / max(1, dk["launches"]),
                 "peak_source": src + " (dense int8 runs at twice the BF16 rate)",
                 "launches": dk["launches"]}
