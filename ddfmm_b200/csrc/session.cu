@@ -442,9 +442,9 @@ static std::vector<char> i8_choose(const std::vector<std::array<int, 3> >& shape
     return on;
 }
 
-// first granule of each gathered column's vector (Digits)
-static std::vector<int> granules(const long long* xs, size_t ncols, long long base, int unit, int gran) {
-    std::vector<int> xg(ncols);
+// first granule of each gathered column's vector (Digits); not zeroed first
+static std::unique_ptr<int[]> granules(const long long* xs, size_t ncols, long long base, int unit, int gran) {
+    std::unique_ptr<int[]> xg(new int[std::max<size_t>(ncols, 1)]);
     host_parallel_for((ncols + 65535) / 65536, [&](size_t c) {
         for (size_t j = c * 65536; j < std::min(ncols, (c + 1) * 65536); ++j) xg[j] = (int)((xs[j] - base) / unit) * gran;
     });
@@ -473,7 +473,7 @@ void Session::add_i8(const std::vector<GemmProblem>& P, const long long* xs, con
         B += i8_packed_bytes(q.m, q.k);
         ra += q.m;
     }
-    const std::vector<int> xg = granules(xs, ncols, dg.base, dg.unit, dg.gran);
+    const std::unique_ptr<int[]> xg = granules(xs, ncols, dg.base, dg.unit, dg.gran);
     if (!d_err_) {
         d_err_ = dalloc<int>(1);
         CK(cudaMemsetAsync(d_err_, 0, sizeof(int), stream_));
@@ -483,7 +483,7 @@ void Session::add_i8(const std::vector<GemmProblem>& P, const long long* xs, con
     launch_i8_pack(dj, (int)jobs.size(), max_tiles, stream_);
     CK(cudaGetLastError());
     st.kind = 8;
-    st.i8 = I8Sub{upload(tiles), upload(xg), upload_n(ys, ncols), dg.X8, (const double*)dg.cx, Y, (int)tiles.size()};
+    st.i8 = I8Sub{upload(tiles), upload_n(xg.get(), ncols), upload_n(ys, ncols), dg.X8, (const double*)dg.cx, Y, (int)tiles.size()};
 }
 
 // FP16 form of one grouped GEMM launch of the mixed form's high-frequency passes
@@ -494,26 +494,27 @@ void Session::add_h16(const std::vector<GemmProblem>& P, const long long* xs, co
     for (const GemmProblem& q : P) h16_tiles(packed_operator(q, true), q.m, q.k, q.col0, q.ncol, tiles);
     for (const H16Tile& t : tiles) st.uop.push_back(t.B);
     st.kind = 10;
-    st.hh = HSub{upload(tiles), upload(granules(xs, ncols, dg.base, dg.unit, dg.gran)), upload_n(ys, ncols), dg.X8,
+    const std::unique_ptr<int[]> xg = granules(xs, ncols, dg.base, dg.unit, dg.gran);
+    st.hh = HSub{upload(tiles), upload_n(xg.get(), ncols), upload_n(ys, ncols), dg.X8,
                  (const float*)dg.cx, reinterpret_cast<float2*>(Y), (int)tiles.size(), 0};
     set_multi(st, st.hh, (int)tiles.size());
 }
 
 // The digits (mixed form: FP16 planes) of the given vectors of X, for the GEMMs that gather them.
-void Session::add_digits(const std::vector<I8Vec>& vecs, const double2* X, const Digits& dg, const char* label) {
+void Session::add_digits(const I8Vec* vecs, size_t n, const double2* X, const Digits& dg, const char* label) {
     Step st{};
     st.kind = 7;
     st.label = label;
-    for (const I8Vec& v : vecs) st.bytes += (umma() ? 16.0 : 30.0) * v.len;
+    for (size_t i = 0; i < n; ++i) st.bytes += (umma() ? 16.0 : 30.0) * vecs[i].len;
     if (umma()) {
         st.kind = 9;
-        st.hs = HSliceSub{upload(vecs), reinterpret_cast<const float2*>(X), dg.X8, (float*)dg.cx, (int)vecs.size(), 0};
+        st.hs = HSliceSub{upload_n(vecs, n), reinterpret_cast<const float2*>(X), dg.X8, (float*)dg.cx, (int)n, 0};
         set_multi(st, st.hs, st.hs.n);
         push_step(st);
         return;
     }
-    st.dg.vecs = upload(vecs);
-    st.dg.n = (int)vecs.size();
+    st.dg.vecs = upload_n(vecs, n);
+    st.dg.n = (int)n;
     st.dg.X = X;
     st.dg.X8 = dg.X8;
     st.dg.cx = (double*)dg.cx;
@@ -1539,16 +1540,17 @@ void Session::build() {
         if (!dn_i8.empty()) room(dn_dg, (size_t)dn_most / 16);
         if (!mixed && (lf_i8 || !up_i8.empty() || !dn_i8.empty())) i8_init();
     }
-    auto node_vecs = [&](const HfNodes& N, int level, const Digits& d) {
+    auto add_node_digits = [&](const HfNodes& N, int level, const double2* X, const Digits& d, const char* label) {
         const auto r = N.range.at(level);
-        std::vector<I8Vec> v((size_t)(r.second - r.first));
-        host_parallel_for((v.size() + 16383) / 16384, [&](size_t c) {
-            for (size_t i = c * 16384; i < std::min(v.size(), (c + 1) * 16384); ++i) {
+        const size_t n = (size_t)(r.second - r.first);
+        std::unique_ptr<I8Vec[]> v(new I8Vec[n]);  // not zeroed first
+        host_parallel_for((n + 16383) / 16384, [&](size_t c) {
+            for (size_t i = c * 16384; i < std::min(n, (c + 1) * 16384); ++i) {
                 const HfNode& u = N.v[r.first + i];
                 v[i] = I8Vec{u.off, (int)((u.off - d.base) / 16), hfcanon[u.canon].r1};
             }
         });
-        return v;
+        add_digits(v.get(), n, X, d, label);
     };
     // ---------------------------------------------------------------- steps: HF upward
     // widths ascending = levels descending; hf_upeq holds w (upeqnden = E1 w)
@@ -1561,7 +1563,7 @@ void Session::build() {
         if (W == 1.0 && lf_i8) {
             std::vector<I8Vec> v;
             for (int l : lflevels[level + 1]) v.push_back(I8Vec{(long long)l * nE, l * lf_dg.gran, nE});
-            add_digits(v, lf_upeq, lf_dg, "lf_digits");
+            add_digits(v.data(), v.size(), lf_upeq, lf_dg, "lf_digits");
         }
         // M2M: w = sum_children [E2 E3 ue2uc E1(child)] w_child (src/wave3d_eval.cpp:796-849),
         // one launch for the 8 child positions: a problem per (wedge, child), all adding into
@@ -1583,7 +1585,7 @@ void Session::build() {
             add_gemm(probs, L.x, L.y, W == 1.0 ? lf_upeq : hf_upeq, hf_upeq, GEMM_ATOMIC, width_label("hf_m2m", W),
                      W == 1.0 ? &lf_dg : &up_dg, &m2m_i8[level]);
         }
-        if (up_i8.count(level)) add_digits(node_vecs(up, level, up_dg), hf_upeq, up_dg, "hf_digits_up");
+        if (up_i8.count(level)) add_node_digits(up, level, hf_upeq, up_dg, "hf_digits_up");
     }
 
     phase("steps_hf_up");
@@ -1612,7 +1614,7 @@ void Session::build() {
         }
         if (dn_i8.count(level)) {
             dn_dg.base = dn.v[dr.first].off;  // one level's digits at a time
-            add_digits(node_vecs(dn, level, dn_dg), hf_dnchk, dn_dg, "hf_digits_down");
+            add_node_digits(dn, level, hf_dnchk, dn_dg, "hf_digits_down");
         }
         // L2L into the children's (pdir) u, or LF dnchkval at W=1 (src/wave3d_eval.cpp:938-991),
         // one launch for the 8 child positions: a problem per (wedge, child)

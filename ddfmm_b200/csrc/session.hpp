@@ -200,7 +200,7 @@ private:
     bool narrow_ = false;                // set while it emits the products with few columns
     void add_i8(const std::vector<GemmProblem>& P, const long long* xs, const long long* ys, size_t ncols, double2* Y,
                 const Digits& dg, Step& st);
-    void add_digits(const std::vector<I8Vec>& vecs, const double2* X, const Digits& dg, const char* label);
+    void add_digits(const I8Vec* vecs, size_t n, const double2* X, const Digits& dg, const char* label);
     void add_h16(const std::vector<GemmProblem>& P, const long long* xs, const long long* ys, size_t ncols, double2* Y,
                  const Digits& dg, Step& st);
     const float* packed_operator(const GemmProblem& q, bool h16);
