@@ -197,9 +197,8 @@ Session::~Session() {
     stage_release();
     for (cudaEvent_t e : ev_) cudaEventDestroy(e);
     for (void* p : allocs_) cudaFree(p);
-    for (cudaEvent_t e : {fork_, lf_up_, join_})
-        if (e) cudaEventDestroy(e);
-    if (side_) cudaStreamDestroy(side_);
+    for (cudaEvent_t e : branch_ev_) cudaEventDestroy(e);
+    for (cudaStream_t b : branch_) cudaStreamDestroy(b);
     if (graph_) cudaGraphExecDestroy(graph_);
     if (stream_) cudaStreamDestroy(stream_);
 }
@@ -1641,10 +1640,12 @@ void Session::build() {
     // Small instances do not fill the GPU in any pass: their V-list sums and near field
     // run beside the high-frequency passes (run_steps).  The line is the size of the
     // summed target spectra, which then need memory of their own.
-    overlap_ = !hflevels.empty() && (size_t)nLF * G3 * es <= ((size_t)128 << 20);
+    overlap_ = !hflevels.empty() && !lflevels.empty() && (size_t)nLF * G3 * es <= ((size_t)128 << 20);
     if (overlap_) {
-        CK(cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking));
-        for (cudaEvent_t* e : {&fork_, &lf_up_, &join_}) CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+        branch_.resize(std::min<size_t>(lflevels.size(), kBranches));
+        for (cudaStream_t& b : branch_) CK(cudaStreamCreateWithFlags(&b, cudaStreamNonBlocking));
+        branch_ev_.resize(2 + 2 * branch_.size() + 2 * lflevels.size());
+        for (cudaEvent_t& e : branch_ev_) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
     // ---------------------------------------------------------------- steps: LF downward
     for (auto& kv : lflevels) {  // levels ascending = widths descending
@@ -1652,6 +1653,9 @@ void Session::build() {
         const LfLevelOps& L = lfops[level];
         const auto& ids = kv.second;
         double W = L.W;
+        // the widest level's check values also receive the high-frequency L2L, atomically:
+        // what adds to them otherwise waits for it on the main stream
+        const Step::Lane below = kv.first == lflevels.begin()->first ? Step::MAIN : Step::SIDE_LATE;
         begin_block(3, W);
         // V list: FFT M2L (src/wave3d_eval.cpp:602-661).  The pointwise sums run by
         // target parent (kernels.cuh, VlistGroups): the targets of a parent share one
@@ -1712,7 +1716,7 @@ void Session::build() {
                     set_multi(a, a.hva, ngroups);
                 }
                 push_step(a);
-                lane_ = Step::MAIN;
+                lane_ = below;
                 Step iv{};
                 iv.kind = 6;
                 iv.label = "lf_vlist_inv";
@@ -1729,6 +1733,7 @@ void Session::build() {
                     set_multi(iv, iv.hvi, iv.v.ntrg);
                 }
                 push_step(iv);
+                lane_ = Step::MAIN;
             }
         }
         // X list (src/wave3d_eval.cpp:663-686), into dnchk or, for small leaves, into extval
@@ -1754,8 +1759,9 @@ void Session::build() {
             }
             lane_ = Step::SIDE_EARLY;
             add_pt(itemsA, srcsA, "lf_xlist");
-            lane_ = Step::MAIN;
+            lane_ = below;
             add_pt(itemsB, srcsB, "lf_xlist");
+            lane_ = Step::MAIN;
         }
         // U list (src/wave3d_eval.cpp:585-600) and W list (:688-718) into extval
         {
@@ -2029,28 +2035,77 @@ void Session::run_steps(cudaStream_t s) {
     }
 }
 
-// The steps on two streams.  Side stream: U and direct X lists at once, V-list
-// transforms and sums and W lists once the upward low-frequency passes are done
-// (they only read points, densities and outgoing LF densities); each adds into
-// values that nothing on the caller's stream touches before the join, where the
-// downward low-frequency passes begin.  Works on a capturing stream: the side
-// stream joins the capture at the fork and leaves it at the join.
+// The steps with a branch (stream) per low-frequency level beside the caller's
+// stream.  A level's branch runs, in the serial order, its S2M (the finest level's
+// stays on the main stream, which starts with it), its U and direct X lists, and once
+// the upward low-frequency passes are done its V-list transforms and sums, W list and,
+// below the widest level, what adds into its check values; then its L2T, once the main
+// stream has the level's densities.  Every one of them writes values, check values or
+// spectra of its own level's boxes, and before the join nothing on the main stream
+// touches those.  Works on a capturing stream: the branches join the capture at the
+// fork and leave it at the last join.  An adaptive tree of five levels (cluster, K = 8)
+// takes 530 us with one side stream for all levels, 496 with a branch each (a first,
+// cold eval 907 and 728).
 void Session::run_overlapped(cudaStream_t s) {
-    CK(cudaEventRecord(fork_, s));
-    CK(cudaStreamWaitEvent(side_, fork_, 0));
+    const size_t nb = branch_.size();
+    auto level = [](const Step& st) {  // 0 for the widest
+        const int w = (int)((st.key >> 32) & 0xffff);
+        return (st.key >> 48) < 2 ? 999 - w : w - 1001;
+    };
+    auto branch = [&](const Step& st) { return branch_[(size_t)level(st) % nb]; };
+    size_t used = 0;
+    auto after = [&](cudaStream_t to, cudaStream_t from) {  // `to` goes on once `from` has come here
+        CK(cudaEventRecord(branch_ev_[used], from));
+        CK(cudaStreamWaitEvent(to, branch_ev_[used], 0));
+        ++used;
+    };
+    auto all_after = [&]() {
+        CK(cudaEventRecord(branch_ev_[used], s));
+        for (cudaStream_t b : branch_) CK(cudaStreamWaitEvent(b, branch_ev_[used], 0));
+        ++used;
+    };
+    const int finest = level(steps_[0]);
+    auto apart = [&](const Step& st) {  // S2M of the levels that others come before, L2T of those that others follow
+        const int pass = (int)(st.key >> 48);
+        return st.kind == 1 && level(st) != finest && (pass == 0 || (pass == 3 && !std::strcmp(st.label, "lf_l2t")));
+    };
+    all_after();
+    std::map<int, size_t> s2m;  // level -> event
     for (const Step& st : steps_)
-        if (st.lane == Step::SIDE_EARLY) launch_step(st, side_, st.v.spec);
+        if ((st.key >> 48) == 0 && apart(st)) {
+            launch_step(st, branch(st), st.v.spec);
+            CK(cudaEventRecord(branch_ev_[used], branch(st)));
+            s2m[level(st)] = used++;
+        }
+    for (const Step& st : steps_)
+        if (st.lane == Step::SIDE_EARLY) launch_step(st, branch(st), st.v.spec);
     size_t i = 0;
-    for (; i < steps_.size() && (steps_[i].key >> 48) == 0; ++i) launch_step(steps_[i], s, steps_[i].v.spec);
-    CK(cudaEventRecord(lf_up_, s));
-    CK(cudaStreamWaitEvent(side_, lf_up_, 0));
+    for (; i < steps_.size() && (steps_[i].key >> 48) == 0; ++i) {
+        auto e = s2m.find(level(steps_[i]));
+        if (e != s2m.end()) {
+            CK(cudaStreamWaitEvent(s, branch_ev_[e->second], 0));
+            s2m.erase(e);
+        }
+        if (!apart(steps_[i])) launch_step(steps_[i], s, steps_[i].v.spec);
+    }
+    all_after();
     for (const Step& st : steps_)
-        if (st.lane == Step::SIDE_LATE) launch_step(st, side_, st.v.spec);
-    CK(cudaEventRecord(join_, side_));
+        if (st.lane == Step::SIDE_LATE) launch_step(st, branch(st), st.v.spec);
     for (; i < steps_.size() && (steps_[i].key >> 48) < 3; ++i) launch_step(steps_[i], s, steps_[i].v.spec);
-    CK(cudaStreamWaitEvent(s, join_, 0));
-    for (; i < steps_.size(); ++i)
-        if (steps_[i].lane == Step::MAIN) launch_step(steps_[i], s, steps_[i].v.spec);
+    for (cudaStream_t b : branch_) after(s, b);
+    std::set<cudaStream_t> open;  // branches with an L2T on them
+    for (; i < steps_.size(); ++i) {
+        const Step& st = steps_[i];
+        if (st.lane != Step::MAIN) continue;
+        if (!apart(st)) {
+            launch_step(st, s, st.v.spec);
+            continue;
+        }
+        after(branch(st), s);
+        launch_step(st, branch(st), st.v.spec);
+        open.insert(branch(st));
+    }
+    for (cudaStream_t b : open) after(s, b);
 }
 
 // Everything between the densities' gather and the values' scatter (whose arrays are

@@ -155,8 +155,8 @@ private:
         // that play the same part (phase, width, step type, occurrence): a Batch
         // merges the steps of its sessions that share a key into one launch.
         long long key;
-        // Stream of the step when an eval overlaps its passes (run_steps): the caller's, or
-        // the side stream from the eval's start or from the end of the upward LF passes
+        // Stream of the step when an eval overlaps its passes (run_overlapped): the caller's, or
+        // its level's branch from the eval's start or from the end of the upward LF passes
         enum Lane { MAIN = 0, SIDE_EARLY = 1, SIDE_LATE = 2 } lane;
         int tpi;  // point interactions: launch shape (launch_pt; 0 = 32 threads per item), set by autotune()
         // mixed form: the step as a one-instance launch (device sub-launch array and
@@ -256,9 +256,10 @@ private:
     void stage_release();  // after a stream sync
     std::vector<Step> steps_;
     Step::Lane lane_ = Step::MAIN;  // of the steps being emitted
-    bool overlap_ = false;          // small instance: passes overlap on two streams
-    cudaStream_t side_ = nullptr;
-    cudaEvent_t fork_ = nullptr, lf_up_ = nullptr, join_ = nullptr;
+    bool overlap_ = false;          // small instance: passes overlap on several streams
+    static constexpr size_t kBranches = 8;
+    std::vector<cudaStream_t> branch_;     // beside the caller's, by low-frequency level
+    std::vector<cudaEvent_t> branch_ev_;
     cudaGraphExec_t graph_ = nullptr;  // run_steps of a small instance, instantiated at setup
     cudaStream_t stream_ = nullptr;
     SessionStats stats_;
