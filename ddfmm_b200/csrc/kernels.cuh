@@ -215,7 +215,7 @@ void launch_gather32(const void* den, const int* perm, void* out, int n, int c64
 void launch_scatter32(const void* in, const int* perm, void* val, int n, int c64, cudaStream_t s);
 void launch_to_c64(const double2* a, float2* b, long long n, cudaStream_t s);
 
-// mixed-form GEMM on tcgen05 (kernels_umma.cu): 128 gathered columns x up to
+// mixed-form low-frequency GEMM on tcgen05 (kernels_umma.cu): 128 gathered columns x up to
 // 128 complex operator rows per tile, operator packed at setup as split TF32.
 struct UmmaProblem {
     const float* B;      // packed operator (umma_pack_kernel layout)

@@ -1,4 +1,5 @@
-// Mixed-form complex GEMM on the 5th-generation tensor cores (tcgen05, TMEM).
+// Mixed-form complex GEMM on the 5th-generation tensor cores (tcgen05, TMEM): the
+// low-frequency products (the high-frequency ones run in kernels_h16.cu).
 //
 // Problem (as in cgemm_kernel): Y[:, c] (op)= A * X[:, c] for gathered
 // columns c, A an m x k complex operator.  One tile is posed as the real GEMM

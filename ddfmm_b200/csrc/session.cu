@@ -394,7 +394,7 @@ const float* Session::packed_operator(const GemmProblem& q, bool h16) {
     return packed_[key] = d;
 }
 
-// tcgen05 form of one grouped GEMM launch: tiles of 128 gathered columns x
+// split-TF32 tcgen05 form of one grouped GEMM launch (low-frequency passes): tiles of 128 gathered columns x
 // 128 complex operator rows, the tiles of one problem adjacent so that blocks
 // in flight share its packed operator in L2.
 void Session::add_umma(const std::vector<GemmProblem>& P, const long long* xs, const long long* ys, size_t ncols,
