@@ -67,6 +67,11 @@ void test_gemm(const double2* A, int m, int k, const double2* X, int ncol, int p
         gemm_init();
         launch_gemm_narrow(P.put(std::vector<GemmProblem>(1, GemmProblem{dA, m, k, m, 0, ncol, nullptr})), P.put(tiles),
                            (int)tiles.size(), P.put(xo), dyo, dX, dY, GEMM_ATOMIC, k, rows, nullptr);
+    } else if (path == 5) {  // the identity, then A, at the offsets of both
+        if (m != k || m > GEMM_PAIR_MAX) throw std::invalid_argument("the pair kernel takes square operators of up to 64 rows");
+        std::vector<double2> one((size_t)m * m, make_double2(0, 0));
+        for (int i = 0; i < m; ++i) one[(size_t)i * m + i] = make_double2(1, 0);
+        launch_gemm_pair(GemmPair{P.put(one), dA, m, m, ncol, P.put(xo), dX, dY}, nullptr);
     } else if (path >= 3) {  // mixed form, on FP32 copies: 3 FP16 planes, 4 split TF32
         auto narrow = [](const std::vector<double2>& v) {
             std::vector<float2> r;

@@ -334,6 +334,39 @@ void launch_gemm(const GemmProblem* probs, const GemmTile* tiles, int ntiles, co
     zgemm_kernel<<<ntiles, 256, GEMM_SMEM, s>>>(probs, tiles, xoff, yoff, X, Y, mode);
 }
 
+// Fragment of rows row and row + 8, K step `step` of an m x k operator, zeros outside
+__device__ __forceinline__ void narrow_load(double2 (&a)[4], const double2* A, int m, int k, int lda, int row, int tig,
+                                            int step) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int j = step * 8 + tig + 4 * (q >> 1), r = row + 8 * (q & 1);
+        a[q] = j < k && r < m ? __ldg(A + (size_t)j * lda + r) : make_double2(0.0, 0.0);
+    }
+}
+// out = the warp's 16 rows x 8 columns (rows row, row + 8 x columns 2 tig, 2 tig + 1 of this
+// thread), a: the first K step's fragment, Xs: this thread's column of the staged block
+__device__ __forceinline__ void narrow_product(double2 (&out)[4], double2 (&a)[4], const double2* A, int m, int k, int lda,
+                                               int row, int tig, const double2* Xs) {
+    double cr[4] = {0.0, 0.0, 0.0, 0.0}, ci[4] = {0.0, 0.0, 0.0, 0.0}, cs[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int s = 0; s < (k + 7) >> 3; ++s) {
+        double ar[4], ai[4], as[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            ar[q] = a[q].x;
+            ai[q] = a[q].y;
+            as[q] = a[q].x + a[q].y;
+        }
+        narrow_load(a, A, m, k, lda, row, tig, s + 1);  // zeros past k
+        const double2 b0 = Xs[s * 8], b1 = Xs[s * 8 + 4];
+        const double br[2] = {b0.x, b1.x}, bi[2] = {b0.y, b1.y}, bs[2] = {b0.x + b0.y, b1.x + b1.y};
+        dmma16(cr, ar, br);
+        dmma16(ci, ai, bi);
+        dmma16(cs, as, bs);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) out[q] = make_double2(cr[q] - ci[q], cs[q] - cr[q] - ci[q]);
+}
+
 // Products with few columns: the operator is read once and hardly reused, so what
 // counts is bytes of it in flight.  zgemm_kernel stages it through shared memory
 // in 16-wide slices beside 64 columns, mostly zeros then, with a block barrier a
@@ -360,18 +393,10 @@ __global__ void __launch_bounds__(256, 3) zgemm_narrow_kernel(const GemmProblem*
     const int ncol = min(8, p.ncol - t.col0);
     const int ksteps = (p.k + 7) >> 3, kp = ksteps * 8 + 4;
     const int row = t.row0 + warp * 16 + g;  // rows row and row + 8 of the operator
-    const bool r0 = row < p.m, r1 = row + 8 < p.m, work = t.row0 + warp * 16 < p.m;
+    const bool work = t.row0 + warp * 16 < p.m;
     const double2 zero = make_double2(0.0, 0.0);
     double2 a[4];
-    auto load = [&](int step) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int k = step * 8 + tig + 4 * (q >> 1);
-            const bool ok = k < p.k && ((q & 1) ? r1 : r0);
-            a[q] = ok ? __ldg(p.A + (size_t)k * p.lda + row + 8 * (q & 1)) : zero;
-        }
-    };
-    if (work) load(0);
+    if (work) narrow_load(a, p.A, p.m, p.k, p.lda, row, tig, 0);
     // the tile's columns, zeros past the last one and past k
     for (int c = warp; c < 8; c += blockDim.x >> 5) {
         const double2* x = c < ncol ? X + xoff[p.col0 + t.col0 + c] : nullptr;
@@ -379,23 +404,8 @@ __global__ void __launch_bounds__(256, 3) zgemm_narrow_kernel(const GemmProblem*
     }
     __syncthreads();
     if (!work) return;
-    double cr[4] = {0.0, 0.0, 0.0, 0.0}, ci[4] = {0.0, 0.0, 0.0, 0.0}, cs[4] = {0.0, 0.0, 0.0, 0.0};
-    const double2* Xs = nsm + g * kp + tig;
-    for (int s = 0; s < ksteps; ++s) {
-        double ar[4], ai[4], as[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            ar[q] = a[q].x;
-            ai[q] = a[q].y;
-            as[q] = a[q].x + a[q].y;
-        }
-        load(s + 1);  // zeros past k
-        const double2 b0 = Xs[s * 8], b1 = Xs[s * 8 + 4];
-        const double br[2] = {b0.x, b1.x}, bi[2] = {b0.y, b1.y}, bs[2] = {b0.x + b0.y, b1.x + b1.y};
-        dmma16(cr, ar, br);
-        dmma16(ci, ai, bi);
-        dmma16(cs, as, bs);
-    }
+    double2 out[4];
+    narrow_product(out, a, p.A, p.m, p.k, p.lda, row, tig, nsm + g * kp + tig);
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
         const int col = 2 * tig + e;
@@ -403,9 +413,9 @@ __global__ void __launch_bounds__(256, 3) zgemm_narrow_kernel(const GemmProblem*
         double2* y = Y + yoff[p.col0 + t.col0 + col];
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-            const int rr = row + 8 * i, q = 2 * i + e;
+            const int rr = row + 8 * i;
             if (rr >= p.m) continue;
-            const double2 v = make_double2(cr[q] - ci[q], cs[q] - cr[q] - ci[q]);
+            const double2 v = out[2 * i + e];
             if (mode == GEMM_SET) {
                 y[rr] = v;
             } else if (mode == GEMM_ADD) {
@@ -417,6 +427,41 @@ __global__ void __launch_bounds__(256, 3) zgemm_narrow_kernel(const GemmProblem*
             }
         }
     }
+}
+
+// Two products in a row on few columns, y = B (A x) with A r x m and B m x r, m and r at
+// most 64: a block does 8 columns, the four warps 16 rows each of both, the
+// intermediate column (FP64, as it was when it went through memory) in shared memory.
+// What counts here is the launch that this saves in a small instance's chain of
+// dependent launches, each a few microseconds of latency: K = 4, P = 4 sphere 58.5 ->
+// 55.2 us an eval, a K = 8 cluster (ten of these launches fewer) 497 -> 487 us.
+__global__ void __launch_bounds__(128) zgemm_pair_kernel(const GemmPair P) {
+    __shared__ double2 xs[8 * 68], ms[8 * 68];  // columns 64 + 4 apart: conflict-free fragment reads
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tig = lane & 3, row = warp * 16 + g;
+    const int c0 = blockIdx.x * 8, ncol = min(8, P.ncol - c0);
+    const double2 zero = make_double2(0.0, 0.0);
+    double2 a[4], out[4];
+    narrow_load(a, P.A, P.r, P.m, P.r, row, tig, 0);
+    for (int c = warp; c < 8; c += 4) {
+        const double2* x = c < ncol ? P.X + P.off[c0 + c] : nullptr;
+        for (int k = lane; k < 64; k += 32) xs[c * 68 + k] = x && k < P.m ? x[k] : zero;
+    }
+    __syncthreads();
+    narrow_product(out, a, P.A, P.r, P.m, P.r, row, tig, xs + g * 68 + tig);
+    narrow_load(a, P.B, P.m, P.r, P.m, row, tig, 0);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) ms[(2 * tig + (q & 1)) * 68 + row + 8 * (q >> 1)] = out[q];  // zeros past r
+    __syncthreads();
+    narrow_product(out, a, P.B, P.m, P.r, P.m, row, tig, ms + g * 68 + tig);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int col = 2 * tig + (q & 1), rr = row + 8 * (q >> 1);
+        if (col < ncol && rr < P.m) P.Y[P.off[c0 + col] + rr] = out[q];
+    }
+}
+
+void launch_gemm_pair(const GemmPair& P, cudaStream_t s) {
+    if (P.ncol > 0) zgemm_pair_kernel<<<(P.ncol + 7) / 8, 128, 0, s>>>(P);
 }
 
 void gemm_init() {

@@ -74,6 +74,17 @@ void launch_gemm(const GemmProblem* probs_dev, const GemmTile* tiles_dev, int nt
 // launch's longest k, narrow_smem(kmax) <= NARROW_SMEM.
 constexpr int NARROW_SMEM = 72 << 10;
 size_t narrow_smem(int k);
+// Y[off[c] ..] = B (A X[off[c] ..]) for ncol columns: A r x m, B m x r, column-major and dense, m, r <= GEMM_PAIR_MAX
+constexpr int GEMM_PAIR_MAX = 64;
+struct GemmPair {
+    const double2* A;
+    const double2* B;
+    int m, r, ncol;
+    const long long* off;
+    const double2* X;
+    double2* Y;
+};
+void launch_gemm_pair(const GemmPair& P, cudaStream_t s);
 void launch_gemm_narrow(const GemmProblem* probs_dev, const GemmTile* tiles_dev, int ntiles, const long long* xoff,
                         const long long* yoff, const double2* X, double2* Y, int mode, int kmax, int rows,
                         cudaStream_t s);

@@ -1417,6 +1417,27 @@ void Session::build() {
         std::vector<std::vector<long long> > xo(1, x), yo(1, y);
         add_gemm(ps, xo, yo, X, Y, mode, label);
     };
+    // y = B (A x) on the boxes at the given offsets: one launch where both operators fit
+    // zgemm_pair_kernel and its 8-column blocks leave SMs free as zgemm_narrow_kernel's
+    // would (K = 4, P = 4: two launches of 10.8 us event to event, one of 14.7; K = 16: 26.4
+    // and 17.4 us), else two, whose wider tiles read the operators less often
+    auto twice = [&](const double2* A, const double2* B, int r, const std::vector<long long>& at, const double2* X, double2* Y,
+                     const char* label) {
+        if (mixed || nE > GEMM_PAIR_MAX || r > GEMM_PAIR_MAX || at.empty() || (at.size() + 63) / 64 >= 148) {
+            single(GemmProblem{opm(A, (size_t)r * nE), r, nE, r, 0, 0}, at, at, X, lf_mid, GEMM_SET, label);
+            single(GemmProblem{opm(B, (size_t)r * nE), nE, r, nE, 0, 0}, at, at, lf_mid, Y, GEMM_SET, label);
+            return;
+        }
+        Step st{};
+        st.kind = 11;
+        st.label = label;
+        st.flops = 16.0 * r * nE * (double)at.size();
+        st.bytes = 16.0 * (2.0 * r * nE + 2.0 * nE * (double)at.size());
+        st.gp = GemmPair{A, B, nE, r, (int)at.size(), upload(at), X, Y};
+        stats_.flops_gemm += st.flops;
+        stats_.gemm_launches++;
+        push_step(st);
+    };
     for (auto it = lflevels.rbegin(); it != lflevels.rend(); ++it) {
         const LfLevelOps& L = lfops[it->first];
         const auto& ids = it->second;
@@ -1456,15 +1477,9 @@ void Session::build() {
             add_gemm(probs, x, y, lf_upeq, lf_upchk, GEMM_ATOMIC, "lf_m2m");  // siblings add into one parent
         }
         // upeqnden = v * (1/sigma .* (U^H * upchk))   (src/wave3d_eval.cpp:466-478)
-        std::vector<long long> a, b2;
-        for (int l : ids) {
-            a.push_back((long long)l * nE);
-            b2.push_back((long long)l * nE);
-        }
-        single(GemmProblem{opm(L.up_s, (size_t)L.r * nE), L.r, nE, L.r, 0, 0}, a, b2, lf_upchk, lf_mid, GEMM_SET,
-               "lf_uc2ue");
-        single(GemmProblem{opm(L.v, (size_t)L.r * nE), nE, L.r, nE, 0, 0}, a, b2, lf_mid, lf_upeq, GEMM_SET,
-               "lf_uc2ue");
+        std::vector<long long> a;
+        for (int l : ids) a.push_back((long long)l * nE);
+        twice(L.up_s, L.v, L.r, a, lf_upchk, lf_upeq, "lf_uc2ue");
     }
 
     phase("steps_lf_up");
@@ -1812,10 +1827,7 @@ void Session::build() {
         // dneqnden = up^T (1/sigma .* (v^T dnchk))   (src/wave3d_eval.cpp:536-547, src/mlib3d.cpp:147-152)
         std::vector<long long> a;
         for (int l : ids) a.push_back((long long)l * nE);
-        single(GemmProblem{opm(L.vT_s, (size_t)L.r * nE), L.r, nE, L.r, 0, 0}, a, a, lf_dnchk, lf_mid, GEMM_SET,
-               "lf_dc2de");
-        single(GemmProblem{opm(L.upT, (size_t)L.r * nE), nE, L.r, nE, 0, 0}, a, a, lf_mid, lf_dneq, GEMM_SET,
-               "lf_dc2de");
+        twice(L.vT_s, L.upT, L.r, a, lf_dnchk, lf_dneq, "lf_dc2de");
         // L2T at leaves (src/wave3d_eval.cpp:550-560)
         {
             std::vector<PtItem> items;
@@ -1902,6 +1914,7 @@ static const char* kernel_name(int kind, int tpi, bool narrow) {
         case 8: return "i8_gemm_kernel";
         case 9: return "h16_slice_kernel";
         case 10: return "h16_gemm_kernel";
+        case 11: return "zgemm_pair_kernel";
         default: return "umma_cgemm_kernel";
     }
 }
@@ -1947,6 +1960,7 @@ void Session::launch_step(const Step& st, cudaStream_t s, double2* spec) {
             break;
         case 7: launch_i8_slice(st.dg.vecs, st.dg.n, st.dg.X, st.dg.X8, st.dg.cx, s); break;
         case 8: launch_i8_gemm(st.i8, d_err_, s); break;
+        case 11: launch_gemm_pair(st.gp, s); break;
         case 9:
             launch_h16_slice(static_cast<const HSliceSub*>(st.msubs), st.mpre, 1, st.mtotal, nullptr, s, st.hs);
             break;

@@ -142,11 +142,12 @@ private:
     struct Step {
         int kind;  // 0 gemm, 1 pt, 2 vfwd, 3 V-list sums, 5 tcgen05 gemm, 6 V-list inverse,
                    // 7 digits of vectors, 8 int8 tcgen05 gemm, 9 FP16 planes of vectors,
-                   // 10 FP16 tcgen05 gemm
+                   // 10 FP16 tcgen05 gemm, 11 two products in a row
         const char* label;  // pass name for profiling
         double flops;       // algorithmic flops of the launch
         double bytes;       // algorithmic DRAM bytes of the launch
         GemmLaunch g;
+        GemmPair gp;
         PtLaunch pt;
         VLaunch v;
         I8Sub i8;

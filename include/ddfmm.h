@@ -167,8 +167,9 @@ int ddfmm_session_test_gemm_stall(ddfmm_session* s, double wait_s);
  * current device through a translation kernel -- path 0: the FP64 tensor path,
  * 1: the int8 tensor path (exact integer products of digit planes), 2: the FP64
  * tensor path for few columns (PLAIN_FP64 form); 3: the FP16 tensor path (two
- * planes per number), 4: split TF32 (MIXED form, on FP32 copies).  Columns are
- * gathered and scattered as an eval's are. */
+ * planes per number), 4: split TF32 (MIXED form, on FP32 copies); 5: the kernel
+ * of two products in a row, the identity and A (m = k <= 64; Y = A X).  Columns
+ * are gathered and scattered as an eval's are. */
 int ddfmm_test_gemm(const double* A, int m, int k, const double* X, int ncol, int path, double* Y);
 
 /* Host-only (no GPU): build the octree and interaction lists of
