@@ -76,7 +76,6 @@ Batch::Batch(const std::vector<Session*>& sessions) : sessions_(sessions) {
     BCK(cudaGetDevice(&prev));
     BCK(cudaSetDevice(device_));
     BCK(cudaMalloc(&d_err_, sizeof(int)));
-    BCK(cudaMemset(d_err_, 0, sizeof(int)));
     allocs_.push_back(d_err_);
 
     // eval prologue: zero the accumulators, densities into leaf order
@@ -231,7 +230,8 @@ Batch::~Batch() {
 float2* Batch::den(int i) const { return reinterpret_cast<float2*>(sessions_.at(i)->d_den_io_); }
 float2* Batch::val(int i) const { return reinterpret_cast<float2*>(sessions_.at(i)->d_val_io_); }
 
-void Batch::run(const int* active, cudaStream_t s) {
+void Batch::run(const int* active, cudaStream_t s, unsigned long long stall_ns) {
+    BCK(cudaMemsetAsync(d_err_, 0, sizeof(int), s));  // a failure is reported by its own eval only
     for (const Launch& L : launches_) {
         switch (L.kind) {
             case ZERO:
@@ -241,13 +241,14 @@ void Batch::run(const int* active, cudaStream_t s) {
             case GATHER:
             case SCATTER:
                 launch_move32(static_cast<const MoveSub*>(L.subs), static_cast<const int*>(L.prefix), L.nsub,
-                              (int)L.total, active, L.kind == SCATTER, s);
+                              (int)L.total, active, L.kind == SCATTER, d_err_, s);
                 break;
             case GEMM:
                 launch_umma_cgemm(static_cast<const UmmaSub*>(L.subs), static_cast<const int*>(L.prefix), L.nsub,
                                   (int)L.total, active, d_err_, s,
-                                  L.nsub == 1 ? reinterpret_cast<const UmmaSub*>(L.one) : nullptr, 0, 0,
+                                  L.nsub == 1 ? reinterpret_cast<const UmmaSub*>(L.one) : nullptr, stall_ns, stall_ns > 0,
                                   static_cast<const int*>(L.order));
+                stall_ns = 0;
                 break;
             case SPLIT16:
                 launch_h16_slice(static_cast<const HSliceSub*>(L.subs), static_cast<const int*>(L.prefix), L.nsub,
@@ -280,6 +281,13 @@ void Batch::run(const int* active, cudaStream_t s) {
 }
 
 void Batch::run_graph(const int* active, cudaStream_t s) {
+    for (Session* S : sessions_)
+        if (S->stall_wait_ns_) {  // armed failure-path hook: this eval's launches themselves
+            const unsigned long long ns = S->stall_wait_ns_;
+            S->stall_wait_ns_ = 0;
+            run(active, s, ns);
+            return;
+        }
     for (const Graph& g : graphs_)
         if (g.active == active) {
             BCK(cudaGraphLaunch(g.exec, s));
@@ -314,11 +322,7 @@ void Batch::check_error(cudaStream_t s) {
     int h = 0;
     BCK(cudaMemcpyAsync(&h, d_err_, sizeof(int), cudaMemcpyDeviceToHost, s));
     BCK(cudaStreamSynchronize(s));
-    if (h) {
-        BCK(cudaMemsetAsync(d_err_, 0, sizeof(int), s));
-        BCK(cudaStreamSynchronize(s));
-        throw std::runtime_error("CUDA error: a tensor-core GEMM block timed out waiting on its pipeline");
-    }
+    if (h) throw std::runtime_error("CUDA error: a tensor-core GEMM block timed out waiting on its pipeline");
 }
 
 }  // namespace ddfmm

@@ -30,16 +30,16 @@ public:
     float2* den(int i) const;
     float2* val(int i) const;
     // One matvec of every instance i with active[i] != 0 (device array of
-    // size() ints; nullptr = all), enqueued on s.
-    void run(const int* active, cudaStream_t s);
+    // size() ints; nullptr = all), enqueued on s.  stall_ns > 0: the failure-path hook of
+    // Session::arm_gemm_stall on its first tensor-core GEMM launch.
+    void run(const int* active, cudaStream_t s, unsigned long long stall_ns = 0);
     // The same through a CUDA graph, captured on first use for each `active`
-    // array (a few are kept: one per mask array of the caller).  Graphs of
-    // different mask arrays may run at once on different streams when their
-    // active instances are disjoint.
+    // array (a few are kept: one per mask array of the caller).  Runs of one
+    // batch follow one another: they share the word that reports a failed GEMM.
     void run_graph(const int* active, cudaStream_t s);
     int launches() const { return (int)launches_.size(); }
-    // Throws if a tensor-core GEMM block gave up waiting (the flag is reset);
-    // synchronises s.
+    // Throws if a tensor-core GEMM block of the last run gave up waiting (its values are
+    // then all NaN); synchronises s.
     void check_error(cudaStream_t s);
 
 private:
@@ -64,7 +64,7 @@ private:
     std::vector<Launch> launches_;
     std::vector<void*> allocs_;
     int device_ = 0;
-    int* d_err_ = nullptr;
+    int* d_err_ = nullptr;  // set by a GEMM block that gave up; zeroed at a run's start
     struct Graph {
         const int* active;
         cudaGraph_t graph;

@@ -956,16 +956,18 @@ __global__ void gather_kernel(const double2* __restrict__ den, const int* __rest
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = den[perm[i]];
 }
+// The values are NaN where a GEMM of this eval gave up (*err, kernels.cuh)
 __global__ void scatter_kernel(const double2* __restrict__ in, const int* __restrict__ perm,
-                               double2* __restrict__ val, int n) {
+                               double2* __restrict__ val, int n, const int* err) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) val[perm[i]] = in[i];
+    const double nan = __longlong_as_double(0x7ff8000000000000ll);
+    if (i < n) val[perm[i]] = *err ? make_double2(nan, nan) : in[i];
 }
 void launch_gather_den(const double2* den, const int* perm, double2* out, int n, cudaStream_t s) {
     if (n > 0) gather_kernel<<<(n + 255) / 256, 256, 0, s>>>(den, perm, out, n);
 }
-void launch_scatter_val(const double2* in, const int* perm, double2* val, int n, cudaStream_t s) {
-    if (n > 0) scatter_kernel<<<(n + 255) / 256, 256, 0, s>>>(in, perm, val, n);
+void launch_scatter_val(const double2* in, const int* perm, double2* val, int n, const int* err, cudaStream_t s) {
+    if (n > 0) scatter_kernel<<<(n + 255) / 256, 256, 0, s>>>(in, perm, val, n, err);
 }
 
 // Direct FP64 sum at check targets (the reference's Wave3d::check,

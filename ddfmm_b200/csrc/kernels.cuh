@@ -219,11 +219,11 @@ void launch_vlist_group32(const VaSub* subs, const int* prefix, int nsub, int ng
 void launch_vlist_inverse32(const ViSub* subs, const int* prefix, int nsub, int ntrg, int G, const int* active,
                             cudaStream_t s, const ViSub* one);
 void launch_move32(const MoveSub* subs, const int* prefix, int nsub, int n, const int* active, int scatter,
-                   cudaStream_t s);
+                   const int* err, cudaStream_t s);
 void launch_zero(const ZeroSub* subs, const long long* prefix, int nsub, long long n8, const int* active,
                  cudaStream_t s);
 void launch_gather32(const void* den, const int* perm, void* out, int n, int c64, cudaStream_t s);
-void launch_scatter32(const void* in, const int* perm, void* val, int n, int c64, cudaStream_t s);
+void launch_scatter32(const void* in, const int* perm, void* val, int n, int c64, const int* err, cudaStream_t s);
 void launch_to_c64(const double2* a, float2* b, long long n, cudaStream_t s);
 
 // mixed-form low-frequency GEMM on tcgen05 (kernels_umma.cu): 128 gathered columns x up to
@@ -368,9 +368,12 @@ void launch_h16_slice(const HSliceSub* subs, const int* prefix, int nsub, int n,
 void launch_h16_gemm(const HSub* subs, const int* prefix, int nsub, int ntiles, const int* active, int* err,
                      cudaStream_t s, const HSub& one, const int* order = nullptr);
 
-// gather/scatter helpers
+// gather/scatter helpers.  err: the int that the pipelined GEMM launches of an eval set
+// when a block gave up on its pipeline; zero at the eval's start.  Outputs are then
+// incomplete, and an enqueued eval has no status to return, so the scatter that ends it
+// writes NaN for every value.
 void launch_gather_den(const double2* den, const int* perm, double2* out, int n, cudaStream_t s);
-void launch_scatter_val(const double2* in, const int* perm, double2* val, int n, cudaStream_t s);
+void launch_scatter_val(const double2* in, const int* perm, double2* val, int n, const int* err, cudaStream_t s);
 void launch_direct(const double* pos, const double2* den, int n, const int* chk, int nchk,
                    double2* out, int kernel, cudaStream_t s);
 

@@ -794,9 +794,14 @@ void launch_vlist_inverse32(const ViSub* subs, const int* prefix, int nsub, int 
 }
 
 // Batch I/O: complex64 densities in point-id order into leaf order (gather),
-// leaf-order values back to point-id order (scatter); one thread per point.
+// leaf-order values back to point-id order (scatter; NaN where *err, kernels.cuh);
+// one thread per point.
+__device__ __forceinline__ float2 value_or_nan(float2 v, const int* err) {
+    const float nan = __int_as_float(0x7fc00000);
+    return *err ? make_float2(nan, nan) : v;
+}
 __global__ void move32_kernel(const MoveSub* __restrict__ subs, const int* __restrict__ prefix, int nsub, int n,
-                              const int* __restrict__ active, int scatter) {
+                              const int* __restrict__ active, int scatter, const int* err) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int j = find_sub(prefix, nsub, i);
@@ -806,13 +811,13 @@ __global__ void move32_kernel(const MoveSub* __restrict__ subs, const int* __res
     const float2* in = static_cast<const float2*>(S.in);
     float2* out = static_cast<float2*>(S.out);
     if (scatter)
-        out[S.perm[l]] = in[l];
+        out[S.perm[l]] = value_or_nan(in[l], err);
     else
         out[l] = in[S.perm[l]];
 }
 void launch_move32(const MoveSub* subs, const int* prefix, int nsub, int n, const int* active, int scatter,
-                   cudaStream_t s) {
-    if (n > 0) move32_kernel<<<(n + 255) / 256, 256, 0, s>>>(subs, prefix, nsub, n, active, scatter);
+                   const int* err, cudaStream_t s) {
+    if (n > 0) move32_kernel<<<(n + 255) / 256, 256, 0, s>>>(subs, prefix, nsub, n, active, scatter, err);
 }
 
 // Zeroing of several instances' arrays, 8-byte words.
@@ -849,17 +854,17 @@ __global__ void gather32c_kernel(const float2* __restrict__ den, const int* __re
     if (i < n) out[i] = den[perm[i]];
 }
 __global__ void scatter32_kernel(const float2* __restrict__ in, const int* __restrict__ perm,
-                                 double2* __restrict__ val, int n) {
+                                 double2* __restrict__ val, int n, const int* err) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
-        float2 v = in[i];
+        float2 v = value_or_nan(in[i], err);
         val[perm[i]] = make_double2(v.x, v.y);
     }
 }
 __global__ void scatter32c_kernel(const float2* __restrict__ in, const int* __restrict__ perm,
-                                  float2* __restrict__ val, int n) {
+                                  float2* __restrict__ val, int n, const int* err) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) val[perm[i]] = in[i];
+    if (i < n) val[perm[i]] = value_or_nan(in[i], err);
 }
 // den / val are complex128 (c64 = 0) or complex64 (c64 = 1) arrays in point-id order
 void launch_gather32(const void* den, const int* perm, void* out, int n, int c64, cudaStream_t s) {
@@ -871,14 +876,14 @@ void launch_gather32(const void* den, const int* perm, void* out, int n, int c64
         gather32_kernel<<<(n + 255) / 256, 256, 0, s>>>(static_cast<const double2*>(den), perm,
                                                         static_cast<float2*>(out), n);
 }
-void launch_scatter32(const void* in, const int* perm, void* val, int n, int c64, cudaStream_t s) {
+void launch_scatter32(const void* in, const int* perm, void* val, int n, int c64, const int* err, cudaStream_t s) {
     if (n <= 0) return;
     if (c64)
         scatter32c_kernel<<<(n + 255) / 256, 256, 0, s>>>(static_cast<const float2*>(in), perm,
-                                                          static_cast<float2*>(val), n);
+                                                          static_cast<float2*>(val), n, err);
     else
         scatter32_kernel<<<(n + 255) / 256, 256, 0, s>>>(static_cast<const float2*>(in), perm,
-                                                         static_cast<double2*>(val), n);
+                                                         static_cast<double2*>(val), n, err);
 }
 
 __global__ void to_c64_kernel(const double2* __restrict__ a, float2* __restrict__ b, long long n) {

@@ -473,10 +473,6 @@ void Session::add_i8(const std::vector<GemmProblem>& P, const long long* xs, con
         ra += q.m;
     }
     const std::unique_ptr<int[]> xg = granules(xs, ncols, dg.base, dg.unit, dg.gran);
-    if (!d_err_) {
-        d_err_ = dalloc<int>(1);
-        CK(cudaMemsetAsync(d_err_, 0, sizeof(int), stream_));
-    }
     const I8PackJob* dj = upload(jobs);
     flush_uploads();
     launch_i8_pack(dj, (int)jobs.size(), max_tiles, stream_);
@@ -551,6 +547,7 @@ void Session::push_step(Step st) {
         if (base == order[i]) rank = (long long)i;
     const long long occ = block_counts_[base]++;
     st.lane = lane_;
+    bounded_waits_ |= st.kind == 5 || st.kind == 8 || st.kind == 10;
     st.key = ((long long)cur_phase_ << 48) | (cur_wkey_ << 32) | (rank << 16) | occ;
     steps_.push_back(st);
 }
@@ -582,15 +579,11 @@ void Session::flush_packs() {
 }
 
 void Session::check_device_error() {
-    if (!d_err_) return;
+    if (!bounded_waits_) return;
     int h = 0;
     CK(cudaMemcpyAsync(&h, d_err_, sizeof(int), cudaMemcpyDeviceToHost, stream_));
     CK(cudaStreamSynchronize(stream_));
-    if (h) {
-        CK(cudaMemsetAsync(d_err_, 0, sizeof(int), stream_));
-        CK(cudaStreamSynchronize(stream_));
-        throw std::runtime_error("CUDA error: a tensor-core GEMM block timed out waiting on its pipeline");
-    }
+    if (h) throw std::runtime_error("CUDA error: a tensor-core GEMM block timed out waiting on its pipeline");
 }
 
 void Session::arm_gemm_stall(double wait_s) {
@@ -854,8 +847,6 @@ void Session::build() {
     if (umma()) {
         umma_init();
         h16_init();
-        d_err_ = dalloc<int>(1);
-        CK(cudaMemsetAsync(d_err_, 0, sizeof(int), stream_));
     }
 
     for (auto& kv : lflevels) {
@@ -1130,13 +1121,15 @@ void Session::build() {
     phase("hf_nodes");
     stats_.hf_up_nodes = (long long)up.v.size();
     stats_.hf_down_nodes = (long long)dn.v.size();
-    // every accumulator of an eval in one allocation, zeroed by one memset at its start
+    // every accumulator of an eval in one allocation, zeroed by one memset at its start,
+    // and with them the flag of GEMMs that gave up: an eval reports its own failure only
     const size_t acc_elems[5] = {(size_t)npts_, (size_t)nLF * nE, (size_t)nLF * nE, (size_t)upeq_total,
                                  (size_t)dnchk_total};
     size_t acc_off[6] = {0};
     for (int i = 0; i < 5; ++i) acc_off[i + 1] = acc_off[i] + ((acc_elems[i] + 31) & ~(size_t)31);
-    double2* acc = salloc(acc_off[5]);
-    zero_at_start_.push_back(Memset{acc, es * acc_off[5]});
+    double2* acc = salloc(acc_off[5] + 1);
+    zero_at_start_.push_back(Memset{acc, es * (acc_off[5] + 1)});
+    d_err_ = (int*)E(acc, acc_off[5]);
     d_val_sorted_ = acc;
     double2* lf_upchk = E(acc, acc_off[1]);
     double2* lf_dnchk = E(acc, acc_off[2]);
@@ -2181,9 +2174,9 @@ void Session::eval_device(const double2* den, double2* val, cudaStream_t s) {
         launch_gather_den(den, d_perm_, d_den_sorted_, npts_, s);
     run_steps(s);
     if (mixed())
-        launch_scatter32(d_val_sorted_, d_perm_, val, npts_, 0, s);
+        launch_scatter32(d_val_sorted_, d_perm_, val, npts_, 0, d_err_, s);
     else
-        launch_scatter_val(d_val_sorted_, d_perm_, val, npts_, s);
+        launch_scatter_val(d_val_sorted_, d_perm_, val, npts_, d_err_, s);
     CK(cudaGetLastError());
 }
 
@@ -2191,7 +2184,7 @@ void Session::eval_device_c64(const float2* den, float2* val, cudaStream_t s) {
     if (!mixed()) throw std::invalid_argument("complex64 evaluation needs a mixed-precision session");
     launch_gather32(den, d_perm_, d_den_sorted_, npts_, 1, s);
     run_steps(s);
-    launch_scatter32(d_val_sorted_, d_perm_, val, npts_, 1, s);
+    launch_scatter32(d_val_sorted_, d_perm_, val, npts_, 1, d_err_, s);
     CK(cudaGetLastError());
 }
 
@@ -2225,9 +2218,9 @@ void Session::eval_device_scratch(const double2* den, double2* val, cudaStream_t
         launch_gather_den(den, d_perm_, d_den_sorted_, npts_, s);
     run_steps_spec(s, spec);
     if (mixed())
-        launch_scatter32(d_val_sorted_, d_perm_, val, npts_, 0, s);
+        launch_scatter32(d_val_sorted_, d_perm_, val, npts_, 0, d_err_, s);
     else
-        launch_scatter_val(d_val_sorted_, d_perm_, val, npts_, s);
+        launch_scatter_val(d_val_sorted_, d_perm_, val, npts_, d_err_, s);
     CK(cudaGetLastError());
 }
 

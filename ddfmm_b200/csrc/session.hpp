@@ -57,13 +57,13 @@ public:
         return prm_.precision == PRECISION_MIXED || prm_.precision == PRECISION_MIXED_MMA_SYNC;
     }
     bool umma() const { return prm_.precision == PRECISION_MIXED; }
-    // Throws if a tensor-core GEMM gave up waiting on its pipeline since the last
-    // check (the flag is reset); synchronises the session's stream.
+    // Throws if a tensor-core GEMM of the last eval gave up waiting on its pipeline (an
+    // eval's values are then all NaN); synchronises the session's stream.
     void check_device_error();
     // Failure-path test hook (tcgen05 sessions): the next eval's first
     // tensor-core GEMM launch runs with its pipeline waits bounded by wait_s and
     // withholds the operator copies of its block 0, so that block's wait runs
-    // out and the session reports the timeout at its next synchronous call.
+    // out and the eval fails.
     void arm_gemm_stall(double wait_s);
     // Same matvec with the V-list spectra in caller-provided scratch of
     // `capacity` double2 (must hold spectra_elems()); nothing is allocated.
@@ -274,7 +274,8 @@ private:
     double2* d_den_io_ = nullptr;
     double2* d_val_io_ = nullptr;
     std::vector<Memset> zero_at_start_;
-    int* d_err_ = nullptr;  // set by a tensor-core GEMM that timed out
+    int* d_err_ = nullptr;  // set by a tensor-core GEMM that timed out; zeroed at an eval's start
+    bool bounded_waits_ = false;  // an eval launches GEMMs that may set it
     unsigned long long stall_wait_ns_ = 0;  // armed failure-path hook (0: none)
     std::map<std::pair<const void*, long long>, const float*> packed_;  // (operator, m k) -> packed copy
     std::vector<UmmaPackJob> pack_jobs_;

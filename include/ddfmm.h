@@ -94,7 +94,11 @@ int ddfmm_eval_device_c64(ddfmm_session* s, const void* den_dev, void* val_dev, 
 
 /* Same, with den / val already in device memory of the session's GPU
  * (n complex128 each); stream is a cudaStream_t or NULL for the session's
- * own stream.  Returns after enqueueing; the caller synchronises. */
+ * own stream.  Returns after enqueueing; the caller synchronises.  The
+ * tensor-core GEMMs bound every wait on their pipelines (1 s); should one run
+ * out, e.g. on a GPU that stood still that long, ddfmm_eval and
+ * ddfmm_eval_c64 return DDFMM_ECUDA, and an enqueued eval, which has no status
+ * left to return, makes every value NaN.  The session's next eval is unaffected. */
 int ddfmm_eval_device(ddfmm_session* s, const void* den_dev, void* val_dev, void* stream);
 
 /* No counterpart in the reference.  ddfmm_eval_device for callers that
@@ -157,9 +161,9 @@ int ddfmm_precompute_operators(int kernel, int accu, int wmax, int threads, cons
  * session: the next eval's first tensor-core GEMM launch bounds its pipeline
  * waits by wait_s (0 < wait_s <= 1) and its first block withholds the copies
  * that block waits on, so that wait runs out; the block then drains its work,
- * frees its tensor memory and flags the session, whose next synchronous call
- * (ddfmm_eval and the like) returns DDFMM_ECUDA.  Nothing faults and the
- * context stays usable.  DDFMM_EINVAL on other sessions. */
+ * frees its tensor memory and flags the eval, which fails as described at
+ * ddfmm_eval_device.  Nothing faults and the context stays usable.  A batch
+ * call takes the hook of a session in it.  DDFMM_EINVAL on other sessions. */
 int ddfmm_session_test_gemm_stall(ddfmm_session* s, double wait_s);
 
 /* Test entry point, no counterpart in the reference: Y += A X (A m x k, X k x
@@ -229,7 +233,9 @@ int ddfmm_batch_create(ddfmm_session* const* sessions, int n, ddfmm_batch** out)
  * when every val[i] is filled. */
 int ddfmm_batch_eval_c64(ddfmm_batch* b, const float* const* den, float* const* val);
 /* The same with device arrays, enqueued on `stream` (a cudaStream_t, or NULL
- * for the batch's own stream); returns after enqueueing. */
+ * for the batch's own stream); returns after enqueueing.  A GEMM that gave up
+ * (ddfmm_eval_device) makes every value of the call NaN; ddfmm_batch_eval_c64
+ * returns DDFMM_ECUDA. */
 int ddfmm_batch_eval_device_c64(ddfmm_batch* b, const void* const* den_dev, void* const* val_dev, void* stream);
 /* Launches per batch matvec (the merged sequence). */
 int ddfmm_batch_launches(ddfmm_batch* b, int* launches);
