@@ -1467,7 +1467,13 @@ void Session::build() {
                     y[ind].push_back((long long)l * nE);
                 }
             }
-            add_gemm(probs, x, y, lf_upeq, lf_upchk, GEMM_ATOMIC, "lf_m2m");  // siblings add into one parent
+            if (!up.v.empty() || !dn.v.empty()) {
+                add_gemm(probs, x, y, lf_upeq, lf_upchk, GEMM_ATOMIC, "lf_m2m");  // siblings add into one parent
+            } else {
+                // no high-frequency passes (K = 1, 2): nothing else of an eval adds in an order
+                // of its own, so without atomics here a matvec repeats bit for bit
+                for (int ind = 0; ind < 8; ++ind) single(probs[ind], x[ind], y[ind], lf_upeq, lf_upchk, GEMM_ADD, "lf_m2m");
+            }
         }
         // upeqnden = v * (1/sigma .* (U^H * upchk))   (src/wave3d_eval.cpp:466-478)
         std::vector<long long> a;
