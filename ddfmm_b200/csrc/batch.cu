@@ -230,9 +230,12 @@ Batch::~Batch() {
 float2* Batch::den(int i) const { return reinterpret_cast<float2*>(sessions_.at(i)->d_den_io_); }
 float2* Batch::val(int i) const { return reinterpret_cast<float2*>(sessions_.at(i)->d_val_io_); }
 
-void Batch::run(const int* active, cudaStream_t s, unsigned long long stall_ns) {
+void Batch::run(const int* active, cudaStream_t s, unsigned long long stall_ns, int stall_kind) {
     BCK(cudaMemsetAsync(d_err_, 0, sizeof(int), s));  // a failure is reported by its own eval only
     for (const Launch& L : launches_) {
+        unsigned long long ns = 0;
+        if (stall_ns && ((L.kind == GEMM && stall_kind == 5) || (L.kind == GEMM16 && stall_kind == 10)))
+            std::swap(ns, stall_ns);
         switch (L.kind) {
             case ZERO:
                 launch_zero(static_cast<const ZeroSub*>(L.subs), static_cast<const long long*>(L.prefix), L.nsub,
@@ -246,9 +249,8 @@ void Batch::run(const int* active, cudaStream_t s, unsigned long long stall_ns) 
             case GEMM:
                 launch_umma_cgemm(static_cast<const UmmaSub*>(L.subs), static_cast<const int*>(L.prefix), L.nsub,
                                   (int)L.total, active, d_err_, s,
-                                  L.nsub == 1 ? reinterpret_cast<const UmmaSub*>(L.one) : nullptr, stall_ns, stall_ns > 0,
+                                  L.nsub == 1 ? reinterpret_cast<const UmmaSub*>(L.one) : nullptr, ns, ns > 0,
                                   static_cast<const int*>(L.order));
-                stall_ns = 0;
                 break;
             case SPLIT16:
                 launch_h16_slice(static_cast<const HSliceSub*>(L.subs), static_cast<const int*>(L.prefix), L.nsub,
@@ -257,7 +259,7 @@ void Batch::run(const int* active, cudaStream_t s, unsigned long long stall_ns) 
             case GEMM16:
                 launch_h16_gemm(static_cast<const HSub*>(L.subs), static_cast<const int*>(L.prefix), L.nsub, (int)L.total,
                                 active, d_err_, s, *reinterpret_cast<const HSub*>(L.one),
-                                static_cast<const int*>(L.order));
+                                static_cast<const int*>(L.order), ns, ns > 0);
                 break;
             case PT:
                 launch_pt32(static_cast<const PtSub*>(L.subs), static_cast<const int*>(L.prefix), L.nsub, (int)L.total,
@@ -285,7 +287,7 @@ void Batch::run_graph(const int* active, cudaStream_t s) {
         if (S->stall_wait_ns_) {  // armed failure-path hook: this eval's launches themselves
             const unsigned long long ns = S->stall_wait_ns_;
             S->stall_wait_ns_ = 0;
-            run(active, s, ns);
+            run(active, s, ns, S->stall_kind_);
             return;
         }
     for (const Graph& g : graphs_)

@@ -31,8 +31,8 @@ public:
     float2* val(int i) const;
     // One matvec of every instance i with active[i] != 0 (device array of
     // size() ints; nullptr = all), enqueued on s.  stall_ns > 0: the failure-path hook of
-    // Session::arm_gemm_stall on its first tensor-core GEMM launch.
-    void run(const int* active, cudaStream_t s, unsigned long long stall_ns = 0);
+    // Session::arm_gemm_stall on its first launch of step kind stall_kind.
+    void run(const int* active, cudaStream_t s, unsigned long long stall_ns = 0, int stall_kind = 0);
     // The same through a CUDA graph, captured on first use for each `active`
     // array (a few are kept: one per mask array of the caller).  Runs of one
     // batch follow one another: they share the word that reports a failed GEMM.

@@ -300,7 +300,14 @@ int ddfmm_precompute_operators(int kernel, int accu, int wmax, int threads, cons
 
 int ddfmm_session_test_gemm_stall(ddfmm_session* s, double wait_s) {
     if (!s || !s->impl) return fail(DDFMM_EINVAL, "NULL session");
-    return guarded([&] { s->impl->arm_gemm_stall(wait_s); });
+    return guarded([&] { s->impl->arm_gemm_stall(wait_s, 5); });
+}
+
+int ddfmm_session_test_gemm_stall_in(ddfmm_session* s, double wait_s, int kernel) {
+    if (!s || !s->impl) return fail(DDFMM_EINVAL, "NULL session");
+    if (kernel < 0 || kernel > 2) return fail(DDFMM_EINVAL, "kernel must be 0, 1 or 2");
+    static const int kinds[3] = {5, 10, 8};
+    return guarded([&] { s->impl->arm_gemm_stall(wait_s, kinds[kernel]); });
 }
 
 int ddfmm_test_gemm(const double* A, int m, int k, const double* X, int ncol, int path, double* Y) {

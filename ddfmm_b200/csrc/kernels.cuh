@@ -315,8 +315,8 @@ size_t i8_packed_bytes(int m, int k);
 // the tiles of one problem: m x k operator packed at B with row scales ra, columns col0 .. col0 + ncol
 void i8_tiles(const char* B, const double* ra, int m, int k, int col0, int ncol, std::vector<I8Tile>& out);
 void launch_i8_pack(const I8PackJob* jobs_dev, int njobs, int max_tiles, cudaStream_t s);
-// *err is set when a block gave up waiting on its pipeline
-void launch_i8_gemm(const I8Sub& sub, int* err, cudaStream_t s);
+// *err is set when a block gave up waiting on its pipeline; wait_ns, withhold as in launch_umma_cgemm
+void launch_i8_gemm(const I8Sub& sub, int* err, cudaStream_t s, unsigned long long wait_ns = 0, int withhold = 0);
 // gemm_test.cu: Y += A X through one of the GEMM kernels (paths as in ddfmm.h)
 void test_gemm(const double2* A, int m, int k, const double2* X, int ncol, int path, double2* Y);
 
@@ -362,11 +362,12 @@ size_t h16_packed_floats(int m, int k);
 const float* h16_scales(const float* packed, int m, int k);  // the row scales of a packed operator
 void h16_tiles(const float* packed, int m, int k, int col0, int ncol, std::vector<H16Tile>& out);
 void launch_h16_pack(const H16PackJob* jobs_dev, int njobs, int max_tiles, cudaStream_t s);
-// nsub == 1: `one` is that sub-launch (sent as a kernel parameter); order as in launch_umma_cgemm
+// nsub == 1: `one` is that sub-launch (sent as a kernel parameter); order, wait_ns, withhold as in launch_umma_cgemm
 void launch_h16_slice(const HSliceSub* subs, const int* prefix, int nsub, int n, const int* active, cudaStream_t s,
                       const HSliceSub& one);
 void launch_h16_gemm(const HSub* subs, const int* prefix, int nsub, int ntiles, const int* active, int* err,
-                     cudaStream_t s, const HSub& one, const int* order = nullptr);
+                     cudaStream_t s, const HSub& one, const int* order = nullptr, unsigned long long wait_ns = 0,
+                     int withhold = 0);
 
 // gather/scatter helpers.  err: the int that the pipelined GEMM launches of an eval set
 // when a block gave up on its pipeline; zero at the eval's start.  Outputs are then

@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(HTHREADS, 1) h16_gemm_kernel(const HSub one, c
                                                                const int* __restrict__ gprefix, int nsub, int ntiles,
                                                                const int* __restrict__ order,
                                                                const int* __restrict__ active, int* err,
-                                                               unsigned long long wait_ns) {
+                                                               unsigned long long wait_ns, int withhold) {
     extern __shared__ __align__(1024) unsigned char hsm_raw[];
     __shared__ HSub ssubs[MULTI ? H_SUBS_SMEM : 1];
     __shared__ int sprefix[MULTI ? H_SUBS_SMEM + 1 : 1];
@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(HTHREADS, 1) h16_gemm_kernel(const HSub one, c
                     break;
                 }
                 parity ^= 1;
-                if (lane == 0) {
+                if (lane == 0 && !(withhold && blockIdx.x == 0)) {  // withheld: full[warp] never completes
                     mbar_expect_tx(&full[warp], bytes);
                     bulk_g2s(sm + warp * H_SLOT_BYTES + H_X_BYTES, reinterpret_cast<const char*>(T.B) + (size_t)kb * bytes,
                              bytes, &full[warp]);
@@ -561,14 +561,17 @@ void h16_init() {
 }
 
 void launch_h16_gemm(const HSub* subs, const int* prefix, int nsub, int ntiles, const int* active, int* err,
-                     cudaStream_t s, const HSub& one, const int* order) {
+                     cudaStream_t s, const HSub& one, const int* order, unsigned long long wait_ns, int withhold) {
     if (ntiles == 0) return;
+    if (wait_ns == 0) wait_ns = U_WAIT_NS;
     const int sms = g_h16_sms > 0 ? g_h16_sms : 148;
     const int grid = ntiles < sms ? ntiles : sms;
     if (nsub == 1)
-        h16_gemm_kernel<false><<<grid, HTHREADS, H_SMEM, s>>>(one, subs, prefix, nsub, ntiles, nullptr, active, err, U_WAIT_NS);
+        h16_gemm_kernel<false><<<grid, HTHREADS, H_SMEM, s>>>(one, subs, prefix, nsub, ntiles, nullptr, active, err, wait_ns,
+                                                                 withhold);
     else
-        h16_gemm_kernel<true><<<grid, HTHREADS, H_SMEM, s>>>(HSub{}, subs, prefix, nsub, ntiles, order, active, err, U_WAIT_NS);
+        h16_gemm_kernel<true><<<grid, HTHREADS, H_SMEM, s>>>(HSub{}, subs, prefix, nsub, ntiles, order, active, err, wait_ns,
+                                                                withhold);
 }
 
 }  // namespace ddfmm

@@ -420,7 +420,7 @@ __device__ __forceinline__ void tmem_ld4(uint32_t addr, int n, int (&d)[4][8]) {
 }
 }  // namespace
 
-__global__ void __launch_bounds__(ITHREADS, 1) i8_gemm_kernel(const I8Sub S, int* err, unsigned long long wait_ns) {
+__global__ void __launch_bounds__(ITHREADS, 1) i8_gemm_kernel(const I8Sub S, int* err, unsigned long long wait_ns, int withhold) {
     extern __shared__ __align__(1024) unsigned char ism_raw[];
     __shared__ __align__(8) uint64_t full[ISTAGES], empty[ISTAGES], acc_full, acc_empty, drained;
     __shared__ uint32_t tmem_base;
@@ -479,7 +479,7 @@ __global__ void __launch_bounds__(ITHREADS, 1) i8_gemm_kernel(const I8Sub S, int
                         ok = false;
                         break;
                     }
-                    if (lane == 0) {
+                    if (lane == 0 && !(withhold && blockIdx.x == 0)) {  // withheld: full[s] never completes
                         const uint32_t bytes = (uint32_t)(ph == 0 ? IS : 4) * T.n * 32;
                         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%1], %0;\n" ::"r"(bytes),
                                      "r"(su32(&full[s]))
@@ -665,10 +665,10 @@ void i8_init() {
     cudaDeviceGetAttribute(&g_i8_sms, cudaDevAttrMultiProcessorCount, dev);
 }
 
-void launch_i8_gemm(const I8Sub& S, int* err, cudaStream_t s) {
+void launch_i8_gemm(const I8Sub& S, int* err, cudaStream_t s, unsigned long long wait_ns, int withhold) {
     if (S.ntiles == 0) return;
     const int sms = g_i8_sms > 0 ? g_i8_sms : 148;
-    i8_gemm_kernel<<<S.ntiles < sms ? S.ntiles : sms, ITHREADS, I_SMEM, s>>>(S, err, I_WAIT_NS);
+    i8_gemm_kernel<<<S.ntiles < sms ? S.ntiles : sms, ITHREADS, I_SMEM, s>>>(S, err, wait_ns ? wait_ns : I_WAIT_NS, withhold);
 }
 
 }  // namespace ddfmm

@@ -586,10 +586,12 @@ void Session::check_device_error() {
     if (h) throw std::runtime_error("CUDA error: a tensor-core GEMM block timed out waiting on its pipeline");
 }
 
-void Session::arm_gemm_stall(double wait_s) {
-    if (!umma()) throw std::invalid_argument("the GEMM stall hook needs a DDFMM_MIXED (tcgen05) session");
+void Session::arm_gemm_stall(double wait_s, int kind) {
+    if (std::none_of(steps_.begin(), steps_.end(), [&](const Step& st) { return st.kind == kind; }))
+        throw std::invalid_argument("the session's evals do not launch this tensor-core GEMM");
     if (!(wait_s > 0 && wait_s <= 1.0)) throw std::invalid_argument("stall wait must be in (0, 1] seconds");
     stall_wait_ns_ = (unsigned long long)(wait_s * 1e9);
+    stall_kind_ = kind;
 }
 
 const char* Session::width_label(const char* pass, double W) {
@@ -1920,6 +1922,8 @@ static const char* kernel_name(int kind, int tpi, bool narrow) {
 
 void Session::launch_step(const Step& st, cudaStream_t s, double2* spec) {
     const bool m = mixed();
+    unsigned long long stall_ns = 0;  // failure-path hook: one launch only
+    if (stall_wait_ns_ && st.kind == stall_kind_) std::swap(stall_ns, stall_wait_ns_);
     switch (st.kind) {
         case 0:
             if (m)
@@ -1958,21 +1962,19 @@ void Session::launch_step(const Step& st, cudaStream_t s, double2* spec) {
                 launch_vlist_inverse(st.v.L, st.v.trg, st.v.ntrg, st.v.tsp, st.v.dnchk, s);
             break;
         case 7: launch_i8_slice(st.dg.vecs, st.dg.n, st.dg.X, st.dg.X8, st.dg.cx, s); break;
-        case 8: launch_i8_gemm(st.i8, d_err_, s); break;
+        case 8: launch_i8_gemm(st.i8, d_err_, s, stall_ns, stall_ns > 0); break;
         case 11: launch_gemm_pair(st.gp, s); break;
         case 9:
             launch_h16_slice(static_cast<const HSliceSub*>(st.msubs), st.mpre, 1, st.mtotal, nullptr, s, st.hs);
             break;
         case 10:
-            launch_h16_gemm(static_cast<const HSub*>(st.msubs), st.mpre, 1, st.mtotal, nullptr, d_err_, s, st.hh);
+            launch_h16_gemm(static_cast<const HSub*>(st.msubs), st.mpre, 1, st.mtotal, nullptr, d_err_, s, st.hh,
+                            nullptr, stall_ns, stall_ns > 0);
             break;
-        case 5: {
-            const unsigned long long wait_ns = stall_wait_ns_;
-            stall_wait_ns_ = 0;  // one launch only
+        case 5:
             launch_umma_cgemm(static_cast<const UmmaSub*>(st.msubs), st.mpre, 1, st.mtotal, nullptr, d_err_, s, &st.hu,
-                              wait_ns, wait_ns ? 1 : 0);
+                              stall_ns, stall_ns > 0);
             break;
-        }
     }
 }
 

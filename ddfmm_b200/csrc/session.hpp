@@ -60,11 +60,10 @@ public:
     // Throws if a tensor-core GEMM of the last eval gave up waiting on its pipeline (an
     // eval's values are then all NaN); synchronises the session's stream.
     void check_device_error();
-    // Failure-path test hook (tcgen05 sessions): the next eval's first
-    // tensor-core GEMM launch runs with its pipeline waits bounded by wait_s and
-    // withholds the operator copies of its block 0, so that block's wait runs
-    // out and the eval fails.
-    void arm_gemm_stall(double wait_s);
+    // Failure-path test hook: the next eval's first launch of a tensor-core GEMM (kind of
+    // Step: 5, 8 or 10) runs with its pipeline waits bounded by wait_s and withholds the
+    // operator copies of its block 0, so that block's wait runs out and the eval fails.
+    void arm_gemm_stall(double wait_s, int kind);
     // Same matvec with the V-list spectra in caller-provided scratch of
     // `capacity` double2 (must hold spectra_elems()); nothing is allocated.
     void eval_device_scratch(const double2* den, double2* val, cudaStream_t s, double2* spec, size_t capacity);
@@ -277,6 +276,7 @@ private:
     int* d_err_ = nullptr;  // set by a tensor-core GEMM that timed out; zeroed at an eval's start
     bool bounded_waits_ = false;  // an eval launches GEMMs that may set it
     unsigned long long stall_wait_ns_ = 0;  // armed failure-path hook (0: none)
+    int stall_kind_ = 5;
     std::map<std::pair<const void*, long long>, const float*> packed_;  // (operator, m k) -> packed copy
     std::vector<UmmaPackJob> pack_jobs_;
     std::vector<H16PackJob> h16_jobs_;

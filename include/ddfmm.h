@@ -158,13 +158,17 @@ int ddfmm_precompute_operators(int kernel, int accu, int wmax, int threads, cons
                                int verbose);
 
 /* Failure-path test hook, no counterpart in the reference.  On a DDFMM_MIXED
- * session: the next eval's first tensor-core GEMM launch bounds its pipeline
+ * session: the next eval's first split-TF32 GEMM launch bounds its pipeline
  * waits by wait_s (0 < wait_s <= 1) and its first block withholds the copies
  * that block waits on, so that wait runs out; the block then drains its work,
  * frees its tensor memory and flags the eval, which fails as described at
  * ddfmm_eval_device.  Nothing faults and the context stays usable.  A batch
  * call takes the hook of a session in it.  DDFMM_EINVAL on other sessions. */
 int ddfmm_session_test_gemm_stall(ddfmm_session* s, double wait_s);
+/* The same for the first launch of one kernel -- 0: split TF32, 1: FP16 planes
+ * (DDFMM_MIXED sessions), 2: int8 digits (DDFMM_PLAIN_FP64 sessions large
+ * enough to use it).  DDFMM_EINVAL if the session's evals do not launch it. */
+int ddfmm_session_test_gemm_stall_in(ddfmm_session* s, double wait_s, int kernel);
 
 /* Test entry point, no counterpart in the reference: Y += A X (A m x k, X k x
  * ncol, Y m x ncol, column-major complex128 host arrays; m, k <= 400) on the
