@@ -21,6 +21,7 @@ EXPORTS = (
     "ddfmm_server_remove_session", "ddfmm_server_submit", "ddfmm_server_wait", "ddfmm_server_poll",
     "ddfmm_server_get_stats", "ddfmm_server_destroy", "ddfmm_operators_check", "ddfmm_session_test_gemm_stall",
     "ddfmm_precompute_operators", "ddfmm_test_gemm", "ddfmm_session_test_gemm_stall_in",
+    "ddfmm_session_test_create",
 )
 PLAIN_FP64, MIXED, MIXED_MMA_SYNC = 0, 1, 2
 
@@ -82,6 +83,8 @@ def load():
                                             C.c_int, C.c_int, C.c_char_p, C.c_char_p, C.c_int, C.c_int,
                                             C.POINTER(C.c_void_p)]
     lib.ddfmm_session_create_ex.restype = C.c_int
+    lib.ddfmm_session_test_create.argtypes = lib.ddfmm_session_create_ex.argtypes[:-1] + [C.c_int, C.POINTER(C.c_void_p)]
+    lib.ddfmm_session_test_create.restype = C.c_int
     fp = C.POINTER(C.c_float)
     lib.ddfmm_eval_c64.argtypes = [C.c_void_p, fp, fp]
     lib.ddfmm_eval_c64.restype = C.c_int

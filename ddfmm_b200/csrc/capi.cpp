@@ -143,12 +143,22 @@ extern "C" {
 int ddfmm_session_create_ex(const double* pos3n, int n, int kernel, int accu, int npq, double K, const double* ctr3,
                             int ptsmax, int maxlevel, int ncell, const char* ld_path, const char* hd_path, int device,
                             int precision, ddfmm_session** out) {
+    return ddfmm_session_test_create(pos3n, n, kernel, accu, npq, K, ctr3, ptsmax, maxlevel, ncell, ld_path, hd_path,
+                                     device, precision, ddfmm::INT8_BY_SIZE, out);
+}
+
+int ddfmm_session_test_create(const double* pos3n, int n, int kernel, int accu, int npq, double K, const double* ctr3,
+                              int ptsmax, int maxlevel, int ncell, const char* ld_path, const char* hd_path, int device,
+                              int precision, int int8_rule, ddfmm_session** out) {
     if (!out) return fail(DDFMM_EINVAL, "out is NULL");
     *out = nullptr;
     ddfmm::SessionParams p;
     int rc = make_params(pos3n, n, kernel, accu, npq, K, ctr3, ptsmax, maxlevel, ncell, ld_path, hd_path, device,
                          precision, &p);
     if (rc != DDFMM_OK) return rc;
+    if (int8_rule < ddfmm::INT8_BY_SIZE || int8_rule > ddfmm::INT8_ALTERNATE)
+        return fail(DDFMM_EINVAL, "int8_rule must be 0, 1 or 2");
+    p.int8_rule = int8_rule;
     ddfmm::Session* impl = nullptr;
     rc = guarded([&] { impl = new ddfmm::Session(pos3n, n, p, ld_path, hd_path); });
     if (rc != DDFMM_OK) return rc;

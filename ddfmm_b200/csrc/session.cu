@@ -1508,7 +1508,11 @@ void Session::build() {
     bool lf_i8 = false;
     if (!mixed || umma()) {
         auto choose = [&](const std::vector<std::array<int, 3> >& shapes) {
-            return umma() ? std::vector<char>(shapes.size(), 1) : i8_choose(shapes);
+            if (umma()) return std::vector<char>(shapes.size(), 1);
+            if (prm_.int8_rule == INT8_BY_SIZE) return i8_choose(shapes);
+            std::vector<char> on(prm_.int8_rule == INT8_ALTERNATE ? shapes.size() : 0);
+            for (size_t i = 0; i < on.size(); i += 2) on[i] = 1;
+            return on;
         };
         long long dn_most = 0;
         for (auto& kv : hflevels) {

@@ -18,12 +18,17 @@
 
 namespace ddfmm {
 
+enum { INT8_BY_SIZE = 0, INT8_NONE = 1, INT8_ALTERNATE = 2 };
+
 struct SessionParams {
     TreeParams tree;
     int accu = 1;    // -wave3d_ACCU: P = 4/6/8 (src/wave3d.cpp:145-158)
     int kernel = 0;  // KERNEL_HELM / KERNEL_EXPR
     int device = 0;
     int precision = 0;  // PRECISION_FP64 (plain) / PRECISION_MIXED / PRECISION_MIXED_MMA_SYNC
+    // plain form, which high-frequency products run on the int8 path: INT8_BY_SIZE, or for
+    // tests of the routes INT8_NONE / INT8_ALTERNATE (every second one of each launch)
+    int int8_rule = 0;
 };
 
 struct SessionStats {

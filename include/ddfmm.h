@@ -170,6 +170,14 @@ int ddfmm_session_test_gemm_stall(ddfmm_session* s, double wait_s);
  * enough to use it).  DDFMM_EINVAL if the session's evals do not launch it. */
 int ddfmm_session_test_gemm_stall_in(ddfmm_session* s, double wait_s, int kernel);
 
+/* ddfmm_session_create_ex for tests of the plain form's routes, no counterpart
+ * in the reference.  int8_rule: which high-frequency products run on the int8
+ * tensor path -- 0: by size, as ddfmm_session_create_ex; 1: none; 2: every
+ * second one of each launch, whatever its size.  Other forms ignore it. */
+int ddfmm_session_test_create(const double* pos3n, int n, int kernel, int accu, int npq, double K, const double* ctr3,
+                              int ptsmax, int maxlevel, int ncell, const char* ld_path, const char* hd_path, int device,
+                              int precision, int int8_rule, ddfmm_session** out);
+
 /* Test entry point, no counterpart in the reference: Y += A X (A m x k, X k x
  * ncol, Y m x ncol, column-major complex128 host arrays; m, k <= 400) on the
  * current device through a translation kernel -- path 0: the FP64 tensor path,
