@@ -797,7 +797,6 @@ void Session::build() {
     double2* lf_upeq = salloc((size_t)nLF * nE);
     double2* lf_mid = salloc((size_t)nLF * nE);
     double2* lf_dneq = salloc((size_t)nLF * nE);
-    double2* lf_spec = salloc((size_t)nLF * G3);
     spectra_elems_ = (size_t)nLF * G3;
     stats_.fft_spectra_bytes = (long long)nLF * G3 * 16;
 
@@ -1160,7 +1159,10 @@ void Session::build() {
         pool += (n + 15) & ~(size_t)15;
         return o;
     };
-    size_t scr = 0, keep = 0;
+    size_t scr = 0;
+    // place of a folded operator: kInt8 | offset in the pool of int8 products' operators, or an
+    // offset in the other pool, or kNone (no box has a child there)
+    constexpr size_t kInt8 = (size_t)1 << 62, kNone = ~(size_t)0;
     // cache keys of the shared operators: (kind, width, wedge, child or offset)
     auto opk = [](const char* kind, double W, const Idx3& d, int a, int b = 0, int c = 0) {
         char buf[128];
@@ -1191,13 +1193,12 @@ void Session::build() {
         ccanon = cp.canon;
         return upward ? cp.uep : cp.dcp;
     };
-    std::vector<char> m2m_seen(dirpts.size(), 0), l2l_seen(dirpts.size(), 0);  // by dense wedge id: already planned
+    std::vector<DirMats*> m2m_of(dirpts.size(), nullptr), l2l_of(dirpts.size(), nullptr);  // by dense wedge id
     for (auto& kv : hflevels) {
         double W = T.width(kv.first);
         auto ur = up.range[kv.first], dr = dn.range[kv.first];
         for (int i = ur.first; i < ur.second; ++i) {
-            if (m2m_seen[up.v[i].did]) continue;
-            m2m_seen[up.v[i].did] = 1;
+            if (m2m_of[up.v[i].did]) continue;
             auto key = std::make_pair(W, up.v[i].dir);
             const DirPts& dp = get_dir(W, up.v[i].dir);
             DirMats M{};
@@ -1211,13 +1212,12 @@ void Session::build() {
             for (int ind = 0; ind < 8 && !M.cached; ++ind) {
                 M.raw[ind] = take(scr, (size_t)M.rmid * M.mcols);
                 M.tmp[ind] = take(scr, (size_t)M.rmid * M.mcols);
-                M.fin[ind] = take(keep, (size_t)M.mrows * M.mcols);
+                M.fin[ind] = kNone;
             }
-            m2m_mats[key] = M;
+            m2m_of[up.v[i].did] = &(m2m_mats[key] = M);
         }
         for (int i = dr.first; i < dr.second; ++i) {
-            if (l2l_seen[dn.v[i].did]) continue;
-            l2l_seen[dn.v[i].did] = 1;
+            if (l2l_of[dn.v[i].did]) continue;
             auto key = std::make_pair(W, dn.v[i].dir);
             const DirPts& dp = get_dir(W, dn.v[i].dir);
             DirMats M{};
@@ -1231,9 +1231,9 @@ void Session::build() {
             for (int ind = 0; ind < 8 && !M.cached; ++ind) {
                 M.raw[ind] = take(scr, (size_t)M.mrows * M.rmid);
                 M.tmp[ind] = take(scr, (size_t)M.mrows * M.rmid);
-                M.fin[ind] = take(keep, (size_t)M.mrows * M.mcols);
+                M.fin[ind] = kNone;
             }
-            l2l_mats[key] = M;
+            l2l_of[dn.v[i].did] = &(l2l_mats[key] = M);
         }
     }
     phase("m2m_l2l_plan");
@@ -1278,7 +1278,6 @@ void Session::build() {
                     if (!pk) {
                         M.raw = take(scr, n);
                         M.tmp = take(scr, n);
-                        M.fin = take(keep, n);
                     }
                     m2l_mats.push_back(M);
                     m2l_id[C.keys[k]] = gid;
@@ -1304,6 +1303,88 @@ void Session::build() {
     }
     phase("m2l_plan");
     stats_.m2l_matrices = (long long)m2l_mats.size();
+    // children with points of every high-frequency box (-1: none)
+    std::vector<int> kids((size_t)nb * 8, -1);
+    for (auto& kv : hflevels)
+        for (int b : kv.second)
+            for (int ind = 0; ind < 8; ++ind) {
+                const int c = T.child(b, ind);
+                if (c >= 0 && T.boxes[c].has_pts()) kids[(size_t)b * 8 + ind] = c;
+            }
+    // the column lists of every level's M2M and L2L launches, built on all host cores (plan.cpp)
+    std::vector<std::pair<double, Idx3> > did_wedge(dirpts.size());
+    for (auto& kv : dirpts) did_wedge[kv.second.did] = kv.first;
+    std::vector<long long> lf_off(nb, -1);
+    for (int l = 0; l < nLF; ++l) lf_off[lfbox[l]] = (long long)l * nE;
+    HfColumns cols = hf_columns(T, up, dn, kids, lf_off, dirpts.size(), hfcanon.size(), false);
+    phase("hf_columns");
+    // ---------------------------------------------------------------- routes of the HF products
+    // plain form: the int8 path for problems large enough; tcgen05 form: FP16 planes for all
+    std::map<int, std::vector<char> > m2m_i8, m2l_i8, l2l_i8;  // level -> problems on the int8 path
+    std::set<int> up_i8, dn_i8;  // levels whose outgoing / incoming vectors are written as digits
+    bool lf_i8 = false;
+    if (!mixed || umma()) {
+        auto choose = [&](const std::vector<std::array<int, 3> >& shapes) {
+            if (umma()) return std::vector<char>(shapes.size(), 1);
+            if (prm_.int8_rule == INT8_BY_SIZE) return i8_choose(shapes);
+            std::vector<char> on(prm_.int8_rule == INT8_ALTERNATE ? shapes.size() : 0);
+            for (size_t i = 0; i < on.size(); i += 2) on[i] = 1;
+            return on;
+        };
+        for (auto& kv : hflevels) {
+            const int level = kv.first;
+            const double W = T.width(level);
+            auto shapes = [&](const ColLists& L, const std::vector<DirMats*>& of) {
+                std::vector<std::array<int, 3> > v;
+                if (umma()) v.resize(L.key.size());  // all of them
+                for (size_t i = v.size(); i < L.key.size(); ++i) {
+                    const DirMats& M = *of[L.key[i] / 8];
+                    v.push_back({{M.mrows, M.mcols, (int)L.x[i].size()}});
+                }
+                return v;
+            };
+            std::vector<std::array<int, 3> > far;
+            for (size_t i = 0; i < m2l_probs[level].size(); ++i) {
+                const int r1 = m2l_mats[m2l_probs[level][i]].r1;
+                far.push_back({{r1, r1, (int)m2l_x[level][i].size()}});
+            }
+            m2m_i8[level] = choose(shapes(cols.m2m.at(level), m2m_of));
+            m2l_i8[level] = choose(far);
+            l2l_i8[level] = choose(shapes(cols.l2l.at(level), l2l_of));
+            if (!m2m_i8[level].empty()) {
+                if (W == 1.0)
+                    lf_i8 = true;
+                else
+                    up_i8.insert(level + 1);
+            }
+            if (!m2l_i8[level].empty()) up_i8.insert(level);
+            if (!l2l_i8[level].empty()) dn_i8.insert(level);
+        }
+    }
+    // The folded operators.  i8_pack_kernel alone reads those of int8 products, so theirs is a
+    // pool that is released once they are packed: FP64 operators kept beside their digits,
+    // digits with memory of their own each way and spectra beside them took 26.6 GB for a
+    // sphere of K = 64 at P = 6, released and shared they take 19.9 (24.0 while it is set up)
+    size_t keep = 0, keep8 = 0;
+    auto lay_out = [&](size_t& fin, size_t n, const std::vector<char>& on, size_t i) {
+        fin = !mixed && !on.empty() && on[i] ? kInt8 | take(keep8, n) : take(keep, n);
+    };
+    for (auto& kv : hflevels) {
+        const int level = kv.first;
+        auto lay_out_all = [&](const ColLists& L, const std::vector<DirMats*>& of, const std::vector<char>& on) {
+            for (size_t i = 0; i < L.key.size(); ++i) {
+                DirMats& M = *of[L.key[i] / 8];
+                if (!M.cached) lay_out(M.fin[L.key[i] % 8], (size_t)M.mrows * M.mcols, on, i);
+            }
+        };
+        lay_out_all(cols.m2m.at(level), m2m_of, m2m_i8[level]);
+        for (size_t i = 0; i < m2l_probs[level].size(); ++i) {
+            M2LMat& M = m2l_mats[m2l_probs[level][i]];
+            if (!M.pk) lay_out(M.fin, (size_t)M.r1 * M.r1, m2l_i8[level], i);
+        }
+        lay_out_all(cols.l2l.at(level), l2l_of, l2l_i8[level]);
+    }
+    phase("routes");
     // right factors E1, E2^T and E3^T as gatherable columns in the scratch pool
     std::vector<size_t> scr_E1(hfcanon.size()), scr_E2t(hfcanon.size()), scr_E3t(hfcanon.size());
     for (size_t c = 0; c < hfcanon.size(); ++c) {
@@ -1312,6 +1393,7 @@ void Session::build() {
         scr_E3t[c] = take(scr, (size_t)hfcanon[c].r2 * hfcanon[c].r2);
     }
     double2* dkeep = dalloc<double2>(keep);
+    double2* dkeep8 = keep8 ? dalloc<double2>(keep8) : nullptr;
     double2* dscr = nullptr;
     if (scr) CK(cudaMalloc(&dscr, sizeof(double2) * scr));
     flush_uploads();
@@ -1360,41 +1442,47 @@ void Session::build() {
     //   L2L  tmp = de2dc E3^T;       mid = E1(child)^T tmp;     fin = mid E2^T
     //   M2L  tmp = M E1;                                        fin = E1^T tmp
     if (scr) {
-        GemmBatch right, left, last;
+        GemmBatch right, left, last, last8;
+        auto fold = [&](const double2* A, int m, int k, size_t bx, int n, size_t fin) {
+            (fin & kInt8 ? last8 : last).product(A, m, k, bx, n, fin & ~kInt8);
+        };
         for (auto& kv : m2m_mats) {
             const DirMats& M = kv.second;
             for (int ind = 0; ind < 8 && !M.cached; ++ind) {
+                if (M.fin[ind] == kNone) continue;
                 const bool hf = M.ccanon >= 0;  // else the children are low-frequency boxes
                 const size_t in = hf ? M.tmp[ind] : M.raw[ind], mid = hf ? M.raw[ind] : M.tmp[ind];
                 if (hf) right.product(dscr + M.raw[ind], M.rmid, M.mcols, scr_E1[M.ccanon], M.mcols, M.tmp[ind]);
                 left.product(hfcanon[M.canon].E3, M.rmid, M.rmid, in, M.mcols, mid);
-                last.product(hfcanon[M.canon].E2, M.mrows, M.rmid, mid, M.mcols, M.fin[ind]);
+                fold(hfcanon[M.canon].E2, M.mrows, M.rmid, mid, M.mcols, M.fin[ind]);
             }
         }
         for (auto& kv : l2l_mats) {
             const DirMats& M = kv.second;
             for (int ind = 0; ind < 8 && !M.cached; ++ind) {
+                if (M.fin[ind] == kNone) continue;
                 const bool hf = M.ccanon >= 0;
                 const size_t mid = hf ? M.raw[ind] : M.tmp[ind];
                 right.product(dscr + M.raw[ind], M.mrows, M.rmid, scr_E3t[M.canon], M.rmid, M.tmp[ind]);
                 if (hf) left.product(hfcanon[M.ccanon].E1t, M.mrows, M.mrows, M.tmp[ind], M.rmid, mid);
-                last.product(dscr + mid, M.mrows, M.rmid, scr_E2t[M.canon], M.mcols, M.fin[ind]);
+                fold(dscr + mid, M.mrows, M.rmid, scr_E2t[M.canon], M.mcols, M.fin[ind]);
             }
         }
         for (const M2LMat& M : m2l_mats) {
             if (M.pk) continue;
             right.product(dscr + M.raw, M.r1, M.r1, scr_E1[M.canon], M.r1, M.tmp);
-            last.product(hfcanon[M.canon].E1t, M.r1, M.r1, M.tmp, M.r1, M.fin);
+            fold(hfcanon[M.canon].E1t, M.r1, M.r1, M.tmp, M.r1, M.fin);
         }
         right.run(dscr, dscr, stream_);
         left.run(dscr, dscr, stream_);
         last.run(dscr, dkeep, stream_);
+        last8.run(dscr, dkeep8, stream_);
         CK(cudaStreamSynchronize(stream_));
         CK(cudaFree(dscr));
     }
     phase("fold");
     const double2* dkeepm = opm(dkeep, keep);
-    auto KP = [&](size_t off) { return E((double2*)dkeepm, off); };
+    auto KP = [&](size_t fin) { return fin & kInt8 ? dkeep8 + (fin & ~kInt8) : E((double2*)dkeepm, fin); };
 
     // ---------------------------------------------------------------- steps: LF upward
     auto lf_set = [&](const double* x, int n, Pt3 shift, double scale) {
@@ -1484,81 +1572,50 @@ void Session::build() {
     }
 
     phase("steps_lf_up");
-    // children with points of every high-frequency box (-1: none)
-    std::vector<int> kids((size_t)nb * 8, -1);
-    for (auto& kv : hflevels)
-        for (int b : kv.second)
-            for (int ind = 0; ind < 8; ++ind) {
-                const int c = T.child(b, ind);
-                if (c >= 0 && T.boxes[c].has_pts()) kids[(size_t)b * 8 + ind] = c;
-            }
-    // the column lists of every level's M2M and L2L launches, built on all host cores (plan.cpp)
-    std::vector<std::pair<double, Idx3> > did_wedge(dirpts.size());
-    for (auto& kv : dirpts) did_wedge[kv.second.did] = kv.first;
-    std::vector<long long> lf_off(nb, -1);
-    for (int l = 0; l < nLF; ++l) lf_off[lfbox[l]] = (long long)l * nE;
-    HfColumns cols = hf_columns(T, up, dn, kids, lf_off, dirpts.size(), hfcanon.size(), false);
-    phase("hf_columns");
     // ---------------------------------------------------------------- digits of the HF inputs
-    // plain form: of the launches with problems large enough for the int8 path; tcgen05
-    // form: FP16 planes, of all
-    Digits lf_dg, up_dg, dn_dg;
-    std::map<int, std::vector<char> > m2m_i8, m2l_i8, l2l_i8;  // level -> problems on the int8 path
-    std::set<int> up_i8, dn_i8;  // levels whose outgoing / incoming vectors are written as digits
-    bool lf_i8 = false;
-    if (!mixed || umma()) {
-        auto choose = [&](const std::vector<std::array<int, 3> >& shapes) {
-            if (umma()) return std::vector<char>(shapes.size(), 1);
-            if (prm_.int8_rule == INT8_BY_SIZE) return i8_choose(shapes);
-            std::vector<char> on(prm_.int8_rule == INT8_ALTERNATE ? shapes.size() : 0);
-            for (size_t i = 0; i < on.size(); i += 2) on[i] = 1;
-            return on;
-        };
-        long long dn_most = 0;
-        for (auto& kv : hflevels) {
-            const int level = kv.first;
-            const double W = T.width(level);
-            auto shapes = [&](const ColLists& L, const std::map<std::pair<double, Idx3>, DirMats>& mats) {
-                std::vector<std::array<int, 3> > v;
-                if (umma()) v.resize(L.key.size());  // all of them
-                for (size_t i = v.size(); i < L.key.size(); ++i) {
-                    const DirMats& M = mats.at(std::make_pair(W, did_wedge[L.key[i] / 8].second));
-                    v.push_back({{M.mrows, M.mcols, (int)L.x[i].size()}});
-                }
-                return v;
-            };
-            std::vector<std::array<int, 3> > far;
-            for (size_t i = 0; i < m2l_probs[level].size(); ++i) {
-                const int r1 = m2l_mats[m2l_probs[level][i]].r1;
-                far.push_back({{r1, r1, (int)m2l_x[level][i].size()}});
-            }
-            m2m_i8[level] = choose(shapes(cols.m2m.at(level), m2m_mats));
-            m2l_i8[level] = choose(far);
-            l2l_i8[level] = choose(shapes(cols.l2l.at(level), l2l_mats));
-            if (!m2m_i8[level].empty()) {
-                if (W == 1.0)
-                    lf_i8 = true;
-                else
-                    up_i8.insert(level + 1);
-            }
-            if (!m2l_i8[level].empty()) up_i8.insert(level);
-            if (!l2l_i8[level].empty()) {
-                dn_i8.insert(level);
-                const auto dr = dn.range[level];
-                dn_most = std::max(dn_most, (dr.second == (int)dn.v.size() ? dnchk_total : dn.v[dr.second].off) - dn.v[dr.first].off);
-            }
-        }
-        auto room = [&](Digits& d, size_t granules) {
-            d.X8 = dalloc<char>(granules * (umma() ? H16_GRANULE : I8_GRANULE));
-            d.cx = dalloc<double>(granules);
-        };
+    // (mixed form: FP16 planes) of the vectors that the products on those routes gather
+    Digits lf_dg;
+    std::map<int, Digits> up_dg, dn_dg;  // by level
+    char* dg_X8 = nullptr;               // of the high-frequency levels
+    size_t dg_bytes = 0;
+    {
+        const size_t gb = umma() ? H16_GRANULE : I8_GRANULE, cb = umma() ? sizeof(float) : sizeof(double);
         lf_dg.unit = nE;
         lf_dg.gran = (nE + 15) / 16;
-        if (lf_i8) room(lf_dg, (size_t)nLF * lf_dg.gran);
-        if (!up_i8.empty()) room(up_dg, (size_t)upeq_total / 16);
-        if (!dn_i8.empty()) room(dn_dg, (size_t)dn_most / 16);
-        if (!mixed && (lf_i8 || !up_i8.empty() || !dn_i8.empty())) i8_init();
+        if (lf_i8) {
+            lf_dg.X8 = dalloc<char>((size_t)nLF * lf_dg.gran * gb);
+            lf_dg.cx = dalloc<char>((size_t)nLF * lf_dg.gran * cb);
+        }
+        // Outgoing digits of a level are read by the M2M above it and last by its M2L, then
+        // its incoming ones are written and read by its L2L: one place for both.
+        auto place = [&](const HfNodes& N, int level, long long total, Digits& d) {  // base; granules of the level
+            const auto r = N.range.at(level);
+            if (r.first == r.second) return (size_t)0;
+            d.base = N.v[r.first].off;
+            return (size_t)((r.second == (int)N.v.size() ? total : N.v[r.second].off) - d.base) / 16;
+        };
+        size_t granules = 0;
+        std::map<int, size_t> at;
+        for (auto& kv : hflevels) {
+            const int level = kv.first;
+            at[level] = granules;
+            const size_t u = up_i8.count(level) ? place(up, level, upeq_total, up_dg[level]) : 0;
+            const size_t d = dn_i8.count(level) ? place(dn, level, dnchk_total, dn_dg[level]) : 0;
+            granules += std::max(u, d);
+        }
+        if (granules) {
+            dg_bytes = granules * gb;
+            dg_X8 = dalloc<char>(dg_bytes);
+            char* cx = dalloc<char>(granules * cb);
+            for (std::map<int, Digits>* m : {&up_dg, &dn_dg})
+                for (auto& kv : *m) {
+                    kv.second.X8 = dg_X8 + at[kv.first] * gb;
+                    kv.second.cx = cx + at[kv.first] * cb;
+                }
+        }
+        if (!mixed && (lf_i8 || granules)) i8_init();
     }
+    phase("digit_buffers");
     auto add_node_digits = [&](const HfNodes& N, int level, const double2* X, const Digits& d, const char* label) {
         const auto r = N.range.at(level);
         const size_t n = (size_t)(r.second - r.first);
@@ -1602,9 +1659,9 @@ void Session::build() {
                 }
             }
             add_gemm(probs, L.x, L.y, W == 1.0 ? lf_upeq : hf_upeq, hf_upeq, GEMM_ATOMIC, width_label("hf_m2m", W),
-                     W == 1.0 ? &lf_dg : &up_dg, &m2m_i8[level]);
+                     W == 1.0 ? &lf_dg : &up_dg[level + 1], &m2m_i8[level]);
         }
-        if (up_i8.count(level)) add_node_digits(up, level, hf_upeq, up_dg, "hf_digits_up");
+        if (up_i8.count(level)) add_node_digits(up, level, hf_upeq, up_dg[level], "hf_digits_up");
     }
 
     phase("steps_hf_up");
@@ -1628,13 +1685,10 @@ void Session::build() {
                     if (!opctx_.empty()) opkey_[KP(M.fin)] = M.key;
                 }
             }
-            add_gemm(probs, m2l_x[level], m2l_y[level], hf_upeq, hf_dnchk, GEMM_ATOMIC, width_label("hf_m2l", W), &up_dg,
-                     &m2l_i8[level]);
+            add_gemm(probs, m2l_x[level], m2l_y[level], hf_upeq, hf_dnchk, GEMM_ATOMIC, width_label("hf_m2l", W),
+                     &up_dg[level], &m2l_i8[level]);
         }
-        if (dn_i8.count(level)) {
-            dn_dg.base = dn.v[dr.first].off;  // one level's digits at a time
-            add_node_digits(dn, level, hf_dnchk, dn_dg, "hf_digits_down");
-        }
+        if (dn_i8.count(level)) add_node_digits(dn, level, hf_dnchk, dn_dg[level], "hf_digits_down");
         // L2L into the children's (pdir) u, or LF dnchkval at W=1 (src/wave3d_eval.cpp:938-991),
         // one launch for the 8 child positions: a problem per (wedge, child)
         {
@@ -1652,7 +1706,7 @@ void Session::build() {
                 }
             }
             add_gemm(probs, L.x, L.y, hf_dnchk, W == 1.0 ? lf_dnchk : hf_dnchk, GEMM_ATOMIC, width_label("hf_l2l", W),
-                     &dn_dg, &l2l_i8[level]);
+                     &dn_dg[level], &l2l_i8[level]);
         }
     }
 
@@ -1667,6 +1721,10 @@ void Session::build() {
         branch_ev_.resize(2 + 2 * branch_.size() + 2 * lflevels.size());
         for (cudaEvent_t& e : branch_ev_) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
+    // Source spectra: each eval writes every one it reads.  Where no pass overlaps another the
+    // high-frequency passes are over by then, and their digits' memory will do.
+    const size_t spec_bytes = (size_t)nLF * G3 * es;
+    double2* lf_spec = !overlap_ && spec_bytes <= dg_bytes ? (double2*)dg_X8 : salloc((size_t)nLF * G3);
     // ---------------------------------------------------------------- steps: LF downward
     for (auto& kv : lflevels) {  // levels ascending = widths descending
         int level = kv.first;
@@ -1877,6 +1935,10 @@ void Session::build() {
                      t_emit_gemm_, t_emit_vgroups_, t_big_uploads_, t_pack_, t_pack_alloc_, n_malloc_, t_malloc_,
                      n_stage_, t_stage_wait_, t_stage_copy_);
     flush_packs();
+    if (dkeep8) {  // packed as digits by now
+        CK(cudaStreamSynchronize(stream_));
+        dfree(dkeep8);
+    }
     if (mixed) {
         // the mixed eval reads only the FP32 copies (and, on tcgen05, only the packed
         // GEMM operators): release the FP64 operators and the unpacked GEMM copies
