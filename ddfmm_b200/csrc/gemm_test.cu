@@ -44,7 +44,7 @@ void test_gemm(const double2* A, int m, int k, const double2* X, int ncol, int p
         xo[c] = (long long)at * sx;
         yo[c] = (long long)at * sy;
         xg[c] = at * (sx / 16);
-        vecs[c] = I8Vec{xo[c], xg[c], k};
+        vecs[c] = I8Vec{xo[c], xg[c], (unsigned short)k, (unsigned short)(path == 6)};
         for (int i = 0; i < k; ++i) hx[xo[c] + i] = X[(size_t)c * k + i];
         for (int i = 0; i < m; ++i) hy[yo[c] + i] = Y[(size_t)c * m + i];
     }
@@ -72,7 +72,7 @@ void test_gemm(const double2* A, int m, int k, const double2* X, int ncol, int p
         std::vector<double2> one((size_t)m * m, make_double2(0, 0));
         for (int i = 0; i < m; ++i) one[(size_t)i * m + i] = make_double2(1, 0);
         launch_gemm_pair(GemmPair{P.put(one), dA, m, m, ncol, P.put(xo), dX, dY}, nullptr);
-    } else if (path >= 3) {  // mixed form, on FP32 copies: 3 FP16 planes, 4 split TF32
+    } else if (path == 3 || path == 4) {  // mixed form, on FP32 copies: 3 FP16 planes, 4 split TF32
         auto narrow = [](const std::vector<double2>& v) {
             std::vector<float2> r;
             for (const double2& a : v) r.push_back(make_float2((float)a.x, (float)a.y));
@@ -126,9 +126,17 @@ void test_gemm(const double2* A, int m, int k, const double2* X, int ncol, int p
         i8_tiles(B, ra, m, k, 0, ncol, tiles);
         int* err = P.put(std::vector<int>(1, 0));
         i8_init();
-        launch_i8_pack(P.put(std::vector<I8PackJob>(1, I8PackJob{dA, B, ra, m, k, m, nkb, i8_tile_rows(m)})), 1,
+        unsigned char* prof = nullptr;
+        if (path == 6) {  // the columns as one class, in the place of an operator's output
+            prof = P.put(std::vector<unsigned char>(sx));
+            double* rowmax = P.put(std::vector<double>(sx, 0.0));
+            launch_i8_profile(P.put(std::vector<I8ProfileJob>(1, I8ProfileJob{dX, k, ncol, sx, -1, 0})), 1, rowmax,
+                              I8Profiles{prof, sx}, nullptr);
+            launch_i8_profile_scale(rowmax, 1, sx, prof, nullptr);
+        }
+        launch_i8_pack(P.put(std::vector<I8PackJob>(1, I8PackJob{dA, B, ra, m, k, m, nkb, i8_tile_rows(m), prof})), 1,
                        i8_row_tiles(m), nullptr);
-        launch_i8_slice(P.put(vecs), ncol, dX, X8, cx, nullptr);
+        launch_i8_slice(P.put(vecs), ncol, dX, X8, cx, I8Profiles{prof, sx}, nullptr);
         launch_i8_gemm(I8Sub{P.put(tiles), P.put(xg), dyo, X8, cx, dY, (int)tiles.size()}, err, nullptr);
         int h = 0;
         ck(cudaMemcpy(&h, err, sizeof(int), cudaMemcpyDeviceToHost));

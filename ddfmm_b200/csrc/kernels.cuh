@@ -17,6 +17,7 @@ struct GemmProblem {
     int col0;  // first entry in the column arrays
     int ncol;
     const float* packed;  // tcgen05 form: an already packed copy of A (A may then be null)
+    int profile;          // int8 path: 1 + the row of the profile table that scales its columns' vectors; 0: none
 };
 // A launch is a list of output tiles of up to GEMM_TILE_M rows x GEMM_TILE_N columns.
 constexpr int GEMM_TILE_M = 64, GEMM_TILE_N = 64;
@@ -284,9 +285,26 @@ constexpr int I8_GRANULE = 16 * 2 * I8_DIGITS;  // bytes of the digits of 16 com
 struct I8Vec {      // a vector to write as digits
     long long src;  // its first element in X
     int gran;       // its first granule (and its entry of cx)
-    int len;        // complex numbers
+    unsigned short len;      // complex numbers
+    unsigned short profile;  // as in GemmProblem
 };
-void launch_i8_slice(const I8Vec* vecs, int n, const double2* X, char* X8, double* cx, cudaStream_t s);
+// Profile table: a row of `stride` exponents, 0 .. 60, for each class of vectors.  Component j of
+// a vector of row p is scaled by 2^-prof[p * stride + j] before it is written as digits, column
+// j of an operator on it by the inverse (kernels_i8.cu).
+struct I8Profiles {
+    const unsigned char* prof;
+    int stride;
+};
+struct I8ProfileJob {  // an operator that adds into vectors of class `out` from vectors of class `in` (-1: none)
+    const double2* A;
+    int m, k, lda, in, out;
+};
+// largest component of each row of operators, columns weighted by class `in`'s profile
+// (2^prof), into rowmax (classes x stride, from 0); then the profiles of all classes from it
+void launch_i8_profile(const I8ProfileJob* jobs, int n, double* rowmax, const I8Profiles& T, cudaStream_t s);
+void launch_i8_profile_scale(const double* rowmax, int classes, int stride, unsigned char* prof, cudaStream_t s);
+void launch_i8_slice(const I8Vec* vecs, int n, const double2* X, char* X8, double* cx, const I8Profiles& T,
+                     cudaStream_t s);
 struct alignas(16) I8Tile {  // everything about a tile, so that its next one can be read ahead
     const char* B;         // the row tile's packed operator (i8_pack_kernel)
     const double* ra;      // output scales of its rows
@@ -307,6 +325,7 @@ struct I8PackJob {
     char* dst;
     double* ra;
     int m, k, lda, nkb, rows_t;
+    const unsigned char* prof;  // of its columns, or null
 };
 void i8_init();
 int i8_row_tiles(int m);

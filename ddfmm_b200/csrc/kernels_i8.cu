@@ -4,16 +4,23 @@
 // an m x k complex operator.  The FP64 tensor path peaks at 37 TF/s; the int8
 // path does 34 exact integer products per FP64 product at over 100 times that
 // rate.  Every column (and every operator row) is written as
-//     x_j = 2^(ex - 54) q_j,   q_j = sum_{i=0}^{6} d_i 256^(6-i),  d_i in [-128, 127],
-// 2^ex above the vector's largest component: 54 bits below it, a rounding of at
-// most half the last place of the largest FP64 entry.  With X's digits d and A's
+//     x_j = 2^(ex - 55) q_j,   q_j = sum_{i=0}^{6} d_i 256^(6-i),  d_i in [-128, 127],
+// 2^ex above the vector's largest component: 55 bits below it (54 where its mantissa
+// is above 1.988), a quarter of the largest FP64 entry's last place.  With X's digits d and A's
 // digits e, a product of two numbers is sum_{i,j} d_i e_j 256^(12-i-j); the terms
 // i + j <= 7 are kept (34 of 49; the dropped ones are below 2^-58 of the largest
 // product).  Those of one diagonal i + j are summed over k by the tensor core in
 // int32 without any rounding, the eight diagonals joined in int64 and rounded to
-// FP64 twice per output, so the sums over k carry no rounding error at all: on
-// folded translation operators at P = 4, 6, 8 the result is 0.9-2.2e-16 from a
-// long-double product in relative 2-norm, the three-MMA FP64 form 3-8e-16.
+// FP64 twice per output, so the sums over k carry no rounding error at all.
+//
+// 55 bits below the largest component are worth as many of each product only where
+// the components are of one size.  Outgoing vectors' are not: they differ by up to 10^8
+// where the operators' columns differ the other way round.  Both are scaled by powers
+// of two before they become digits (i8_profile_kernel).  Against long-double products, on
+// the operators and vectors of evals (spheres, ellipsoids and clusters, K = 8 .. 32, both
+// kernels, P = 4, 6, 8, four kinds of densities), the relative 2-norm error is 5e-17 to
+// 7e-16 by pass, the three-MMA FP64 form's 3e-16 to 1.6e-15 and larger in each of them; M2L
+// products without the scaling were off by 4e-14, 5e-12 and 1e-10 at P = 4, 6, 8.
 //
 // One tile is 128 gathered columns (the MMA's M, one TMEM lane each) x up to 56
 // complex operator rows; operator row i becomes the int8 rows [Ar, -Ai] and
@@ -51,6 +58,8 @@
 // sets *err.
 #include <cuda_runtime.h>
 
+#include <cfloat>
+#include <climits>
 #include <cstdint>
 #include <stdexcept>
 
@@ -202,37 +211,43 @@ __device__ __forceinline__ bool i8_phase(uint32_t tmem, uint32_t dx0, int nkb, I
 }
 
 // ---------------------------------------------------------------- digits
-// The seven balanced base-256 digits of q, |q| <= 2^54: adding 128 to every
+// The seven balanced base-256 digits of q, |q| <= 0.996 2^55: adding 128 to every
 // digit place makes them the bytes of one sum; flipping each byte's top bit
 // takes the 128 off again.  Byte i of the result is digit 6 - i.
 constexpr unsigned long long I_BIAS = 0x0080808080808080ull;
 __device__ __forceinline__ unsigned long long i8_digits(long long q) { return ((unsigned long long)q + I_BIAS) ^ I_BIAS; }
 
-// Largest |x| of a vector by its high word (sign off): the vector's exponent ex
-// (largest |x| < 2^ex), the factor 2^(54 - ex) as two powers of two (a vector
-// below 2^-900 is brought up first, so subnormals keep their bits) and
-// 2^(ex - 1); NaN when the vector holds an infinity or a NaN, zero when it is zero.
+// Scale of a vector (operator row) whose largest component has the high word `top` (sign
+// off): s = 2^(55 - ex), which makes it an integer below 0.9942 2^55 (seven balanced digits
+// reach 0.9960 2^55), and out = 2^(ex - 1).  A vector with nothing above 2^-823 is brought up by
+// 2^200 first (low), so subnormals keep their bits.  NaN when the vector holds an infinity or
+// a NaN.
+constexpr int I_UP = 200;
+constexpr uint32_t I_LOW = 200u << 20;  // top below it: low
 struct I8Scale {
-    double up, s, out;
+    double s, out;
 };
-__device__ __forceinline__ I8Scale i8_scale(uint32_t top) {
+__device__ __forceinline__ double i8_pow2(int e) { return __longlong_as_double((long long)(1023 + e) << 52); }
+__device__ __forceinline__ I8Scale i8_scale(uint32_t top, bool low) {
     I8Scale r;
     const int be = (int)(top >> 20);
     if (be == 0x7ff) {
-        r.up = r.s = 0.0;
+        r.s = 0.0;
         r.out = __longlong_as_double(0x7ff8000000000000ll);
         return r;
     }
-    const int b1 = be < 1 ? 1 : be;  // subnormals: below 2^-1022
-    const bool low = b1 < 123;
-    r.up = low ? __longlong_as_double((long long)(1023 + 200) << 52) : 1.0;
-    r.s = __longlong_as_double((long long)(2099 - b1 - (low ? 200 : 0)) << 52);  // 2^(1076 - b1 [- 200])
-    r.out = __longlong_as_double((long long)(b1 == 0 ? 1 : b1) << 52);           // 2^(b1 - 1023) = 2^(ex - 1)
+    if (top == 0) {  // zero
+        r.s = r.out = 1.0;
+        return r;
+    }
+    const int b1 = be + ((top & 0xfffffu) >= 0xfd000u);  // ex + 1022
+    r.s = __longlong_as_double((long long)(2100 - b1) << 52);
+    const int bo = b1 - (low ? I_UP : 0);
+    r.out = bo >= 1 ? __longlong_as_double((long long)bo << 52) : __longlong_as_double(bo >= -51 ? 1ll << (bo + 51) : 0ll);
     return r;
 }
-__device__ __forceinline__ long long i8_quant(double x, const I8Scale& S) { return __double2ll_rn(x * S.up * S.s); }
+__device__ __forceinline__ long long i8_quant(double x, const I8Scale& S) { return __double2ll_rn(x * S.s); }
 __device__ __forceinline__ uint32_t top_word(double x) { return (uint32_t)__double2hiint(x) & 0x7fffffffu; }
-// high word of |x| counting a nonzero low word of a value whose high word is zero
 __device__ __forceinline__ uint32_t top_of(double2 v) { return max(top_word(v.x), top_word(v.y)); }
 
 // eight digit bytes, place p of eight numbers: byte p of w[0..7]
@@ -254,50 +269,115 @@ __device__ __forceinline__ uint2 gather_bytes(const unsigned long long (&w)[8], 
 
 // Digits of vectors: one warp per vector, four lanes per granule of 16 complex
 // numbers (each lane 4 of them: 8 bytes in each of the 7 planes).  Bound by
-// HBM: 16 bytes read and 14 written per complex number.
+// HBM: 16 bytes read and 14 written per complex number; the profiles come from L2.
 __global__ void __launch_bounds__(256) i8_slice_kernel(const I8Vec* __restrict__ vecs, int n,
                                                        const double2* __restrict__ X, char* __restrict__ X8,
-                                                       double* __restrict__ cx) {
+                                                       double* __restrict__ cx, const I8Profiles T) {
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (w >= n) return;
     const I8Vec V = vecs[w];
     const double2* x = X + V.src;
-    uint32_t top = 0;
+    const unsigned char* prof = V.profile ? T.prof + (size_t)(V.profile - 1) * T.stride : nullptr;
     double2 v[4];
-    const int ng = (V.len + 15) >> 4;
-    for (int g0 = 0; g0 < ng; g0 += 8) {  // 8 granules a pass
-        const int j0 = g0 * 16 + lane * 4;
+    auto load = [&](int j0, int up) {
+        const uint32_t e = prof && j0 < V.len ? __ldg(reinterpret_cast<const uint32_t*>(prof + j0)) : 0u;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            v[j] = j0 + j < V.len ? x[j0 + j] : make_double2(0.0, 0.0);
-            top = max(top, top_of(v[j]));
+            const double2 a = j0 + j < V.len ? x[j0 + j] : make_double2(0.0, 0.0);
+            const double f = i8_pow2(up - (int)((e >> (8 * j)) & 255u));
+            v[j] = make_double2(a.x * f, a.y * f);
         }
-    }
-    top = __reduce_max_sync(0xffffffffu, top);
-    const I8Scale S = i8_scale(top);
-    if (lane == 0) cx[V.gran] = S.out;
-    for (int g0 = 0; g0 < ng; g0 += 8) {
-        const int j0 = g0 * 16 + lane * 4;
-        if (ng > 8) {
+    };
+    auto top_at = [&](int up) {  // of the whole vector
+        uint32_t top = 0;
+        for (int j0 = 0; j0 < V.len; j0 += 128) {
+            load(j0 + lane * 4, up);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) v[j] = j0 + j < V.len ? x[j0 + j] : make_double2(0.0, 0.0);
+            for (int j = 0; j < 4; ++j) top = max(top, top_of(v[j]));
         }
-        if (g0 + (lane >> 2) < ng) {
+        return __reduce_max_sync(0xffffffffu, top);
+    };
+    int up = 0;
+    uint32_t top = top_at(up);
+    if (top < I_LOW) top = top_at(up = I_UP);
+    const I8Scale S = i8_scale(top, up > 0);
+    if (lane == 0) cx[V.gran] = S.out;
+    for (int j0 = 0; j0 < V.len; j0 += 128) {
+        if (V.len > 128) load(j0 + lane * 4, up);
+        const int g = (j0 >> 4) + (lane >> 2);
+        if (g * 16 < V.len) {
             unsigned long long q[8];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 q[2 * j] = i8_digits(i8_quant(v[j].x, S));
                 q[2 * j + 1] = i8_digits(i8_quant(v[j].y, S));
             }
-            char* o = X8 + (size_t)(V.gran + g0 + (lane >> 2)) * I8_GRANULE + (lane & 3) * 8;
+            char* o = X8 + (size_t)(V.gran + g) * I8_GRANULE + (lane & 3) * 8;
 #pragma unroll
             for (int p = 0; p < IS; ++p) *reinterpret_cast<uint2*>(o + p * 32) = gather_bytes(q, IS - 1 - p);
         }
     }
 }
 
-void launch_i8_slice(const I8Vec* vecs, int n, const double2* X, char* X8, double* cx, cudaStream_t s) {
-    if (n > 0) i8_slice_kernel<<<(unsigned)(((size_t)n * 32 + 255) / 256), 256, 0, s>>>(vecs, n, X, X8, cx);
+void launch_i8_slice(const I8Vec* vecs, int n, const double2* X, char* X8, double* cx, const I8Profiles& T,
+                     cudaStream_t s) {
+    if (n > 0) i8_slice_kernel<<<(unsigned)(((size_t)n * 32 + 255) / 256), 256, 0, s>>>(vecs, n, X, X8, cx, T);
+}
+
+// Profiles of classes of vectors (setup only).  An outgoing vector w of a (width, wedge)
+// is the output of the M2M operators into it, whose rows differ by up to 10^8 in size (E2's
+// do), and the operators on w have columns as much smaller where w is large; 55 bits
+// below the largest component, or operator entry, would leave little of the products that
+// count.  Scaled by the rows' largest entries both are flat.  (Maxima: the profile does not
+// depend on the order in which operators add to it.)  A block an operator, a thread a row.
+__global__ void __launch_bounds__(128) i8_profile_kernel(const I8ProfileJob* __restrict__ jobs, int n, double* rowmax,
+                                                         const I8Profiles T) {
+    for (int j = blockIdx.x; j < n; j += gridDim.x) {
+        const I8ProfileJob J = jobs[j];
+        for (int r = threadIdx.x; r < J.m; r += 128) {
+            double top = 0.0;
+            for (int k = 0; k < J.k; ++k) {
+                const double2 a = J.A[(size_t)k * J.lda + r];
+                const double w = J.in >= 0 ? i8_pow2(T.prof[(size_t)J.in * T.stride + k]) : 1.0;
+                top = fmax(top, fmax(fabs(a.x), fabs(a.y)) * w);
+            }
+            // positive numbers are ordered as their bits are
+            atomicMax(reinterpret_cast<unsigned long long*>(rowmax + (size_t)J.out * T.stride + r),
+                      (unsigned long long)__double_as_longlong(top));
+        }
+    }
+}
+// The profile of a class: e_j - e0, e_j the exponent of row j's largest entry and e0 the
+// smallest of them but no less than the largest one - 60; rows of zeros count as the smallest.
+// (Vectors are scaled down only: none overflows.)  One block a class.
+__global__ void __launch_bounds__(128) i8_profile_scale_kernel(const double* __restrict__ rowmax, int stride,
+                                                               unsigned char* __restrict__ prof) {
+    __shared__ int lo, hi;
+    const double* s = rowmax + (size_t)blockIdx.x * stride;
+    auto expo = [](double v) { return v > 0.0 && v <= DBL_MAX ? ilogb(v) : INT_MIN; };
+    if (threadIdx.x == 0) {
+        lo = INT_MAX;
+        hi = INT_MIN;
+    }
+    __syncthreads();
+    for (int r = threadIdx.x; r < stride; r += 128) {
+        const int e = expo(s[r]);
+        if (e != INT_MIN) {
+            atomicMin(&lo, e);
+            atomicMax(&hi, e);
+        }
+    }
+    __syncthreads();
+    const int e0 = hi == INT_MIN ? 0 : max(lo, hi - 60);
+    for (int r = threadIdx.x; r < stride; r += 128)
+        prof[(size_t)blockIdx.x * stride + r] = (unsigned char)(max(expo(s[r]), e0) - e0);
+}
+
+void launch_i8_profile(const I8ProfileJob* jobs, int n, double* rowmax, const I8Profiles& T, cudaStream_t s) {
+    if (n > 0) i8_profile_kernel<<<n < 65535 ? n : 65535, 128, 0, s>>>(jobs, n, rowmax, T);
+}
+void launch_i8_profile_scale(const double* rowmax, int classes, int stride, unsigned char* prof, cudaStream_t s) {
+    if (classes > 0) i8_profile_scale_kernel<<<classes, 128, 0, s>>>(rowmax, stride, prof);
 }
 
 // Operator digits (setup only): block (row tile, job).  Row scales first, then
@@ -306,26 +386,35 @@ void launch_i8_slice(const I8Vec* vecs, int n, const double2* X, char* X8, doubl
 __global__ void __launch_bounds__(256) i8_pack_kernel(const I8PackJob* __restrict__ jobs, int njobs) {
     __shared__ uint32_t tops[4][64];
     __shared__ I8Scale sc[64];
+    __shared__ bool low[64];
     const int tid = threadIdx.x;
     for (int j = blockIdx.y; j < njobs; j += gridDim.y) {
         const I8PackJob J = jobs[j];
         const int row0 = blockIdx.x * J.rows_t;
         if (row0 >= J.m) continue;  // uniform over the block
-        __syncthreads();
-        {
+        // column k as the vectors' profile leaves it, brought up where the row is low
+        auto entry = [&](int r, int k, bool up) {
+            const double2 a = J.A[(size_t)k * J.lda + row0 + r];
+            const double f = i8_pow2((J.prof ? J.prof[k] : 0) + (up ? I_UP : 0));
+            return make_double2(a.x * f, a.y * f);
+        };
+        for (int up = 0; up < 2; ++up) {
+            __syncthreads();
             const int r = tid & 63;
             uint32_t top = 0;
-            if (r < J.rows_t && row0 + r < J.m)
-                for (int k = tid >> 6; k < J.k; k += 4) top = max(top, top_of(J.A[(size_t)k * J.lda + row0 + r]));
+            if (r < J.rows_t && row0 + r < J.m && (up == 0 || low[r]))
+                for (int k = tid >> 6; k < J.k; k += 4) top = max(top, top_of(entry(r, k, up)));
             tops[tid >> 6][r] = top;
+            __syncthreads();
+            if (tid < J.rows_t) {
+                const uint32_t t = max(max(tops[0][tid], tops[1][tid]), max(tops[2][tid], tops[3][tid]));
+                if (up == 0) low[tid] = t < I_LOW;
+                if (up == 0 || low[tid]) sc[tid] = i8_scale(t, up);
+            }
         }
-        __syncthreads();
-        if (tid < J.rows_t) {
-            sc[tid] = i8_scale(max(max(tops[0][tid], tops[1][tid]), max(tops[2][tid], tops[3][tid])));
-            // the output scale of a row: 2^(ea - 1) 2^-34 (the epilogue's sums count units
-            // of diagonal 3: 256^9 2^(ex - 54) 2^(ea - 54) = 2^(ex + ea - 36), and cx = 2^(ex - 1))
-            if (row0 + tid < J.m) J.ra[row0 + tid] = sc[tid].out * 0x1p-34;
-        }
+        // the output scale of a row: 2^(ea - 1) 2^-36 (the epilogue's sums count units
+        // of diagonal 3: 256^9 2^(ex - 55) 2^(ea - 55) = 2^(ex + ea - 38), and cx = 2^(ex - 1))
+        if (tid < J.rows_t && row0 + tid < J.m) J.ra[row0 + tid] = sc[tid].out * 0x1p-36;
         __syncthreads();
         const int nq = J.nkb * 4, N = 2 * J.rows_t;
         char* dst = J.dst + (size_t)blockIdx.x * J.nkb * IS * N * 32;
@@ -336,7 +425,7 @@ __global__ void __launch_bounds__(256) i8_pack_kernel(const I8PackJob* __restric
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const bool ok = row0 + r < J.m && k0 + i < J.k;
-                const double2 a = ok ? J.A[(size_t)(k0 + i) * J.lda + row0 + r] : make_double2(0.0, 0.0);
+                const double2 a = ok ? entry(r, k0 + i, low[r]) : make_double2(0.0, 0.0);
                 const long long qr = i8_quant(a.x, S), qi = i8_quant(a.y, S);
                 w0[2 * i] = w1[2 * i + 1] = i8_digits(qr);
                 w0[2 * i + 1] = i8_digits(-qi);

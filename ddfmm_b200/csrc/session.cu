@@ -467,7 +467,8 @@ void Session::add_i8(const std::vector<GemmProblem>& P, const long long* xs, con
     double* ra = dalloc<double>(rows);
     for (size_t i = 0; i < P.size(); ++i) {
         const GemmProblem& q = P[i];
-        jobs.push_back(I8PackJob{q.A, B, ra, q.m, q.k, q.lda, (q.k + 15) / 16, i8_tile_rows(q.m)});
+        const unsigned char* prof = q.profile ? i8_prof_.prof + (size_t)(q.profile - 1) * i8_prof_.stride : nullptr;
+        jobs.push_back(I8PackJob{q.A, B, ra, q.m, q.k, q.lda, (q.k + 15) / 16, i8_tile_rows(q.m), prof});
         i8_tiles(B, ra, q.m, q.k, q.col0, q.ncol, tiles);
         B += i8_packed_bytes(q.m, q.k);
         ra += q.m;
@@ -1326,6 +1327,7 @@ void Session::build() {
     if (!mixed || umma()) {
         auto choose = [&](const std::vector<std::array<int, 3> >& shapes) {
             if (umma()) return std::vector<char>(shapes.size(), 1);
+            if (hfcanon.size() >= 65535) return std::vector<char>();  // I8Vec::profile has 16 bits
             if (prm_.int8_rule == INT8_BY_SIZE) return i8_choose(shapes);
             std::vector<char> on(prm_.int8_rule == INT8_ALTERNATE ? shapes.size() : 0);
             for (size_t i = 0; i < on.size(); i += 2) on[i] = 1;
@@ -1616,14 +1618,44 @@ void Session::build() {
         if (!mixed && (lf_i8 || granules)) i8_init();
     }
     phase("digit_buffers");
+    // Profiles of the outgoing vectors (kernels_i8.cu), by width upward: a width's operators
+    // read vectors of the one below.  Incoming vectors are flat as they are.
+    if (!mixed && !up_i8.empty()) {
+        int stride = 0;
+        for (const Canon& c : hfcanon) stride = std::max(stride, (c.r1 + 15) & ~15);
+        unsigned char* prof = dalloc<unsigned char>(hfcanon.size() * stride);
+        i8_prof_ = I8Profiles{prof, stride};
+        double* rowmax = nullptr;
+        CK(cudaMalloc(&rowmax, sizeof(double) * hfcanon.size() * stride));
+        CK(cudaMemsetAsync(rowmax, 0, sizeof(double) * hfcanon.size() * stride, stream_));
+        for (auto hit = hflevels.rbegin(); hit != hflevels.rend(); ++hit) {
+            std::vector<I8ProfileJob> v;
+            for (int k : cols.m2m.at(hit->first).key) {
+                const DirMats& M = *m2m_of[k / 8];
+                v.push_back(I8ProfileJob{KP(M.fin[k % 8]), M.mrows, M.mcols, M.mrows, M.ccanon, M.canon});
+            }
+            I8ProfileJob* dj = nullptr;
+            CK(cudaMalloc(&dj, sizeof(I8ProfileJob) * std::max<size_t>(v.size(), 1)));
+            CK(cudaMemcpyAsync(dj, v.data(), sizeof(I8ProfileJob) * v.size(), cudaMemcpyHostToDevice, stream_));
+            launch_i8_profile(dj, (int)v.size(), rowmax, i8_prof_, stream_);
+            launch_i8_profile_scale(rowmax, (int)hfcanon.size(), stride, prof, stream_);
+            CK(cudaGetLastError());
+            CK(cudaStreamSynchronize(stream_));
+            CK(cudaFree(dj));
+        }
+        CK(cudaFree(rowmax));
+        phase("digit_profiles");
+    }
     auto add_node_digits = [&](const HfNodes& N, int level, const double2* X, const Digits& d, const char* label) {
+        const bool profile = !mixed && &N == &up;
         const auto r = N.range.at(level);
         const size_t n = (size_t)(r.second - r.first);
         std::unique_ptr<I8Vec[]> v(new I8Vec[n]);  // not zeroed first
         host_parallel_for((n + 16383) / 16384, [&](size_t c) {
             for (size_t i = c * 16384; i < std::min(n, (c + 1) * 16384); ++i) {
                 const HfNode& u = N.v[r.first + i];
-                v[i] = I8Vec{u.off, (int)((u.off - d.base) / 16), hfcanon[u.canon].r1};
+                v[i] = I8Vec{u.off, (int)((u.off - d.base) / 16), (unsigned short)hfcanon[u.canon].r1,
+                             (unsigned short)(profile ? u.canon + 1 : 0)};
             }
         });
         add_digits(v.get(), n, X, d, label);
@@ -1638,7 +1670,7 @@ void Session::build() {
         begin_block(1, W);
         if (W == 1.0 && lf_i8) {
             std::vector<I8Vec> v;
-            for (int l : lflevels[level + 1]) v.push_back(I8Vec{(long long)l * nE, l * lf_dg.gran, nE});
+            for (int l : lflevels[level + 1]) v.push_back(I8Vec{(long long)l * nE, l * lf_dg.gran, (unsigned short)nE, 0});
             add_digits(v.data(), v.size(), lf_upeq, lf_dg, "lf_digits");
         }
         // M2M: w = sum_children [E2 E3 ue2uc E1(child)] w_child (src/wave3d_eval.cpp:796-849),
@@ -1654,7 +1686,7 @@ void Session::build() {
                 if (M.cached) {
                     probs.push_back(GemmProblem{nullptr, M.mrows, M.mcols, M.mrows, 0, 0, M.pk[ind]});
                 } else {
-                    probs.push_back(GemmProblem{KP(M.fin[ind]), M.mrows, M.mcols, M.mrows, 0, 0});
+                    probs.push_back(GemmProblem{KP(M.fin[ind]), M.mrows, M.mcols, M.mrows, 0, 0, nullptr, M.ccanon + 1});
                     if (!opctx_.empty()) opkey_[KP(M.fin[ind])] = opk("m2m", W, dir, ind);
                 }
             }
@@ -1681,7 +1713,7 @@ void Session::build() {
                 if (M.pk) {
                     probs.push_back(GemmProblem{nullptr, M.r1, M.r1, M.r1, 0, 0, M.pk});
                 } else {
-                    probs.push_back(GemmProblem{KP(M.fin), M.r1, M.r1, M.r1, 0, 0});
+                    probs.push_back(GemmProblem{KP(M.fin), M.r1, M.r1, M.r1, 0, 0, nullptr, M.canon + 1});
                     if (!opctx_.empty()) opkey_[KP(M.fin)] = M.key;
                 }
             }
@@ -2027,7 +2059,7 @@ void Session::launch_step(const Step& st, cudaStream_t s, double2* spec) {
             else
                 launch_vlist_inverse(st.v.L, st.v.trg, st.v.ntrg, st.v.tsp, st.v.dnchk, s);
             break;
-        case 7: launch_i8_slice(st.dg.vecs, st.dg.n, st.dg.X, st.dg.X8, st.dg.cx, s); break;
+        case 7: launch_i8_slice(st.dg.vecs, st.dg.n, st.dg.X, st.dg.X8, st.dg.cx, i8_prof_, s); break;
         case 8: launch_i8_gemm(st.i8, d_err_, s, stall_ns, stall_ns > 0); break;
         case 11: launch_gemm_pair(st.gp, s); break;
         case 9:

@@ -201,6 +201,7 @@ private:
     void add_gemm(std::vector<GemmProblem>& probs, std::vector<std::vector<long long> >& xo,
                   std::vector<std::vector<long long> >& yo, const double2* X, double2* Y, int mode,
                   const char* label, const Digits* dg = nullptr, const std::vector<char>* on_i8 = nullptr);
+    I8Profiles i8_prof_{};  // of outgoing vectors, by canonical wedge
     const Digits* i8_target_ = nullptr;  // set while add_gemm emits the int8 (mixed form: FP16) part of a launch
     bool narrow_ = false;                // set while it emits the products with few columns
     void add_i8(const std::vector<GemmProblem>& P, const long long* xs, const long long* ys, size_t ncols, double2* Y,

@@ -56,9 +56,11 @@ class Mlib3d:
 
 
 class Wave3d:
-    """precision: _lib.PLAIN_FP64 (every pass in FP64), _lib.MIXED (complex
-    FP32 storage, 3xTF32 translations on tcgen05, FP32 near field) or
-    _lib.MIXED_MMA_SYNC (the same with the translations on mma.sync)."""
+    """precision: _lib.PLAIN_FP64 (FP64; large high-frequency products from
+    55-bit digits on the int8 tensor cores, no less accurate), _lib.MIXED
+    (complex FP32 storage, translations as split FP16 or TF32 products on
+    tcgen05, FP32 near field) or _lib.MIXED_MMA_SYNC (complex FP32 with
+    3xTF32 translations on mma.sync)."""
 
     def __init__(self, prefix="wave3d_", device=0, precision=0):
         self.prefix = prefix
