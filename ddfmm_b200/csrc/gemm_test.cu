@@ -2,6 +2,7 @@
 // ddfmm_test_gemm): what a translation of an eval runs, on the caller's matrices.
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -127,12 +128,11 @@ void test_gemm(const double2* A, int m, int k, const double2* X, int ncol, int p
         int* err = P.put(std::vector<int>(1, 0));
         i8_init();
         unsigned char* prof = nullptr;
-        if (path == 6) {  // the columns as one class, in the place of an operator's output
-            prof = P.put(std::vector<unsigned char>(sx));
-            double* rowmax = P.put(std::vector<double>(sx, 0.0));
-            launch_i8_profile(P.put(std::vector<I8ProfileJob>(1, I8ProfileJob{dX, k, ncol, sx, -1, 0})), 1, rowmax,
-                              I8Profiles{prof, sx}, nullptr);
-            launch_i8_profile_scale(rowmax, 1, sx, prof, nullptr);
+        if (path == 6) {  // the columns as one class of vectors
+            std::vector<double> size(k, 0.0);
+            for (size_t e = 0; e < (size_t)k * ncol; ++e)
+                size[e % k] = std::fmax(size[e % k], std::fmax(std::fabs(X[e].x), std::fabs(X[e].y)));
+            prof = P.put(i8_profile(size.data(), k, sx));
         }
         launch_i8_pack(P.put(std::vector<I8PackJob>(1, I8PackJob{dA, B, ra, m, k, m, nkb, i8_tile_rows(m), prof})), 1,
                        i8_row_tiles(m), nullptr);

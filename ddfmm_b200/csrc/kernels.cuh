@@ -295,14 +295,8 @@ struct I8Profiles {
     const unsigned char* prof;
     int stride;
 };
-struct I8ProfileJob {  // an operator that adds into vectors of class `out` from vectors of class `in` (-1: none)
-    const double2* A;
-    int m, k, lda, in, out;
-};
-// largest component of each row of operators, columns weighted by class `in`'s profile
-// (2^prof), into rowmax (classes x stride, from 0); then the profiles of all classes from it
-void launch_i8_profile(const I8ProfileJob* jobs, int n, double* rowmax, const I8Profiles& T, cudaStream_t s);
-void launch_i8_profile_scale(const double* rowmax, int classes, int stride, unsigned char* prof, cudaStream_t s);
+// the row of a class from the typical sizes of its n components, padded with zeros to `stride`
+std::vector<unsigned char> i8_profile(const double* size, int n, int stride);
 void launch_i8_slice(const I8Vec* vecs, int n, const double2* X, char* X8, double* cx, const I8Profiles& T,
                      cudaStream_t s);
 struct alignas(16) I8Tile {  // everything about a tile, so that its next one can be read ahead

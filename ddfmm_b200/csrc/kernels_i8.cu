@@ -14,9 +14,12 @@
 // FP64 twice per output, so the sums over k carry no rounding error at all.
 //
 // 55 bits below the largest component are worth as many of each product only where
-// the components are of one size.  Outgoing vectors' are not: they differ by up to 10^8
-// where the operators' columns differ the other way round.  Both are scaled by powers
-// of two before they become digits (i8_profile_kernel).  Against long-double products, on
+// the components are of one size.  Outgoing vectors' are not: w stands for the
+// equivalent densities E1 w, of one size, and E1 = inv(R1) of a pivoted QR has columns that
+// grow by up to 10^8.  The sizes 1 / max |E1 column j| are a class's profile: component j is scaled
+// by a power of two that evens it out before it becomes digits, column j of an operator by the
+// inverse.  (They are within 0.75-1.25 of the row maxima of the M2M operators into a class, and
+// come with the operator files: no session's geometry shows in them.)  Against long-double products, on
 // the operators and vectors of evals (spheres, ellipsoids and clusters, K = 8 .. 32, both
 // kernels, P = 4, 6, 8, four kinds of densities), the relative 2-norm error is 5e-17 to
 // 7e-16 by pass, the three-MMA FP64 form's 3e-16 to 1.6e-15 and larger in each of them; M2L
@@ -58,8 +61,10 @@
 // sets *err.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cfloat>
 #include <climits>
+#include <cmath>
 #include <cstdint>
 #include <stdexcept>
 
@@ -324,60 +329,22 @@ void launch_i8_slice(const I8Vec* vecs, int n, const double2* X, char* X8, doubl
     if (n > 0) i8_slice_kernel<<<(unsigned)(((size_t)n * 32 + 255) / 256), 256, 0, s>>>(vecs, n, X, X8, cx, T);
 }
 
-// Profiles of classes of vectors (setup only).  An outgoing vector w of a (width, wedge)
-// is the output of the M2M operators into it, whose rows differ by up to 10^8 in size (E2's
-// do), and the operators on w have columns as much smaller where w is large; 55 bits
-// below the largest component, or operator entry, would leave little of the products that
-// count.  Scaled by the rows' largest entries both are flat.  (Maxima: the profile does not
-// depend on the order in which operators add to it.)  A block an operator, a thread a row.
-__global__ void __launch_bounds__(128) i8_profile_kernel(const I8ProfileJob* __restrict__ jobs, int n, double* rowmax,
-                                                         const I8Profiles T) {
-    for (int j = blockIdx.x; j < n; j += gridDim.x) {
-        const I8ProfileJob J = jobs[j];
-        for (int r = threadIdx.x; r < J.m; r += 128) {
-            double top = 0.0;
-            for (int k = 0; k < J.k; ++k) {
-                const double2 a = J.A[(size_t)k * J.lda + r];
-                const double w = J.in >= 0 ? i8_pow2(T.prof[(size_t)J.in * T.stride + k]) : 1.0;
-                top = fmax(top, fmax(fabs(a.x), fabs(a.y)) * w);
-            }
-            // positive numbers are ordered as their bits are
-            atomicMax(reinterpret_cast<unsigned long long*>(rowmax + (size_t)J.out * T.stride + r),
-                      (unsigned long long)__double_as_longlong(top));
-        }
+// e_j - e0, e_j the exponent of size j and e0 the smallest of them but no less than the
+// largest one - 60; sizes that are no positive number count as the smallest.  (Vectors are scaled
+// down only: none overflows.)
+std::vector<unsigned char> i8_profile(const double* size, int n, int stride) {
+    std::vector<unsigned char> row(stride, 0);
+    auto expo = [](double v) { return v > 0.0 && v <= DBL_MAX ? std::ilogb(v) : INT_MIN; };
+    int lo = INT_MAX, hi = INT_MIN;
+    for (int j = 0; j < n; ++j) {
+        const int e = expo(size[j]);
+        if (e == INT_MIN) continue;
+        lo = std::min(lo, e);
+        hi = std::max(hi, e);
     }
-}
-// The profile of a class: e_j - e0, e_j the exponent of row j's largest entry and e0 the
-// smallest of them but no less than the largest one - 60; rows of zeros count as the smallest.
-// (Vectors are scaled down only: none overflows.)  One block a class.
-__global__ void __launch_bounds__(128) i8_profile_scale_kernel(const double* __restrict__ rowmax, int stride,
-                                                               unsigned char* __restrict__ prof) {
-    __shared__ int lo, hi;
-    const double* s = rowmax + (size_t)blockIdx.x * stride;
-    auto expo = [](double v) { return v > 0.0 && v <= DBL_MAX ? ilogb(v) : INT_MIN; };
-    if (threadIdx.x == 0) {
-        lo = INT_MAX;
-        hi = INT_MIN;
-    }
-    __syncthreads();
-    for (int r = threadIdx.x; r < stride; r += 128) {
-        const int e = expo(s[r]);
-        if (e != INT_MIN) {
-            atomicMin(&lo, e);
-            atomicMax(&hi, e);
-        }
-    }
-    __syncthreads();
-    const int e0 = hi == INT_MIN ? 0 : max(lo, hi - 60);
-    for (int r = threadIdx.x; r < stride; r += 128)
-        prof[(size_t)blockIdx.x * stride + r] = (unsigned char)(max(expo(s[r]), e0) - e0);
-}
-
-void launch_i8_profile(const I8ProfileJob* jobs, int n, double* rowmax, const I8Profiles& T, cudaStream_t s) {
-    if (n > 0) i8_profile_kernel<<<n < 65535 ? n : 65535, 128, 0, s>>>(jobs, n, rowmax, T);
-}
-void launch_i8_profile_scale(const double* rowmax, int classes, int stride, unsigned char* prof, cudaStream_t s) {
-    if (classes > 0) i8_profile_scale_kernel<<<classes, 128, 0, s>>>(rowmax, stride, prof);
+    const int e0 = hi == INT_MIN ? 0 : std::max(lo, hi - 60);
+    for (int j = 0; j < n; ++j) row[j] = (unsigned char)(std::max(expo(size[j]), e0) - e0);
+    return row;
 }
 
 // Operator digits (setup only): block (row tile, job).  Row scales first, then

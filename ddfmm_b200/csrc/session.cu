@@ -1618,33 +1618,21 @@ void Session::build() {
         if (!mixed && (lf_i8 || granules)) i8_init();
     }
     phase("digit_buffers");
-    // Profiles of the outgoing vectors (kernels_i8.cu), by width upward: a width's operators
-    // read vectors of the one below.  Incoming vectors are flat as they are.
+    // Profiles of the outgoing vectors (kernels_i8.cu).  Incoming vectors are flat as they are.
     if (!mixed && !up_i8.empty()) {
         int stride = 0;
         for (const Canon& c : hfcanon) stride = std::max(stride, (c.r1 + 15) & ~15);
-        unsigned char* prof = dalloc<unsigned char>(hfcanon.size() * stride);
-        i8_prof_ = I8Profiles{prof, stride};
-        double* rowmax = nullptr;
-        CK(cudaMalloc(&rowmax, sizeof(double) * hfcanon.size() * stride));
-        CK(cudaMemsetAsync(rowmax, 0, sizeof(double) * hfcanon.size() * stride, stream_));
-        for (auto hit = hflevels.rbegin(); hit != hflevels.rend(); ++hit) {
-            std::vector<I8ProfileJob> v;
-            for (int k : cols.m2m.at(hit->first).key) {
-                const DirMats& M = *m2m_of[k / 8];
-                v.push_back(I8ProfileJob{KP(M.fin[k % 8]), M.mrows, M.mcols, M.mrows, M.ccanon, M.canon});
+        std::vector<unsigned char> prof;
+        for (const Canon& c : hfcanon) {
+            std::vector<double> size(c.r1, 0.0);
+            for (int j = 0; j < c.r1; ++j) {
+                for (int i = 0; i < c.r1; ++i) size[j] = std::max(size[j], std::abs(c.op->E1(i, j)));
+                size[j] = 1.0 / size[j];
             }
-            I8ProfileJob* dj = nullptr;
-            CK(cudaMalloc(&dj, sizeof(I8ProfileJob) * std::max<size_t>(v.size(), 1)));
-            CK(cudaMemcpyAsync(dj, v.data(), sizeof(I8ProfileJob) * v.size(), cudaMemcpyHostToDevice, stream_));
-            launch_i8_profile(dj, (int)v.size(), rowmax, i8_prof_, stream_);
-            launch_i8_profile_scale(rowmax, (int)hfcanon.size(), stride, prof, stream_);
-            CK(cudaGetLastError());
-            CK(cudaStreamSynchronize(stream_));
-            CK(cudaFree(dj));
+            const std::vector<unsigned char> row = i8_profile(size.data(), c.r1, stride);
+            prof.insert(prof.end(), row.begin(), row.end());
         }
-        CK(cudaFree(rowmax));
-        phase("digit_profiles");
+        i8_prof_ = I8Profiles{upload(prof), stride};
     }
     auto add_node_digits = [&](const HfNodes& N, int level, const double2* X, const Digits& d, const char* label) {
         const bool profile = !mixed && &N == &up;

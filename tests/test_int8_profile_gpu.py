@@ -1,7 +1,7 @@
 """The int8 path on graded vectors: components that differ by many orders of magnitude and
 meet operator columns as much smaller, as an outgoing vector and the operators on it do.
-With the vectors' profile (powers of two, from the largest entry of each row of what they are
-products of; here of the vectors themselves) both are flat before they are written as digits.
+With the vectors' profile (powers of two, from the sizes of their components; here the largest
+of all vectors) both are flat before they are written as digits.
 
 Tolerance, per output: as in tests/test_gemm_paths_gpu.py for the scaled factors, 2^-51 (k max|A'_row|
 max|x'| + |y|).  A' and x' are formed here with the rows' largest components themselves; a power
