@@ -45,7 +45,7 @@ void test_gemm(const double2* A, int m, int k, const double2* X, int ncol, int p
         xo[c] = (long long)at * sx;
         yo[c] = (long long)at * sy;
         xg[c] = at * (sx / 16);
-        vecs[c] = I8Vec{xo[c], xg[c], (unsigned short)k, (unsigned short)(path == 6)};
+        vecs[c] = I8Vec{xo[c], xg[c], (unsigned short)k, (unsigned short)(path >= 6)};
         for (int i = 0; i < k; ++i) hx[xo[c] + i] = X[(size_t)c * k + i];
         for (int i = 0; i < m; ++i) hy[yo[c] + i] = Y[(size_t)c * m + i];
     }
@@ -53,6 +53,13 @@ void test_gemm(const double2* A, int m, int k, const double2* X, int ncol, int p
     const double2* dX = P.put(hx);
     double2* dY = P.put(hy);
     const long long* dyo = P.put(yo);
+    I8Profiles prof{nullptr, sx};
+    if (path >= 6) {  // the columns as one class of vectors
+        std::vector<double> size(k, 0.0);
+        for (size_t e = 0; e < (size_t)k * ncol; ++e)
+            size[e % k] = std::fmax(size[e % k], std::fmax(std::fabs(X[e].x), std::fabs(X[e].y)));
+        prof.prof = P.put(i8_profile(size.data(), k, sx));
+    }
     if (path == 0) {
         std::vector<GemmTile> tiles;
         for (int r = 0; r < m; r += GEMM_TILE_M)
@@ -73,7 +80,7 @@ void test_gemm(const double2* A, int m, int k, const double2* X, int ncol, int p
         std::vector<double2> one((size_t)m * m, make_double2(0, 0));
         for (int i = 0; i < m; ++i) one[(size_t)i * m + i] = make_double2(1, 0);
         launch_gemm_pair(GemmPair{P.put(one), dA, m, m, ncol, P.put(xo), dX, dY}, nullptr);
-    } else if (path == 3 || path == 4) {  // mixed form, on FP32 copies: 3 FP16 planes, 4 split TF32
+    } else if (path == 3 || path == 4 || path == 7) {  // mixed form, on FP32 copies: 3 FP16 planes, 4 split TF32
         auto narrow = [](const std::vector<double2>& v) {
             std::vector<float2> r;
             for (const double2& a : v) r.push_back(make_float2((float)a.x, (float)a.y));
@@ -84,7 +91,7 @@ void test_gemm(const double2* A, int m, int k, const double2* X, int ncol, int p
         std::vector<float2> fy = narrow(hy);
         float2* fY = P.put(fy);
         int* err = P.put(std::vector<int>(1, 0));
-        if (path == 3) {
+        if (path != 4) {
             float* B = P.put(std::vector<float>(h16_packed_floats(m, k)));
             char* X16 = P.put(std::vector<char>((size_t)ncol * (sx / 16) * H16_GRANULE));
             float* cx = P.put(std::vector<float>((size_t)ncol * (sx / 16)));
@@ -92,9 +99,9 @@ void test_gemm(const double2* A, int m, int k, const double2* X, int ncol, int p
             h16_tiles(B, m, k, 0, ncol, tiles);
             h16_init();
             launch_h16_pack(P.put(std::vector<H16PackJob>(1, H16PackJob{fA, B, const_cast<float*>(h16_scales(B, m, k)), m, k,
-                                                                        m, h16_tile_rows(m)})),
+                                                                        m, h16_tile_rows(m), prof.prof})),
                             1, h16_row_tiles(m), nullptr);
-            launch_h16_slice(nullptr, nullptr, 1, ncol, nullptr, nullptr, HSliceSub{P.put(vecs), fX, X16, cx, ncol, 0});
+            launch_h16_slice(nullptr, nullptr, 1, ncol, nullptr, nullptr, HSliceSub{P.put(vecs), fX, X16, cx, ncol, 0, prof});
             launch_h16_gemm(nullptr, nullptr, 1, (int)tiles.size(), nullptr, err, nullptr,
                             HSub{P.put(tiles), P.put(xg), dyo, X16, cx, fY, (int)tiles.size(), 0});
         } else {
@@ -127,16 +134,9 @@ void test_gemm(const double2* A, int m, int k, const double2* X, int ncol, int p
         i8_tiles(B, ra, m, k, 0, ncol, tiles);
         int* err = P.put(std::vector<int>(1, 0));
         i8_init();
-        unsigned char* prof = nullptr;
-        if (path == 6) {  // the columns as one class of vectors
-            std::vector<double> size(k, 0.0);
-            for (size_t e = 0; e < (size_t)k * ncol; ++e)
-                size[e % k] = std::fmax(size[e % k], std::fmax(std::fabs(X[e].x), std::fabs(X[e].y)));
-            prof = P.put(i8_profile(size.data(), k, sx));
-        }
-        launch_i8_pack(P.put(std::vector<I8PackJob>(1, I8PackJob{dA, B, ra, m, k, m, nkb, i8_tile_rows(m), prof})), 1,
+        launch_i8_pack(P.put(std::vector<I8PackJob>(1, I8PackJob{dA, B, ra, m, k, m, nkb, i8_tile_rows(m), prof.prof})), 1,
                        i8_row_tiles(m), nullptr);
-        launch_i8_slice(P.put(vecs), ncol, dX, X8, cx, I8Profiles{prof, sx}, nullptr);
+        launch_i8_slice(P.put(vecs), ncol, dX, X8, cx, prof, nullptr);
         launch_i8_gemm(I8Sub{P.put(tiles), P.put(xg), dyo, X8, cx, dY, (int)tiles.size()}, err, nullptr);
         int h = 0;
         ck(cudaMemcpy(&h, err, sizeof(int), cudaMemcpyDeviceToHost));

@@ -17,7 +17,7 @@ struct GemmProblem {
     int col0;  // first entry in the column arrays
     int ncol;
     const float* packed;  // tcgen05 form: an already packed copy of A (A may then be null)
-    int profile;          // int8 path: 1 + the row of the profile table that scales its columns' vectors; 0: none
+    int profile;          // int8 and FP16 paths: 1 + the row of the profile table that scales its columns' vectors; 0: none
 };
 // A launch is a list of output tiles of up to GEMM_TILE_M rows x GEMM_TILE_N columns.
 constexpr int GEMM_TILE_M = 64, GEMM_TILE_N = 64;
@@ -282,20 +282,20 @@ void launch_umma_cgemm(const UmmaSub* subs, const int* prefix, int nsub, int nti
 constexpr int I8_DIGITS = 7;
 constexpr int I8_TILE_ROWS = 56;
 constexpr int I8_GRANULE = 16 * 2 * I8_DIGITS;  // bytes of the digits of 16 complex numbers
-struct I8Vec {      // a vector to write as digits
+struct alignas(16) I8Vec {  // a vector to write as digits
     long long src;  // its first element in X
     int gran;       // its first granule (and its entry of cx)
     unsigned short len;      // complex numbers
-    unsigned short profile;  // as in GemmProblem
+    unsigned short profile;  // as in GemmProblem; a launch's vectors all have one or none has
 };
-// Profile table: a row of `stride` exponents, 0 .. 60, for each class of vectors.  Component j of
-// a vector of row p is scaled by 2^-prof[p * stride + j] before it is written as digits, column
-// j of an operator on it by the inverse (kernels_i8.cu).
+// Profile table: a row of `stride` biased exponents b = 67 .. 127 (as FP32 has them) for each class
+// of vectors.  Component j of a vector of row p is scaled by 2^(b - 127), b = prof[p * stride + j],
+// before it is written as digits, column j of an operator on it by the inverse (kernels_i8.cu).
 struct I8Profiles {
     const unsigned char* prof;
     int stride;
 };
-// the row of a class from the typical sizes of its n components, padded with zeros to `stride`
+// the row of a class from the typical sizes of its n components, padded with 127 to `stride`
 std::vector<unsigned char> i8_profile(const double* size, int n, int stride);
 void launch_i8_slice(const I8Vec* vecs, int n, const double2* X, char* X8, double* cx, const I8Profiles& T,
                      cudaStream_t s);
@@ -345,6 +345,7 @@ struct HSliceSub {  // one instance's vectors to write as planes
     float* cx;  // output scale of the vector that starts at a granule
     int n;
     int inst;
+    I8Profiles prof;  // prof.prof null: no vector has a profile, in any sub-launch of the launch
 };
 struct alignas(16) H16Tile {  // everything about a tile, so that its next one can be read ahead
     const float* B;           // the row tile's packed operator (h16_pack_kernel)
@@ -367,6 +368,7 @@ struct H16PackJob {
     float* dst;
     float* ra;
     int m, k, lda, rows_t;
+    const unsigned char* prof;  // of its columns, or null
 };
 void h16_init();
 int h16_row_tiles(int m);

@@ -5,7 +5,10 @@
 // two to a largest component in [2^13, 2^14) and written as two FP16 planes,
 // hi = FP16(x), lo = FP16(x - hi): 22 bits of every component that is not more
 // than 2^17 below the largest, and an absolute 2^-39 of the largest below that.
-// A product is hi hi + lo hi + hi lo in FP32, like the three TF32 products of
+// Outgoing vectors' components differ by more at P = 8: they and the operators on them
+// are evened out by the vectors' profiles first, as in kernels_i8.cu (on a K = 8 cluster at
+// P = 8 M2L products are 1.1e-6 off with them, 1.7e-5 without, split TF32 2.2e-6; elsewhere
+// 0.4-2.4e-6 by pass on evals' own vectors, split TF32 0.8-4.5e-6).  A product is hi hi + lo hi + hi lo in FP32, like the three TF32 products of
 // umma_cgemm_kernel with rounded instead of truncated halves, at twice their
 // rate and half their operand bytes.  On random products of 16 to 400 terms the
 // result is 0.2-2.9e-6 from a long-double one in relative 2-norm, that kernel's
@@ -78,27 +81,35 @@ __device__ __forceinline__ void h16_mma(uint32_t d, uint64_t a, uint64_t b, uint
         : "memory");
 }
 
-// Scale of a vector whose largest |x| has the bits `top`: x up s in [2^13, 2^14) for
-// that component (two powers of two, so subnormal vectors keep their bits) and
-// out = 2^(e - 14) with 2^e above it; NaN for a vector holding an infinity or a NaN.
+// Scale of a vector whose largest |x| has the bits `top`: x s in [2^13, 2^14) for that
+// component; NaN for a vector holding an infinity or a NaN.  A vector with nothing above
+// 2^-63 is brought up by 2^100 first (low), so subnormals keep their bits.  With |x| < 2^e
+// (before that) an output is the sum of planes' products times 2^(e - 14) for the vector and
+// for the operator row: stored as 2^(e - 1) (h16_out, exact for every FP32 vector) and 2^(e - 27).
+constexpr int H_UP = 100;
+constexpr uint32_t H_LOW = 64u << 23;  // top below it: low
 struct H16Scale {
-    float up, s, out;
+    float s;
+    int b;  // e + 126
 };
-__device__ __forceinline__ H16Scale h16_scale(uint32_t top) {
+__device__ __forceinline__ float h16_pow2(int e) {  // 2^e; 0 below 2^-149
+    return e >= -126 ? __uint_as_float((uint32_t)(127 + e) << 23) : e >= -149 ? __uint_as_float(1u << (e + 149)) : 0.f;
+}
+__device__ __forceinline__ H16Scale h16_scale(uint32_t top, bool low) {
     H16Scale r;
     const int be = (int)(top >> 23);
     if (be == 255) {
-        r.up = r.s = 0.f;
-        r.out = __uint_as_float(0x7fc00000u);
+        r.s = 0.f;
+        r.b = 255;
         return r;
     }
-    const int b1 = be < 1 ? 1 : be;  // |x| < 2^(b1 - 126)
-    const bool low = b1 < 40;
-    r.up = low ? __uint_as_float((127 + 60) << 23) : 1.f;
-    r.s = __uint_as_float((uint32_t)(267 - b1 - (low ? 60 : 0)) << 23);  // 2^(140 - b1 [- 60])
-    // 2^(b1 - 140) = 2^(e - 14): below 2^-126 as a subnormal power of two
-    r.out = b1 >= 14 ? __uint_as_float((uint32_t)(b1 - 13) << 23) : __uint_as_float(1u << (b1 + 9));
+    const int b1 = top == 0 ? 127 : be < 13 ? 13 : be;  // boosted by 2^100 it is 18 or more
+    r.s = h16_pow2(140 - b1);
+    r.b = b1 - (low ? H_UP : 0);
     return r;
+}
+__device__ __forceinline__ float h16_out(const H16Scale& S, int by) {  // 2^(e - by)
+    return S.b == 255 ? __uint_as_float(0x7fc00000u) : h16_pow2(S.b - 126 - by);
 }
 // two values: hi and lo halves of each
 __device__ __forceinline__ void h16_split(float x, float y, uint32_t& hi, uint32_t& lo) {
@@ -127,50 +138,103 @@ __device__ __forceinline__ int sub_of(const T* prefix, int nsub, T i) {
 // ---------------------------------------------------------------- planes
 // One warp per vector, four lanes per granule (4 complex numbers each: 16 bytes
 // of hi, 16 of lo); a vector of up to 128 numbers is read once and kept in registers.
-// Bound by HBM: 8 bytes read and 8 written per complex number; 4.0 TB/s on 2.3
+// Bound by HBM: 8 bytes read and 8 written per complex number; 4.3-4.4 TB/s on 2.5
 // million vectors of 100 (16-byte loads: the same; two vectors a warp: 2% faster
 // there, a tenth slower where vectors do not fill the SMs).
-__global__ void __launch_bounds__(256) h16_slice_kernel(const HSliceSub one, const HSliceSub* __restrict__ subs,
-                                                        const int* __restrict__ prefix, int nsub, int n,
-                                                        const int* __restrict__ active) {
-    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (w >= n) return;
-    const int j = nsub > 1 ? sub_of(prefix, nsub, w) : 0;
-    const HSliceSub S = nsub > 1 ? subs[j] : one;
-    if (active && !active[S.inst]) return;
-    const I8Vec V = S.vecs[nsub > 1 ? w - prefix[j] : w];
-    const float2* x = S.X + V.src;
+// A vector's planes by one warp; UP: components brought up by 2^UP first.  False, and nothing
+// written, where the vector is low and was not brought up.
+template <bool PROF, int UP>
+__device__ __forceinline__ bool h16_slice_vector(const float2* x, const unsigned char* prof, float* cx, char* out, int len,
+                                                 int lane) {
     float2 v[4];
     auto load = [&](int j0) {
+        uint32_t b = 0x7f7f7f7fu;
+        if (PROF && j0 < len) b = __ldg(reinterpret_cast<const uint32_t*>(prof + j0));
 #pragma unroll
-        for (int i = 0; i < 4; ++i) v[i] = j0 + i < V.len ? x[j0 + i] : make_float2(0.f, 0.f);
+        for (int i = 0; i < 4; ++i) v[i] = j0 + i < len ? x[j0 + i] : make_float2(0.f, 0.f);
+        if (PROF || UP) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float f = __uint_as_float((((b >> (8 * i)) & 255u) + UP) << 23);
+                v[i] = make_float2(v[i].x * f, v[i].y * f);
+            }
+        }
     };
     uint32_t top = 0;
-    for (int j0 = 0; j0 < V.len; j0 += 128) {
+    for (int j0 = 0; j0 < len; j0 += 128) {
         load(j0 + lane * 4);
 #pragma unroll
         for (int i = 0; i < 4; ++i) top = max(top, max(abs_bits(v[i].x), abs_bits(v[i].y)));
     }
-    const H16Scale C = h16_scale(__reduce_max_sync(0xffffffffu, top));
-    if (lane == 0) S.cx[V.gran] = C.out;
-    for (int j0 = 0; j0 < V.len; j0 += 128) {
-        if (V.len > 128) load(j0 + lane * 4);
+    top = __reduce_max_sync(0xffffffffu, top);
+    if (!UP && top < H_LOW) return false;
+    const H16Scale C = h16_scale(top, UP > 0);
+    if (lane == 0) *cx = h16_out(C, 1);
+    for (int j0 = 0; j0 < len; j0 += 128) {
+        if (len > 128) load(j0 + lane * 4);
         const int g = (j0 >> 4) + (lane >> 2);
-        if (g * 16 < V.len) {
+        if (g * 16 < len) {
             uint32_t hi[4], lo[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) h16_split(v[i].x * C.up * C.s, v[i].y * C.up * C.s, hi[i], lo[i]);
-            char* o = S.X16 + (size_t)(V.gran + g) * H16_GRANULE + (lane & 3) * 16;
+            for (int i = 0; i < 4; ++i) h16_split(v[i].x * C.s, v[i].y * C.s, hi[i], lo[i]);
+            char* o = out + g * H16_GRANULE + (lane & 3) * 16;
             *reinterpret_cast<uint4*>(o) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
             *reinterpret_cast<uint4*>(o + 64) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
         }
     }
+    return true;
+}
+// rare: out of the kernel's way, which runs six blocks an SM at 40 registers (the outgoing
+// vectors of a K = 64 sphere 0.84 ms; five blocks 1.00)
+template <bool PROF>
+__device__ __noinline__ void h16_slice_low(const float2* x, const unsigned char* prof, float* cx, char* out, int len,
+                                           int lane) {
+    h16_slice_vector<PROF, H_UP>(x, prof, cx, out, len, lane);
+}
+struct HSliceRef {  // vector w of a launch
+    const float2* x;
+    const unsigned char* prof;
+    float* cx;
+    char* out;
+    int len;
+};
+template <bool PROF>
+__device__ __forceinline__ HSliceRef h16_slice_ref(const HSliceSub& S, int i) {
+    const I8Vec V = S.vecs[i];
+    return HSliceRef{S.X + V.src, PROF ? S.prof.prof + (size_t)(V.profile - 1) * S.prof.stride : nullptr, S.cx + V.gran,
+                     S.X16 + (size_t)V.gran * H16_GRANULE, V.len};
+}
+template <bool PROF>  // finds the vector again: nothing of it has to be kept for this
+__device__ __noinline__ void h16_slice_low_multi(const HSliceSub* subs, const int* prefix, int nsub, int w) {
+    const int j = sub_of(prefix, nsub, w);
+    const HSliceRef R = h16_slice_ref<PROF>(subs[j], w - prefix[j]);
+    h16_slice_vector<PROF, H_UP>(R.x, R.prof, R.cx, R.out, R.len, threadIdx.x & 31);
+}
+
+// PROF: the vectors have profiles (a launch's all do or none does).
+template <bool MULTI, bool PROF>
+__global__ void __launch_bounds__(256, 6) h16_slice_kernel(const HSliceSub one, const HSliceSub* __restrict__ subs,
+                                                           const int* __restrict__ prefix, int nsub, int n,
+                                                           const int* __restrict__ active) {
+    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (w >= n) return;
+    const int j = MULTI ? sub_of(prefix, nsub, w) : 0;
+    const HSliceSub& S = MULTI ? subs[j] : one;
+    if (active && !active[S.inst]) return;
+    const HSliceRef R = h16_slice_ref<PROF>(S, MULTI ? w - prefix[j] : w);
+    if (h16_slice_vector<PROF, 0>(R.x, R.prof, R.cx, R.out, R.len, lane)) return;
+    if (MULTI)
+        h16_slice_low_multi<PROF>(subs, prefix, nsub, (blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    else
+        h16_slice_low<PROF>(R.x, R.prof, R.cx, R.out, R.len, lane);
 }
 
 void launch_h16_slice(const HSliceSub* subs, const int* prefix, int nsub, int n, const int* active, cudaStream_t s,
                       const HSliceSub& one) {
-    if (n > 0)
-        h16_slice_kernel<<<(unsigned)((n + 7) / 8), 256, 0, s>>>(one, subs, prefix, nsub, n, active);
+    if (n <= 0) return;
+    auto kernel = nsub == 1 ? (one.prof.prof ? h16_slice_kernel<false, true> : h16_slice_kernel<false, false>)
+                            : (one.prof.prof ? h16_slice_kernel<true, true> : h16_slice_kernel<true, false>);
+    kernel<<<(unsigned)((n + 7) / 8), 256, 0, s>>>(one, subs, prefix, nsub, n, active);
 }
 
 int h16_tile_rows(int m) {
@@ -190,27 +254,36 @@ const float* h16_scales(const float* packed, int m, int k) {
 __global__ void __launch_bounds__(256) h16_pack_kernel(const H16PackJob* __restrict__ jobs, int njobs) {
     __shared__ uint32_t tops[2][128];
     __shared__ H16Scale sc[128];
+    __shared__ bool low[128];
     const int tid = threadIdx.x;
     for (int j = blockIdx.y; j < njobs; j += gridDim.y) {
         const H16PackJob J = jobs[j];
         const int row0 = blockIdx.x * J.rows_t;
         if (row0 >= J.m) continue;  // uniform over the block
-        __syncthreads();
-        {
+        // column k as the vectors' profile leaves it, brought up where the row is low
+        auto entry = [&](int r, int k, bool up) {
+            const float2 a = J.A[(size_t)k * J.lda + row0 + r];
+            const float f = h16_pow2(J.prof ? 127 - J.prof[k] : 0), g = h16_pow2(up ? H_UP : 0);
+            return make_float2(a.x * f * g, a.y * f * g);
+        };
+        for (int up = 0; up < 2; ++up) {
+            __syncthreads();
             const int r = tid & 127;
             uint32_t top = 0;
-            if (r < J.rows_t && row0 + r < J.m)
+            if (r < J.rows_t && row0 + r < J.m && (up == 0 || low[r]))
                 for (int k = tid >> 7; k < J.k; k += 2) {
-                    const float2 a = J.A[(size_t)k * J.lda + row0 + r];
+                    const float2 a = entry(r, k, up);
                     top = max(top, max(abs_bits(a.x), abs_bits(a.y)));
                 }
             tops[tid >> 7][r] = top;
+            __syncthreads();
+            if (tid < J.rows_t) {
+                const uint32_t t = max(tops[0][tid], tops[1][tid]);
+                if (up == 0) low[tid] = t < H_LOW;
+                if (up == 0 || low[tid]) sc[tid] = h16_scale(t, up);
+            }
         }
-        __syncthreads();
-        if (tid < J.rows_t) {
-            sc[tid] = h16_scale(max(tops[0][tid], tops[1][tid]));
-            if (row0 + tid < J.m) J.ra[row0 + tid] = sc[tid].out;
-        }
+        if (tid < J.rows_t && row0 + tid < J.m) J.ra[row0 + tid] = h16_out(sc[tid], 27);
         __syncthreads();
         const int nkb = (J.k + 15) / 16, nq = nkb * 4, N = 2 * J.rows_t;
         char* dst = reinterpret_cast<char*>(J.dst) + (size_t)blockIdx.x * nkb * 2 * N * 64;
@@ -221,8 +294,8 @@ __global__ void __launch_bounds__(256) h16_pack_kernel(const H16PackJob* __restr
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const bool ok = row0 + r < J.m && k0 + i < J.k;
-                const float2 a = ok ? J.A[(size_t)(k0 + i) * J.lda + row0 + r] : make_float2(0.f, 0.f);
-                const float re = a.x * C.up * C.s, im = a.y * C.up * C.s;
+                const float2 a = ok ? entry(r, k0 + i, low[r]) : make_float2(0.f, 0.f);
+                const float re = a.x * C.s, im = a.y * C.s;
                 h16_split(re, -im, h0[i], l0[i]);
                 h16_split(im, re, h1[i], l1[i]);
             }

@@ -275,6 +275,8 @@ __device__ __forceinline__ uint2 gather_bytes(const unsigned long long (&w)[8], 
 // Digits of vectors: one warp per vector, four lanes per granule of 16 complex
 // numbers (each lane 4 of them: 8 bytes in each of the 7 planes).  Bound by
 // HBM: 16 bytes read and 14 written per complex number; the profiles come from L2.
+// PROF: the vectors have profiles (a launch's all do or none does).
+template <bool PROF>
 __global__ void __launch_bounds__(256) i8_slice_kernel(const I8Vec* __restrict__ vecs, int n,
                                                        const double2* __restrict__ X, char* __restrict__ X8,
                                                        double* __restrict__ cx, const I8Profiles T) {
@@ -282,29 +284,34 @@ __global__ void __launch_bounds__(256) i8_slice_kernel(const I8Vec* __restrict__
     if (w >= n) return;
     const I8Vec V = vecs[w];
     const double2* x = X + V.src;
-    const unsigned char* prof = V.profile ? T.prof + (size_t)(V.profile - 1) * T.stride : nullptr;
+    const unsigned char* prof = PROF ? T.prof + (size_t)(V.profile - 1) * T.stride : nullptr;
     double2 v[4];
     auto load = [&](int j0, int up) {
-        const uint32_t e = prof && j0 < V.len ? __ldg(reinterpret_cast<const uint32_t*>(prof + j0)) : 0u;
+        uint32_t b = 0x7f7f7f7fu;
+        if (PROF && j0 < V.len) b = __ldg(reinterpret_cast<const uint32_t*>(prof + j0));
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const double2 a = j0 + j < V.len ? x[j0 + j] : make_double2(0.0, 0.0);
-            const double f = i8_pow2(up - (int)((e >> (8 * j)) & 255u));
-            v[j] = make_double2(a.x * f, a.y * f);
+        for (int j = 0; j < 4; ++j) v[j] = j0 + j < V.len ? x[j0 + j] : make_double2(0.0, 0.0);
+        if (PROF || up) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const double f = __hiloint2double((int)(((b >> (8 * j)) & 255u) + (uint32_t)(896 + up)) << 20, 0);
+                v[j] = make_double2(v[j].x * f, v[j].y * f);
+            }
         }
     };
-    auto top_at = [&](int up) {  // of the whole vector
-        uint32_t top = 0;
+    int up = 0;
+    uint32_t top;  // of the whole vector
+    while (true) {
+        top = 0;
         for (int j0 = 0; j0 < V.len; j0 += 128) {
             load(j0 + lane * 4, up);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) top = max(top, top_of(v[j]));
+            for (int i = 0; i < 4; ++i) top = max(top, top_of(v[i]));
         }
-        return __reduce_max_sync(0xffffffffu, top);
-    };
-    int up = 0;
-    uint32_t top = top_at(up);
-    if (top < I_LOW) top = top_at(up = I_UP);
+        top = __reduce_max_sync(0xffffffffu, top);
+        if (top >= I_LOW || up) break;
+        up = I_UP;
+    }
     const I8Scale S = i8_scale(top, up > 0);
     if (lane == 0) cx[V.gran] = S.out;
     for (int j0 = 0; j0 < V.len; j0 += 128) {
@@ -326,14 +333,16 @@ __global__ void __launch_bounds__(256) i8_slice_kernel(const I8Vec* __restrict__
 
 void launch_i8_slice(const I8Vec* vecs, int n, const double2* X, char* X8, double* cx, const I8Profiles& T,
                      cudaStream_t s) {
-    if (n > 0) i8_slice_kernel<<<(unsigned)(((size_t)n * 32 + 255) / 256), 256, 0, s>>>(vecs, n, X, X8, cx, T);
+    if (n <= 0) return;
+    auto kernel = T.prof ? i8_slice_kernel<true> : i8_slice_kernel<false>;
+    kernel<<<(unsigned)(((size_t)n * 32 + 255) / 256), 256, 0, s>>>(vecs, n, X, X8, cx, T);
 }
 
-// e_j - e0, e_j the exponent of size j and e0 the smallest of them but no less than the
-// largest one - 60; sizes that are no positive number count as the smallest.  (Vectors are scaled
+// 127 - (e_j - e0), e_j the exponent of size j and e0 the smallest of them but no less than
+// the largest one - 60; sizes that are no positive number count as the smallest.  (Vectors are scaled
 // down only: none overflows.)
 std::vector<unsigned char> i8_profile(const double* size, int n, int stride) {
-    std::vector<unsigned char> row(stride, 0);
+    std::vector<unsigned char> row(stride, 127);
     auto expo = [](double v) { return v > 0.0 && v <= DBL_MAX ? std::ilogb(v) : INT_MIN; };
     int lo = INT_MAX, hi = INT_MIN;
     for (int j = 0; j < n; ++j) {
@@ -343,7 +352,7 @@ std::vector<unsigned char> i8_profile(const double* size, int n, int stride) {
         hi = std::max(hi, e);
     }
     const int e0 = hi == INT_MIN ? 0 : std::max(lo, hi - 60);
-    for (int j = 0; j < n; ++j) row[j] = (unsigned char)(std::max(expo(size[j]), e0) - e0);
+    for (int j = 0; j < n; ++j) row[j] = (unsigned char)(127 - (std::max(expo(size[j]), e0) - e0));
     return row;
 }
 
@@ -362,7 +371,7 @@ __global__ void __launch_bounds__(256) i8_pack_kernel(const I8PackJob* __restric
         // column k as the vectors' profile leaves it, brought up where the row is low
         auto entry = [&](int r, int k, bool up) {
             const double2 a = J.A[(size_t)k * J.lda + row0 + r];
-            const double f = i8_pow2((J.prof ? J.prof[k] : 0) + (up ? I_UP : 0));
+            const double f = i8_pow2((J.prof ? 127 - J.prof[k] : 0) + (up ? I_UP : 0));
             return make_double2(a.x * f, a.y * f);
         };
         for (int up = 0; up < 2; ++up) {

@@ -388,7 +388,7 @@ const float* Session::packed_operator(const GemmProblem& q, bool h16) {
     if (k != opkey_.end()) to_publish_.push_back(std::make_pair(opctx_ + "|" + k->second, op));
     if (h16)
         h16_jobs_.push_back(H16PackJob{(const float2*)q.A, d, const_cast<float*>(h16_scales(d, q.m, q.k)), q.m, q.k, q.lda,
-                                       h16_tile_rows(q.m)});
+                                       h16_tile_rows(q.m), profile_of(q)});
     else
         pack_jobs_.push_back(UmmaPackJob{(const float2*)q.A, d, umma_tile_stride(q.k), q.m, q.k, q.lda, umma_nkb(q.k)});
     return packed_[key] = d;
@@ -467,8 +467,7 @@ void Session::add_i8(const std::vector<GemmProblem>& P, const long long* xs, con
     double* ra = dalloc<double>(rows);
     for (size_t i = 0; i < P.size(); ++i) {
         const GemmProblem& q = P[i];
-        const unsigned char* prof = q.profile ? i8_prof_.prof + (size_t)(q.profile - 1) * i8_prof_.stride : nullptr;
-        jobs.push_back(I8PackJob{q.A, B, ra, q.m, q.k, q.lda, (q.k + 15) / 16, i8_tile_rows(q.m), prof});
+        jobs.push_back(I8PackJob{q.A, B, ra, q.m, q.k, q.lda, (q.k + 15) / 16, i8_tile_rows(q.m), profile_of(q)});
         i8_tiles(B, ra, q.m, q.k, q.col0, q.ncol, tiles);
         B += i8_packed_bytes(q.m, q.k);
         ra += q.m;
@@ -502,9 +501,10 @@ void Session::add_digits(const I8Vec* vecs, size_t n, const double2* X, const Di
     st.kind = 7;
     st.label = label;
     for (size_t i = 0; i < n; ++i) st.bytes += (umma() ? 16.0 : 30.0) * vecs[i].len;
+    const I8Profiles prof = n && vecs[0].profile ? profiles_ : I8Profiles{};
     if (umma()) {
         st.kind = 9;
-        st.hs = HSliceSub{upload_n(vecs, n), reinterpret_cast<const float2*>(X), dg.X8, (float*)dg.cx, (int)n, 0};
+        st.hs = HSliceSub{upload_n(vecs, n), reinterpret_cast<const float2*>(X), dg.X8, (float*)dg.cx, (int)n, 0, prof};
         set_multi(st, st.hs, st.hs.n);
         push_step(st);
         return;
@@ -514,6 +514,7 @@ void Session::add_digits(const I8Vec* vecs, size_t n, const double2* X, const Di
     st.dg.X = X;
     st.dg.X8 = dg.X8;
     st.dg.cx = (double*)dg.cx;
+    st.dg.prof = prof;
     push_step(st);
 }
 
@@ -1324,10 +1325,11 @@ void Session::build() {
     std::map<int, std::vector<char> > m2m_i8, m2l_i8, l2l_i8;  // level -> problems on the int8 path
     std::set<int> up_i8, dn_i8;  // levels whose outgoing / incoming vectors are written as digits
     bool lf_i8 = false;
+    const bool profiled = hfcanon.size() < 65535;  // I8Vec::profile has 16 bits
     if (!mixed || umma()) {
         auto choose = [&](const std::vector<std::array<int, 3> >& shapes) {
             if (umma()) return std::vector<char>(shapes.size(), 1);
-            if (hfcanon.size() >= 65535) return std::vector<char>();  // I8Vec::profile has 16 bits
+            if (!profiled) return std::vector<char>();
             if (prm_.int8_rule == INT8_BY_SIZE) return i8_choose(shapes);
             std::vector<char> on(prm_.int8_rule == INT8_ALTERNATE ? shapes.size() : 0);
             for (size_t i = 0; i < on.size(); i += 2) on[i] = 1;
@@ -1619,7 +1621,7 @@ void Session::build() {
     }
     phase("digit_buffers");
     // Profiles of the outgoing vectors (kernels_i8.cu).  Incoming vectors are flat as they are.
-    if (!mixed && !up_i8.empty()) {
+    if (profiled && !up_i8.empty()) {
         int stride = 0;
         for (const Canon& c : hfcanon) stride = std::max(stride, (c.r1 + 15) & ~15);
         std::vector<unsigned char> prof;
@@ -1632,10 +1634,10 @@ void Session::build() {
             const std::vector<unsigned char> row = i8_profile(size.data(), c.r1, stride);
             prof.insert(prof.end(), row.begin(), row.end());
         }
-        i8_prof_ = I8Profiles{upload(prof), stride};
+        profiles_ = I8Profiles{upload(prof), stride};
     }
     auto add_node_digits = [&](const HfNodes& N, int level, const double2* X, const Digits& d, const char* label) {
-        const bool profile = !mixed && &N == &up;
+        const bool profile = profiled && &N == &up;
         const auto r = N.range.at(level);
         const size_t n = (size_t)(r.second - r.first);
         std::unique_ptr<I8Vec[]> v(new I8Vec[n]);  // not zeroed first
@@ -1674,7 +1676,7 @@ void Session::build() {
                 if (M.cached) {
                     probs.push_back(GemmProblem{nullptr, M.mrows, M.mcols, M.mrows, 0, 0, M.pk[ind]});
                 } else {
-                    probs.push_back(GemmProblem{KP(M.fin[ind]), M.mrows, M.mcols, M.mrows, 0, 0, nullptr, M.ccanon + 1});
+                    probs.push_back(GemmProblem{KP(M.fin[ind]), M.mrows, M.mcols, M.mrows, 0, 0, nullptr, profiled ? M.ccanon + 1 : 0});
                     if (!opctx_.empty()) opkey_[KP(M.fin[ind])] = opk("m2m", W, dir, ind);
                 }
             }
@@ -1701,7 +1703,7 @@ void Session::build() {
                 if (M.pk) {
                     probs.push_back(GemmProblem{nullptr, M.r1, M.r1, M.r1, 0, 0, M.pk});
                 } else {
-                    probs.push_back(GemmProblem{KP(M.fin), M.r1, M.r1, M.r1, 0, 0, nullptr, M.canon + 1});
+                    probs.push_back(GemmProblem{KP(M.fin), M.r1, M.r1, M.r1, 0, 0, nullptr, profiled ? M.canon + 1 : 0});
                     if (!opctx_.empty()) opkey_[KP(M.fin)] = M.key;
                 }
             }
@@ -2047,7 +2049,7 @@ void Session::launch_step(const Step& st, cudaStream_t s, double2* spec) {
             else
                 launch_vlist_inverse(st.v.L, st.v.trg, st.v.ntrg, st.v.tsp, st.v.dnchk, s);
             break;
-        case 7: launch_i8_slice(st.dg.vecs, st.dg.n, st.dg.X, st.dg.X8, st.dg.cx, i8_prof_, s); break;
+        case 7: launch_i8_slice(st.dg.vecs, st.dg.n, st.dg.X, st.dg.X8, st.dg.cx, st.dg.prof, s); break;
         case 8: launch_i8_gemm(st.i8, d_err_, s, stall_ns, stall_ns > 0); break;
         case 11: launch_gemm_pair(st.gp, s); break;
         case 9:

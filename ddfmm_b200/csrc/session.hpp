@@ -133,6 +133,7 @@ private:
         const double2* X = nullptr;
         char* X8 = nullptr;
         double* cx = nullptr;
+        I8Profiles prof{};
     };
     // The digits (plain form) or FP16 planes (mixed form) of a GEMM launch's input
     // array: element offset o of a vector is granule (o - base) / unit * gran of X8.
@@ -201,7 +202,10 @@ private:
     void add_gemm(std::vector<GemmProblem>& probs, std::vector<std::vector<long long> >& xo,
                   std::vector<std::vector<long long> >& yo, const double2* X, double2* Y, int mode,
                   const char* label, const Digits* dg = nullptr, const std::vector<char>* on_i8 = nullptr);
-    I8Profiles i8_prof_{};  // of outgoing vectors, by canonical wedge
+    I8Profiles profiles_{};  // of outgoing vectors, by canonical wedge
+    const unsigned char* profile_of(const GemmProblem& q) const {
+        return q.profile ? profiles_.prof + (size_t)(q.profile - 1) * profiles_.stride : nullptr;
+    }
     const Digits* i8_target_ = nullptr;  // set while add_gemm emits the int8 (mixed form: FP16) part of a launch
     bool narrow_ = false;                // set while it emits the products with few columns
     void add_i8(const std::vector<GemmProblem>& P, const long long* xs, const long long* ys, size_t ncols, double2* Y,

@@ -47,7 +47,8 @@ enum { DDFMM_KERNEL_HELM = 0, DDFMM_KERNEL_EXPR = 1 }; /* include/kernel3d.hpp:2
  * applied in complex FP32 -- on the tensor cores (tcgen05, accumulators in
  * tensor memory, FP32 accumulation), high-frequency translations as three FP16
  * products of two planes a number (22 bits, of components within 2^17 of the
- * largest of their vector or operator row) and low-frequency ones as 3xTF32;
+ * largest of their vector or operator row after that scaling) and low-frequency
+ * ones as 3xTF32;
  * the near field in FP32 on FP64 coordinate differences.  Error
  * vs the FP64 direct sum is then set by FP32 rounding (about 1e-6) on top of
  * the method's own (1e-4 / 1e-6 / 1e-8).  MIXED_MMA_SYNC: the same form with
@@ -191,8 +192,8 @@ int ddfmm_session_test_create(const double* pos3n, int n, int kernel, int accu, 
  * 1: the int8 tensor path (exact integer products of digit planes), 2: the FP64
  * tensor path for few columns (PLAIN_FP64 form); 3: the FP16 tensor path (two
  * planes per number), 4: split TF32 (MIXED form, on FP32 copies); 5: the kernel
- * of two products in a row, the identity and A (m = k <= 64; Y = A X); 6: the
- * int8 path, its columns' profile taken from the rows of X.  Columns
+ * of two products in a row, the identity and A (m = k <= 64; Y = A X); 6, 7:
+ * paths 1 and 3 with the columns' profile taken from the rows of X.  Columns
  * are gathered and scattered as an eval's are. */
 int ddfmm_test_gemm(const double* A, int m, int k, const double* X, int ncol, int path, double* Y);
 
