@@ -321,7 +321,7 @@ int ddfmm_session_test_gemm_stall_in(ddfmm_session* s, double wait_s, int kernel
 }
 
 int ddfmm_test_gemm(const double* A, int m, int k, const double* X, int ncol, int path, double* Y) {
-    if (!A || !X || !Y || m < 1 || m > 400 || k < 1 || k > 400 || ncol < 1 || ncol > (1 << 20) || path < 0 || path > 7)
+    if (!A || !X || !Y || m < 1 || m > 400 || k < 1 || k > 400 || ncol < 1 || ncol > (1 << 20) || path < 0 || path > 8)
         return fail(DDFMM_EINVAL, "bad GEMM test arguments");
     return guarded([&] {
         ddfmm::test_gemm(reinterpret_cast<const double2*>(A), m, k, reinterpret_cast<const double2*>(X), ncol, path,

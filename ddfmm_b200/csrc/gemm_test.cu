@@ -35,7 +35,8 @@ struct Pool {  // device copies, freed together
 // are gathered from and scattered to padded vectors in reverse order.
 void test_gemm(const double2* A, int m, int k, const double2* X, int ncol, int path, double2* Y) {
     Pool P;
-    const int sx = (k + 15) / 16 * 16, sy = (m + 15) / 16 * 16;
+    const int kx = path == 8 ? m : k;  // length of an input vector
+    const int sx = (kx + 15) / 16 * 16, sy = (m + 15) / 16 * 16;
     std::vector<double2> hx((size_t)sx * ncol, make_double2(0, 0)), hy((size_t)sy * ncol, make_double2(0, 0));
     std::vector<long long> xo(ncol), yo(ncol);
     std::vector<int> xg(ncol);
@@ -46,7 +47,7 @@ void test_gemm(const double2* A, int m, int k, const double2* X, int ncol, int p
         yo[c] = (long long)at * sy;
         xg[c] = at * (sx / 16);
         vecs[c] = I8Vec{xo[c], xg[c], (unsigned short)k, (unsigned short)(path >= 6)};
-        for (int i = 0; i < k; ++i) hx[xo[c] + i] = X[(size_t)c * k + i];
+        for (int i = 0; i < kx; ++i) hx[xo[c] + i] = X[(size_t)c * kx + i];
         for (int i = 0; i < m; ++i) hy[yo[c] + i] = Y[(size_t)c * m + i];
     }
     const double2* dA = P.put(std::vector<double2>(A, A + (size_t)m * k));
@@ -54,7 +55,7 @@ void test_gemm(const double2* A, int m, int k, const double2* X, int ncol, int p
     double2* dY = P.put(hy);
     const long long* dyo = P.put(yo);
     I8Profiles prof{nullptr, sx};
-    if (path >= 6) {  // the columns as one class of vectors
+    if (path == 6 || path == 7) {  // the columns as one class of vectors
         std::vector<double> size(k, 0.0);
         for (size_t e = 0; e < (size_t)k * ncol; ++e)
             size[e % k] = std::fmax(size[e % k], std::fmax(std::fabs(X[e].x), std::fabs(X[e].y)));
@@ -80,6 +81,12 @@ void test_gemm(const double2* A, int m, int k, const double2* X, int ncol, int p
         std::vector<double2> one((size_t)m * m, make_double2(0, 0));
         for (int i = 0; i < m; ++i) one[(size_t)i * m + i] = make_double2(1, 0);
         launch_gemm_pair(GemmPair{P.put(one), dA, m, m, ncol, P.put(xo), dX, dY}, nullptr);
+    } else if (path == 8) {  // the transpose of A, then A
+        if (m > GEMM_PAIR_MAX || k > GEMM_PAIR_MAX) throw std::invalid_argument("the pair kernel takes up to 64 rows and columns");
+        std::vector<double2> t((size_t)m * k);
+        for (int i = 0; i < m; ++i)
+            for (int j = 0; j < k; ++j) t[(size_t)i * k + j] = A[(size_t)j * m + i];
+        launch_gemm_pair(GemmPair{P.put(t), dA, m, k, ncol, P.put(xo), dX, dY}, nullptr);
     } else if (path == 3 || path == 4 || path == 7) {  // mixed form, on FP32 copies: 3 FP16 planes, 4 split TF32
         auto narrow = [](const std::vector<double2>& v) {
             std::vector<float2> r;

@@ -193,7 +193,8 @@ int ddfmm_session_test_create(const double* pos3n, int n, int kernel, int accu, 
  * tensor path for few columns (PLAIN_FP64 form); 3: the FP16 tensor path (two
  * planes per number), 4: split TF32 (MIXED form, on FP32 copies); 5: the kernel
  * of two products in a row, the identity and A (m = k <= 64; Y = A X); 6, 7:
- * paths 1 and 3 with the columns' profile taken from the rows of X.  Columns
+ * paths 1 and 3 with the columns' profile taken from the rows of X; 8: the
+ * kernel of two products, A^T and A (m, k <= 64; X m x ncol, Y = A A^T X).  Columns
  * are gathered and scattered as an eval's are. */
 int ddfmm_test_gemm(const double* A, int m, int k, const double* X, int ncol, int path, double* Y);
 
