@@ -362,21 +362,6 @@ __device__ __forceinline__ HTileRef h16_tile(const HSub& one, const HSub* subs, 
     r.t = u.t;
     return r;
 }
-__device__ __forceinline__ uint32_t h16_peek(uint64_t* bar, uint32_t parity) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(done)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return done;
-}
-__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* failed, unsigned long long ns) {
-    int ok = 1;
-    if ((threadIdx.x & 31) == 0) ok = !*failed && mbar_wait(bar, parity, failed, ns);
-    return __shfl_sync(0xffffffffu, ok, 0);
-}
 }  // namespace
 
 template <bool MULTI>
@@ -516,7 +501,7 @@ __global__ void __launch_bounds__(HTHREADS, 1) h16_gemm_kernel(const HSub one, c
                     const bool two = k - kb * 16 > 8;  // the second K step holds k
                     h16_mma(d, dx, db, idesc, kb > 0);
                     h16_mma(d, dx + (H_X_PLANE >> 4), db, idesc, 1u);
-                    ready = h16_peek(&full[slot], fpar);  // answered while the rest runs
+                    ready = mbar_peek(&full[slot], fpar);  // answered while the rest runs
                     h16_mma(d, dx, db + blo, idesc, 1u);
                     if (two) {  // 32 bytes on: 2 of the swizzled rows' units, two core matrices of the operator's
                         h16_mma(d, dx + 2, db + 16, idesc, 1u);

@@ -69,6 +69,7 @@
 #include <stdexcept>
 
 #include "kernels.cuh"
+#include "umma.cuh"
 
 namespace ddfmm {
 
@@ -89,11 +90,7 @@ static_assert(I_SMEM + 1024 <= 232448, "shared memory per block");
 constexpr int ITHREADS = 512;
 constexpr int ICH = 8;                        // accumulator columns per TMEM load
 constexpr int ICHUNKS = INMAX / 2 / ICH;      // chunks of a warp's half tile
-constexpr unsigned long long I_WAIT_NS = 1000000000ull;
-constexpr uint32_t I_WAIT_ITERS = 1u << 26;
 static_assert(I_STAGE_BYTES % 256 == 0 && INMAX % 16 == 0 && INMAX <= 128, "swizzle atoms");
-
-__device__ __forceinline__ uint32_t su32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 // byte offset of byte b (0 .. 31) of row r in a 32-byte swizzled K-major plane:
 // 8-row groups of 256 bytes, the row's two 16-byte halves exchanged in rows 4 .. 7
@@ -107,17 +104,6 @@ constexpr uint32_t I_DESC_HI = (256 >> 4) | (1u << 14) | (6u << 29);
 __device__ constexpr uint32_t i8_idesc(int n) {
     return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(IM >> 4) << 24);
 }
-// whether the phase of this parity has completed; the caller may go on before it looks at the answer
-__device__ __forceinline__ uint32_t bar_peek(uint64_t* bar, uint32_t parity) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(done)
-        : "r"(su32(bar)), "r"(parity)
-        : "memory");
-    return done;
-}
 __device__ __forceinline__ void i8_mma(uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t acc) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -126,56 +112,6 @@ __device__ __forceinline__ void i8_mma(uint32_t d, uint32_t a, uint32_t b, uint3
         "r"(a), "r"(b), "r"(idesc), "r"(acc), "r"(0u), "r"(I_DESC_HI)
         : "memory");
 }
-__device__ __forceinline__ void i8_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(su32(bar))
-                 : "memory");
-}
-__device__ __forceinline__ unsigned long long i8_timer() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;\n" : "=l"(t));
-    return t;
-}
-__device__ __forceinline__ void bar_init(uint64_t* bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(su32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void bar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(su32(bar)) : "memory");
-}
-// false after limit_ns, 2^26 polls, or once *failed is set by another role
-__device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity, volatile int* failed,
-                                         unsigned long long limit_ns) {
-    const uint32_t addr = su32(bar);
-    unsigned long long t0 = 0;
-    for (uint32_t it = 0; it < I_WAIT_ITERS; ++it) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}\n"
-            : "=r"(done)
-            : "r"(addr), "r"(parity)
-            : "memory");
-        if (done) return true;
-        if ((it & 255) == 255) {
-            if (failed && *failed) return false;
-            const unsigned long long t = i8_timer();
-            if (t0 == 0)
-                t0 = t;
-            else if (t - t0 > limit_ns)
-                return false;
-        }
-    }
-    return false;
-}
-
-// bar_wait by one lane for its warp: polls take shared-memory cycles from the
-// tensor core's operand reads
-__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* failed,
-                                          unsigned long long limit_ns) {
-    int ok = 1;
-    if ((threadIdx.x & 31) == 0) ok = !*failed && bar_wait(bar, parity, failed, limit_ns);
-    return __shfl_sync(0xffffffffu, ok, 0);
-}
-
 // The MMA issuer's place in the ring: slot, its parity, and whether the slot is
 // already known to be full.
 struct I8Ring {
@@ -193,7 +129,7 @@ template <int N, int PH>
 __device__ __forceinline__ bool i8_phase(uint32_t tmem, uint32_t dx0, int nkb, I8Ring& R, uint64_t* full, uint64_t* empty,
                                          uint64_t* acc_full, volatile int* failed, unsigned long long wait_ns) {
     for (int kb = 0; kb < nkb; ++kb) {
-        if (!R.ready && !bar_wait(full + R.slot, R.parity, failed, wait_ns)) return false;
+        if (!R.ready && !mbar_wait(full + R.slot, R.parity, failed, wait_ns)) return false;
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         const uint32_t dx = dx0 + R.slot * (I_STAGE_BYTES >> 4), db = dx + (I_X_BYTES >> 4);
         uint64_t* const done = empty + R.slot;
@@ -203,15 +139,15 @@ __device__ __forceinline__ bool i8_phase(uint32_t tmem, uint32_t dx0, int nkb, I
 #pragma unroll
         for (int d = PH ? 0 : 4; d < (PH ? 4 : 8); ++d) {
             const int i0 = d < IS ? 0 : d - IS + 1;
-            if (d == (PH ? 2 : 7)) R.ready = bar_peek(full + R.slot, R.parity);
+            if (d == (PH ? 2 : 7)) R.ready = mbar_peek(full + R.slot, R.parity);
 #pragma unroll
             for (int i = i0; i <= d - i0; ++i)
                 i8_mma(tmem + (uint32_t)((d & 3) * N), dx + i * (I_X_PLANE >> 4), db + (d - i) * (N * 2), i8_idesc(N),
                        i > i0 ? 1u : (uint32_t)kb);
         }
-        i8_commit(done);
+        umma_commit(done);
     }
-    i8_commit(acc_full);
+    umma_commit(acc_full);
     return true;
 }
 
@@ -496,16 +432,16 @@ __global__ void __launch_bounds__(ITHREADS, 1) i8_gemm_kernel(const I8Sub S, int
     if (tid == 0) {
         failed_s = 0;
         for (int s = 0; s < ISTAGES; ++s) {
-            bar_init(&full[s], 2);        // the operator copy's bytes, the gathered columns
-            bar_init(&empty[s], 1);       // tcgen05.commit
+            mbar_init(&full[s], 2);        // the operator copy's bytes, the gathered columns
+            mbar_init(&empty[s], 1);       // tcgen05.commit
         }
-        bar_init(&acc_full, 1);     // tcgen05.commit
-        bar_init(&drained, 1);      // tcgen05.commit, after a failure
-        bar_init(&acc_empty, 8);    // epilogue warps
+        mbar_init(&acc_full, 1);     // tcgen05.commit
+        mbar_init(&drained, 1);      // tcgen05.commit, after a failure
+        mbar_init(&acc_empty, 8);    // epilogue warps
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(su32(&tmem_base)), "r"(512)
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_base)), "r"(512)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
@@ -522,7 +458,7 @@ __global__ void __launch_bounds__(ITHREADS, 1) i8_gemm_kernel(const I8Sub S, int
         // phase ahead would read the slot's empty barrier by the wrong parity).  Lane l
         // copies half l % 2 of the 32-byte rows of columns l / 2 + 16 j
         const int hf = lane & 1;
-        const uint32_t dst = su32(sm) + i8_off(lane >> 1, hf * 16);
+        const uint32_t dst = smem_u32(sm) + i8_off(lane >> 1, hf * 16);
         int g = 0;
         bool ok = true;
         I8Tile Tn = i8_tile(S, blockIdx.x);
@@ -547,12 +483,12 @@ __global__ void __launch_bounds__(ITHREADS, 1) i8_gemm_kernel(const I8Sub S, int
                     if (lane == 0 && !(withhold && blockIdx.x == 0)) {  // withheld: full[s] never completes
                         const uint32_t bytes = (uint32_t)(ph == 0 ? IS : 4) * T.n * 32;
                         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%1], %0;\n" ::"r"(bytes),
-                                     "r"(su32(&full[s]))
+                                     "r"(smem_u32(&full[s]))
                                      : "memory");
                         asm volatile(
                             "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
-                                su32(sm + s * I_STAGE_BYTES + I_X_BYTES)),
-                            "l"(T.B + (size_t)kb * IS * T.n * 32), "r"(bytes), "r"(su32(&full[s]))
+                                smem_u32(sm + s * I_STAGE_BYTES + I_X_BYTES)),
+                            "l"(T.B + (size_t)kb * IS * T.n * 32), "r"(bytes), "r"(smem_u32(&full[s]))
                             : "memory");
                     }
                     const uint32_t so = dst + s * I_STAGE_BYTES;
@@ -563,7 +499,7 @@ __global__ void __launch_bounds__(ITHREADS, 1) i8_gemm_kernel(const I8Sub S, int
                     asm volatile("cp.async.wait_all;\n" ::: "memory");
                     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
                     __syncwarp();
-                    if (lane == 0) bar_arrive(&full[s]);
+                    if (lane == 0) mbar_arrive(&full[s]);
                 }
         }
         asm volatile("cp.async.wait_all;\n" ::: "memory");
@@ -572,7 +508,7 @@ __global__ void __launch_bounds__(ITHREADS, 1) i8_gemm_kernel(const I8Sub S, int
         if (warp == 4 && lane == 0) {
             // -------------------------------------------- MMA issue
             I8Ring R{0, 0, 0};
-            const uint32_t dx0 = i8_desc(su32(sm));
+            const uint32_t dx0 = i8_desc(smem_u32(sm));
             uint32_t parity = 1;  // of acc_empty; the first wait passes
             bool ok = true;
             I8Tile T = i8_tile(S, blockIdx.x);
@@ -583,7 +519,7 @@ __global__ void __launch_bounds__(ITHREADS, 1) i8_gemm_kernel(const I8Sub S, int
 #define DDFMM_I8_CASE(n) \
     case n: ok = ph == 0 ? DDFMM_I8_PHASE(n, 0) : DDFMM_I8_PHASE(n, 1); break;
                 for (int ph = 0; ph < 2 && ok; ++ph) {
-                    ok = bar_wait(&acc_empty, parity, failed, wait_ns);
+                    ok = mbar_wait(&acc_empty, parity, failed, wait_ns);
                     parity ^= 1;
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -602,8 +538,8 @@ __global__ void __launch_bounds__(ITHREADS, 1) i8_gemm_kernel(const I8Sub S, int
             }
             if (!ok) {  // let the MMAs already issued finish before TMEM is freed
                 *failed = 1;
-                i8_commit(&drained);
-                bar_wait(&drained, 0, nullptr, wait_ns);
+                umma_commit(&drained);
+                mbar_wait(&drained, 0, nullptr, wait_ns);
             }
         }
     } else {
@@ -648,7 +584,7 @@ __global__ void __launch_bounds__(ITHREADS, 1) i8_gemm_kernel(const I8Sub S, int
                 }
             asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
             __syncwarp();
-            if (lane == 0) bar_arrive(&acc_empty);
+            if (lane == 0) mbar_arrive(&acc_empty);
             ++q;
             if (!warp_wait(&acc_full, q & 1, failed, wait_ns)) {
                 *failed = 1;
@@ -669,7 +605,7 @@ __global__ void __launch_bounds__(ITHREADS, 1) i8_gemm_kernel(const I8Sub S, int
                 }
             asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
             __syncwarp();
-            if (lane == 0) bar_arrive(&acc_empty);
+            if (lane == 0) mbar_arrive(&acc_empty);
             ++q;
             int gn = 0;
             if (col < Tn.ncol) {
@@ -694,7 +630,7 @@ __global__ void __launch_bounds__(ITHREADS, 1) i8_gemm_kernel(const I8Sub S, int
                     if (y)
                         asm volatile(
                             "cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f64 [%0], [%1], %2;\n" ::"l"(y + b),
-                            "r"(su32(mine)), "r"(min(IPR, nr - b) * 16)
+                            "r"(smem_u32(mine)), "r"(min(IPR, nr - b) * 16)
                             : "memory");
                     asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
                 }
@@ -707,8 +643,8 @@ __global__ void __launch_bounds__(ITHREADS, 1) i8_gemm_kernel(const I8Sub S, int
     __syncthreads();
     if (*failed && tid == 0) {
         // bounded drain of operator copies still in flight, then report
-        const unsigned long long t0 = i8_timer();
-        while (i8_timer() - t0 < 200000ull) __nanosleep(1000);
+        const unsigned long long t0 = gtimer();
+        while (gtimer() - t0 < 200000ull) __nanosleep(1000);
         atomicExch(err, 1);
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -733,7 +669,7 @@ void i8_init() {
 void launch_i8_gemm(const I8Sub& S, int* err, cudaStream_t s, unsigned long long wait_ns, int withhold) {
     if (S.ntiles == 0) return;
     const int sms = g_i8_sms > 0 ? g_i8_sms : 148;
-    i8_gemm_kernel<<<S.ntiles < sms ? S.ntiles : sms, ITHREADS, I_SMEM, s>>>(S, err, wait_ns ? wait_ns : I_WAIT_NS, withhold);
+    i8_gemm_kernel<<<S.ntiles < sms ? S.ntiles : sms, ITHREADS, I_SMEM, s>>>(S, err, wait_ns ? wait_ns : U_WAIT_NS, withhold);
 }
 
 }  // namespace ddfmm

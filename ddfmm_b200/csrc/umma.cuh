@@ -1,4 +1,4 @@
-// What the FP32 tcgen05 GEMM kernels share: bounded mbarrier waits, bulk copies,
+// What the tcgen05 GEMM kernels share: bounded mbarrier waits, bulk copies,
 // commits and the parked stores of the epilogue.
 #pragma once
 #include <cstdint>
@@ -50,6 +50,28 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
         }
     }
     return false;
+}
+
+// mbar_wait by one lane for its warp: polls take shared-memory cycles from the tensor
+// core's operand reads.
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* failed,
+                                          unsigned long long limit_ns) {
+    int ok = 1;
+    if ((threadIdx.x & 31) == 0) ok = !*failed && mbar_wait(bar, parity, failed, limit_ns);
+    return __shfl_sync(0xffffffffu, ok, 0);
+}
+
+// Whether the phase of this parity has completed; the caller may go on before it looks at
+// the answer.
+__device__ __forceinline__ uint32_t mbar_peek(uint64_t* bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(done)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return done;
 }
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
