@@ -469,8 +469,6 @@ void gemm_init() {
     cudaFuncSetAttribute(zgemm_narrow_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, NARROW_SMEM);
 }
 
-size_t narrow_smem(int k) { return sizeof(double2) * 8 * ((size_t)(k + 7) / 8 * 8 + 4); }
-
 void launch_gemm_narrow(const GemmProblem* probs, const GemmTile* tiles, int ntiles, const long long* xoff,
                         const long long* yoff, const double2* X, double2* Y, int mode, int kmax, int rows,
                         cudaStream_t s) {

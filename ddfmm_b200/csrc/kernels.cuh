@@ -74,7 +74,9 @@ void launch_gemm(const GemmProblem* probs_dev, const GemmTile* tiles_dev, int nt
 // Products with few columns: tiles of `rows` (64 or 128) operator rows x 8 columns; kmax: the
 // launch's longest k, narrow_smem(kmax) <= NARROW_SMEM.
 constexpr int NARROW_SMEM = 72 << 10;
-size_t narrow_smem(int k);
+constexpr size_t narrow_smem(int k) { return sizeof(double2) * 8 * ((size_t)(k + 7) / 8 * 8 + 4); }
+// every operator's m and k are at most the largest skeleton rank (OperatorLib::validate) or surface
+static_assert(narrow_smem(400) <= NARROW_SMEM, "shared memory of the longest column");
 // Y[off[c] ..] = B (A X[off[c] ..]) for ncol columns: A r x m, B m x r, column-major and dense, m, r <= GEMM_PAIR_MAX
 constexpr int GEMM_PAIR_MAX = 64;
 struct GemmPair {

@@ -1,7 +1,7 @@
 // Process-wide cache of packed translation operators (mixed form).
 //
-// The folded M2M / L2L / M2L operators and the E2 skeleton factors depend on
-// the operator files, the kernel, the accuracy level and the (width, wedge,
+// The folded M2M / L2L / M2L operators, packed as FP16 planes with the vectors'
+// profiles in their columns, depend on the operator files, the kernel, the accuracy level and the (width, wedge,
 // child or offset) they serve -- not on the geometry -- so every session on a
 // device that uses the same files shares one packed copy of each.  Entries are
 // reference counted: a session holds the entries it uses, the cache keeps

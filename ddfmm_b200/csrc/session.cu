@@ -422,9 +422,12 @@ void Session::add_umma(const std::vector<GemmProblem>& P, const long long* xs, c
 // and 2700 a K block (k = 76: 24 k, k = 152: 37 k); the FP64 tensor path does 11
 // complex products a clock with many columns, 8 with few.  So 128 columns of a
 // 100 x 152 operator cost 75 k against 177 k, 32 columns 75 k against 61 k.  The
-// launch must gain what its digits, its second launch and its last wave cost:
-// at K = 8, P = 4 a gain of 24 us an SM by this count is a loss of 30 us (0.435
-// ms on the FP64 path alone, 0.465 ms with the M2L problems split off).
+// launch must gain what its digits, its second launch and its last wave cost.  An eval with
+// that line at 0, 20 k, 60 k and 150 k clocks an SM (us): sphere K = 8, P = 4 341, 299, 289,
+// 289; P = 6 835, 833, 835, 805; P = 8 1904, 1905, 1906, 1904; K = 4, P = 8 516, 490, 487,
+// 486; ellipsoid K = 16, P = 4 423, 363, 345, 346; P = 6 984, 960, 962, 988; sphere K = 16,
+// P = 4 1308, 1243, 1231, 1227; P = 6 3083, 3075, 3026, 3055; exp(ir) 1446, 1404, 1402, 1434;
+// cluster K = 8, P = 4 671, 659, 664, 656; P = 8 2411, 2412, 2409, 2316.
 static std::vector<char> i8_choose(const std::vector<std::array<int, 3> >& shapes) {
     std::vector<char> on(shapes.size(), 0);
     double gain = 0;
@@ -1735,7 +1738,11 @@ void Session::build() {
     phase("steps_hf_down");
     // Small instances do not fill the GPU in any pass: their V-list sums and near field
     // run beside the high-frequency passes (run_steps).  The line is the size of the
-    // summed target spectra, which then need memory of their own.
+    // summed target spectra, which then need memory of their own.  One stream / with branches,
+    // by that size: plain 8 MB 325 / 287 us, 31 MB 1284 / 1237, 105 MB 3098 / 3024, a cluster
+    // with 36 MB 1111 / 663; mixed 53 MB 1206 / 1145, 67 MB 1535 / 1422.  At the line it is even
+    // (plain K = 32: 123 MB 5313 / 5440, 133 MB 3726 / 3588), above it nothing (mixed 207 MB
+    // 4508 / 4461 us, 832 MB 17.54 / 17.58 ms).
     overlap_ = !hflevels.empty() && !lflevels.empty() && (size_t)nLF * G3 * es <= ((size_t)128 << 20);
     if (overlap_) {
         branch_.resize(std::min<size_t>(lflevels.size(), kBranches));
