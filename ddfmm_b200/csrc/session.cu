@@ -1631,7 +1631,10 @@ void Session::build() {
         for (const Canon& c : hfcanon) {
             std::vector<double> size(c.r1, 0.0);
             for (int j = 0; j < c.r1; ++j) {
-                for (int i = 0; i < c.r1; ++i) size[j] = std::max(size[j], std::abs(c.op->E1(i, j)));
+                for (int i = 0; i < c.r1; ++i) {
+                    const cpx& e = c.op->E1(i, j);
+                    size[j] = std::max(size[j], std::max(std::fabs(e.real()), std::fabs(e.imag())));
+                }
                 size[j] = 1.0 / size[j];
             }
             const std::vector<unsigned char> row = i8_profile(size.data(), c.r1, stride);
